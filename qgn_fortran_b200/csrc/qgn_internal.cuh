@@ -72,7 +72,7 @@ struct ModalConst {
     double Htot;
 };
 
-// GetPsi constants of a fixed layer count (2, 4, 8, 16) passed by value as a kernel parameter:
+// GetPsi constants of a fixed layer count passed by value as a kernel parameter:
 // the unrolled arithmetic reads the matrix entries straight from the constant bank, with no
 // shared-memory staging and no load instructions
 template <int NZ>
@@ -92,48 +92,6 @@ inline ModalParams<NZ> modal_params(const ModalConst& mc) {
     for (int i = 0; i < NZ; ++i) m.ev[i] = mc.evals[i];
     m.Htot = mc.Htot;
     return m;
-}
-
-// The GetPsi constants as a kernel argument: by value for a fixed layer count, else the device
-// copy, which the kernel stages in shared memory (modal_view)
-template <int NZ>
-struct ModalArg {
-    ModalParams<NZ> m;
-};
-template <>
-struct ModalArg<0> {
-    const ModalConst* mc;
-};
-
-// shared-memory staging arrays of a GetPsi kernel (used only for NZ = 0)
-#define QGN_MODAL_SHARED(NZ)                                                      \
-    __shared__ double s_proj[(NZ) > 0 ? 1 : kMaxNZ * kMaxNZ];                     \
-    __shared__ double s_back[(NZ) > 0 ? 1 : kMaxNZ * kMaxNZ];                     \
-    __shared__ double s_ev[(NZ) > 0 ? 1 : kMaxNZ]
-
-struct ModalView {
-    const double* proj;
-    const double* back;
-    const double* ev;
-    double Htot;
-};
-
-// where the kernel reads the constants from; for NZ = 0 every thread of the block must call
-// this (it stages the device copy and synchronises)
-template <int NZ>
-__device__ __forceinline__ ModalView modal_view(const ModalArg<NZ>& a, double* s_proj, double* s_back, double* s_ev,
-                                                int nz) {
-    if constexpr (NZ > 0) {
-        return ModalView{a.m.proj, a.m.back, a.m.ev, a.m.Htot};
-    } else {
-        for (int i = threadIdx.x; i < nz * nz; i += blockDim.x) {
-            s_proj[i] = a.mc->proj[i];
-            s_back[i] = a.mc->back[i];
-        }
-        for (int i = threadIdx.x; i < nz; i += blockDim.x) s_ev[i] = a.mc->evals[i];
-        __syncthreads();
-        return ModalView{s_proj, s_back, s_ev, a.mc->Htot};
-    }
 }
 
 // Device scalars of the adaptive controllers.  The controller kernel makes every
@@ -183,13 +141,6 @@ struct Buffers {
     const ModalConst* mc_h = nullptr;   // host copy of *mc, the source of ModalParams
     DevScalars* sc = nullptr;
 };
-
-// the kernel argument of the GetPsi constants (NZ = 0, or no host copy: the device copy)
-template <int NZ>
-inline ModalArg<NZ> modal_arg(const Buffers& b) {
-    if constexpr (NZ > 0) return ModalArg<NZ>{modal_params<NZ>(*b.mc_h)};
-    else return ModalArg<0>{b.mc};
-}
 
 }  // namespace qgn
 
@@ -248,8 +199,13 @@ void closure_free(qgn_ctx* ctx);
 const double2* closure_tendency(const qgn_ctx* ctx);
 void drop_graphs(qgn_ctx* ctx);
 
-// ---- launch wrappers (rhs_kernels.cu) -------------------------------------------------
+// ---- GetPsi (modal.cu) ------------------------------------------------------------------
 cudaError_t launch_modal(const Geom& g, const Buffers& b, const double2* q, double2* psi, cudaStream_t s);
+cudaError_t launch_modal_f32(const Geom& g, const Buffers& b, const float2* q, float2* psi, cudaStream_t s);
+cudaError_t launch_modal_mixed(const Geom& g, const Buffers& b, const double2* q, float2* q32, float2* psi32,
+                               cudaStream_t s);
+
+// ---- launch wrappers (rhs_kernels.cu) -------------------------------------------------
 // extra (optional, compact): a tendency added to the RHS on the kept modes (learned closure)
 cudaError_t launch_rhs(const Geom& g, const Buffers& b, const double2* q, const double2* psi, double2* out,
                        bool do_drag, cudaStream_t s, const double2* extra = nullptr);
@@ -296,8 +252,6 @@ cudaError_t launch_yfwd_stage_yinv(const Geom& g, const Buffers& b, int stage, c
 cudaError_t launch_ark_update(const Geom& g, const Buffers& b, cudaStream_t s);
 cudaError_t launch_ark_stage_mixed(const Geom& g, const Buffers& b, int stage, cudaStream_t s);
 cudaError_t launch_ark_update_mixed(const Geom& g, const Buffers& b, cudaStream_t s);
-cudaError_t launch_modal_mixed(const Geom& g, const Buffers& b, const double2* q, float2* q32, float2* psi32,
-                               cudaStream_t s);
 cudaError_t launch_f2d(size_t n, const float2* a, double2* b, cudaStream_t s);
 cudaError_t launch_combo(const Geom& g, const Buffers& b, const Combo& cb, const double2* q, double2* out,
                          double2* psi, bool want_psi, cudaStream_t s);

@@ -27,30 +27,6 @@
 
 namespace qgn {
 
-template <int NZ>
-__global__ void __launch_bounds__(256, 2) k_modal(Geom g, const __grid_constant__ ModalArg<NZ> ma,
-                                               const double2* __restrict__ q, double2* __restrict__ psi) {
-    QGN_PDL_ENTRY();
-    QGN_MODAL_SHARED(NZ);
-    const int nz = g.nz;
-    const ModalView mv = modal_view<NZ>(ma, s_proj, s_back, s_ev, nz);
-    const size_t P = (size_t)g.nkx * g.nky;
-    const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
-    const int kx = (int)(p / g.nky), m = (int)(p % g.nky);
-    const double kxv = g.dkx * kx, kyv = g.kyval(g.jfull(m));
-    const double k2 = kxv * kxv + kyv * kyv;
-    constexpr int NZC = NZ > 0 ? NZ : kMaxNZ;
-    double2 qv[NZC], pv[NZC];
-#pragma unroll
-    for (int k = 0; k < NZC; ++k)
-        if (k < nz) qv[k] = in_bounds(g, (size_t)k * P + p, g.csize()) ? q[(size_t)k * P + p] : make_double2(0.0, 0.0);
-    modal_invert<NZ>(mv.proj, mv.back, mv.ev, mv.Htot, nz, k2, p == 0, qv, pv);
-#pragma unroll
-    for (int k = 0; k < NZC; ++k)
-        if (k < nz && in_bounds(g, (size_t)k * P + p, g.csize())) psi[(size_t)k * P + p] = pv[k];
-}
-
 // ------------------------------------------------------------------------------------
 // Single-field launches of the tile bodies (rhs_tiles.cuh): one CTA per tile, tile = blockIdx
 // ------------------------------------------------------------------------------------
@@ -204,20 +180,6 @@ static cudaError_t dispatch_n(int n, F&& f) {
 template <class K>
 static cudaError_t set_smem(K kernel, int bytes) {
     return smem_opt_in(kernel, bytes);
-}
-
-cudaError_t launch_modal(const Geom& g, const Buffers& b, const double2* q, double2* psi, cudaStream_t s) {
-    const size_t P = (size_t)g.nkx * g.nky;
-    dim3 grid((unsigned)((P + 255) / 256));
-    const double nb = 2.0 * 16.0 * (double)g.csize();
-    switch (b.mc_h ? g.nz : 0) {
-        case 2: QGN_LAUNCH(KID_MODAL, nb, s, ::qgn::launch(k_modal<2>, grid, 256, 0, s, g, modal_arg<2>(b), q, psi)); break;
-        case 4: QGN_LAUNCH(KID_MODAL, nb, s, ::qgn::launch(k_modal<4>, grid, 256, 0, s, g, modal_arg<4>(b), q, psi)); break;
-        case 8: QGN_LAUNCH(KID_MODAL, nb, s, ::qgn::launch(k_modal<8>, grid, 256, 0, s, g, modal_arg<8>(b), q, psi)); break;
-        case 16: QGN_LAUNCH(KID_MODAL, nb, s, ::qgn::launch(k_modal<16>, grid, 256, 0, s, g, modal_arg<16>(b), q, psi)); break;
-        default: QGN_LAUNCH(KID_MODAL, nb, s, ::qgn::launch(k_modal<0>, grid, 256, 0, s, g, modal_arg<0>(b), q, psi)); break;
-    }
-    return cudaGetLastError();
 }
 
 template <int NY, int NF, class CT, int TV>

@@ -14,6 +14,7 @@
 
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <unordered_set>
 
 namespace qgn {
@@ -38,43 +39,6 @@ __constant__ double c_ai[36] = {
 __constant__ double c_b[6] = {82889.0 / 524892.0, 0.0, 15625.0 / 83664.0, 69875.0 / 102672.0, -2260.0 / 8211.0, 0.25};
 __constant__ double c_be[6] = {31666707.0 / 9881966720.0, 0.0, -256875.0 / 105007616.0, -2768025.0 / 128864768.0,
                                169839.0 / 3864644.0, -5247.0 / 225920.0};
-
-template <int NZ>
-__device__ __forceinline__ void modal_invert_s(const double* proj, const double* back, const double* ev, double Htot,
-                                               int nz, double k2, bool mean_mode, const double2* qv, double2* pv) {
-    constexpr int NZC = NZ > 0 ? NZ : kMaxNZ;
-    const int n = NZ > 0 ? NZ : nz;
-    double2 pm[NZC];
-#pragma unroll
-    for (int k = 0; k < NZC; ++k) {
-        if (k < n) {
-            double2 acc = make_double2(0.0, 0.0);
-#pragma unroll
-            for (int kk = 0; kk < NZC; ++kk)
-                if (kk < n) {
-                    const double c = proj[k * n + kk];
-                    acc.x += c * qv[kk].x;
-                    acc.y += c * qv[kk].y;
-                }
-            const double rden = 1.0 / ((-k2 + ev[k]) * Htot);
-            pm[k] = mean_mode ? make_double2(0.0, 0.0) : make_double2(acc.x * rden, acc.y * rden);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < NZC; ++k) {
-        if (k < n) {
-            double2 acc = make_double2(0.0, 0.0);
-#pragma unroll
-            for (int kk = 0; kk < NZC; ++kk)
-                if (kk < n) {
-                    const double c = back[k * n + kk];
-                    acc.x += pm[kk].x * c;
-                    acc.y += pm[kk].y * c;
-                }
-            pv[k] = acc;
-        }
-    }
-}
 
 struct StagePtrs {
     const double2* N[6];
@@ -156,7 +120,7 @@ __device__ __forceinline__ void comp_add_double(Comp32& acc, double x) {
 // ---- ARK stage s as two streaming kernels ------------------------------------------------------
 // k_ark_comb: one thread per (layer, mode): q_s = Mq (q + dt (sum ae N_j + sum ai L_j)), the
 // sums in FP64 (FP64 storage) or Kahan-compensated FP32 (FP32 storage, mixed mode), q in FP64.
-// GetPsi of q_s follows as a separate all-layers kernel (k_modal / k_modal_f32).
+// GetPsi of q_s follows as a separate all-layers kernel (modal.cu).
 template <class T> struct StoreT;
 template <> struct StoreT<double2> {
     __device__ static double2 put(double x, double y) { return make_double2(x, y); }
@@ -239,35 +203,6 @@ __global__ void __launch_bounds__(256) k_ark_comb(Geom g, CombPtrs<T> cp, const 
     qout[e] = StoreT<T>::put(Mq * (q0.x + dt * ax), Mq * (q0.y + dt * ay));
 }
 
-// GetPsi of an FP32 field with FP64 arithmetic (mixed mode)
-template <int NZ>
-__global__ void __launch_bounds__(256, 2) k_modal_f32(Geom g, const __grid_constant__ ModalArg<NZ> ma,
-                                                      const float2* __restrict__ q, float2* __restrict__ psi) {
-    QGN_PDL_ENTRY();
-    QGN_MODAL_SHARED(NZ);
-    const int nz = g.nz;
-    const ModalView mv = modal_view<NZ>(ma, s_proj, s_back, s_ev, nz);
-    const size_t P = (size_t)g.nkx * g.nky;
-    const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
-    int kx, m;
-    double k2;
-    point_k(g, p, kx, m, k2);
-    constexpr int NZC = NZ > 0 ? NZ : kMaxNZ;
-    double2 qv[NZC], pv[NZC];
-#pragma unroll
-    for (int l = 0; l < NZC; ++l)
-        if (l < nz) {
-            const float2 v = q[(size_t)l * P + p];
-            qv[l] = make_double2(v.x, v.y);
-        }
-    modal_invert_s<NZ>(mv.proj, mv.back, mv.ev, mv.Htot, nz, k2, p == 0, qv, pv);
-#pragma unroll
-    for (int l = 0; l < NZC; ++l)
-        if (l < nz) psi[(size_t)l * P + p] = make_float2((float)pv[l].x, (float)pv[l].y);
-}
-
-
 struct StagePtrs32 {
     const float2* N[6];
     const float2* Qs[6];
@@ -314,52 +249,21 @@ __global__ void __launch_bounds__(256) k_ark_update_mixed(Geom g, StagePtrs32 sp
     qnew[e] = (p == 0) ? make_double2(0.0, 0.0) : make_double2(q0.x + dt * uc.x, q0.y + dt * uc.y);
 }
 
-// FP32 copy of the FP64 state and its GetPsi (FP64 arithmetic, FP32 result)
-template <int NZ>
-__global__ void __launch_bounds__(256, 2) k_modal_mixed(Geom g, const __grid_constant__ ModalArg<NZ> ma,
-                                                     const double2* __restrict__ q, float2* __restrict__ q32,
-                                                     float2* __restrict__ psi32) {
-    QGN_PDL_ENTRY();
-    QGN_MODAL_SHARED(NZ);
-    const int nz = g.nz;
-    const ModalView mv = modal_view<NZ>(ma, s_proj, s_back, s_ev, nz);
-    const size_t P = (size_t)g.nkx * g.nky;
-    const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
-    int kx, m;
-    double k2;
-    point_k(g, p, kx, m, k2);
-    constexpr int NZC = NZ > 0 ? NZ : kMaxNZ;
-    double2 qv[NZC], pv[NZC];
-#pragma unroll
-    for (int l = 0; l < NZC; ++l)
-        if (l < nz) qv[l] = q[(size_t)l * P + p];
-    modal_invert_s<NZ>(mv.proj, mv.back, mv.ev, mv.Htot, nz, k2, p == 0, qv, pv);
-#pragma unroll
-    for (int l = 0; l < NZC; ++l) {
-        if (l < nz) {
-            q32[(size_t)l * P + p] = make_float2((float)qv[l].x, (float)qv[l].y);
-            psi32[(size_t)l * P + p] = make_float2((float)pv[l].x, (float)pv[l].y);
-        }
-    }
-}
-
 __global__ void k_f2d(size_t n, const float2* __restrict__ a, double2* __restrict__ b) {
     QGN_PDL_ENTRY();
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e < n) b[e] = make_double2(a[e].x, a[e].y);
 }
 
-// ---- explicit combinations: out = q + sum_j (a_j dt) R_j, then optionally psi = GetPsi(out) ---
+// ---- explicit combinations: out = q + sum_j (a_j dt) R_j ---------------------------------------
+// with psi = GetPsi(out) in the same pass, one thread per mode over all layers (nz <= 8: the
+// layers fit its registers)
 template <int NZ>
 __global__ void __launch_bounds__(256, 2) k_combo(Geom g, Combo cb, const double2* __restrict__ q,
                                                double2* __restrict__ out, double2* __restrict__ psi,
-                                               const __grid_constant__ ModalArg<NZ> ma,
-                                               const DevScalars* __restrict__ sc, int want_psi) {
+                                               const __grid_constant__ ModalParams<NZ> ma,
+                                               const DevScalars* __restrict__ sc) {
     QGN_PDL_ENTRY();
-    QGN_MODAL_SHARED(NZ);
-    const int nz = g.nz;
-    const ModalView mv = modal_view<NZ>(ma, s_proj, s_back, s_ev, nz);
     const size_t P = (size_t)g.nkx * g.nky;
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
@@ -367,30 +271,46 @@ __global__ void __launch_bounds__(256, 2) k_combo(Geom g, Combo cb, const double
     double k2;
     point_k(g, p, kx, m, k2);
     const double dt = sc->dt;
-    constexpr int NZC = NZ > 0 ? NZ : kMaxNZ;
-    double2 qv[NZC], pv[NZC];
+    double2 qv[NZ], pv[NZ];
 #pragma unroll
-    for (int l = 0; l < NZC; ++l) {
-        if (l < nz) {
-            const size_t idx = (size_t)l * P + p;
-            double2 v = q[idx];
-            for (int j = 0; j < cb.n; ++j) {
-                const double c = cb.a[j] * dt;
-                const double2 r = cb.R[j][idx];
-                v.x += c * r.x;
-                v.y += c * r.y;
-            }
-            qv[l] = v;
+    for (int l = 0; l < NZ; ++l) qv[l] = q[(size_t)l * P + p];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j >= cb.n) break;
+        const double c = cb.a[j] * dt;
+        const double2* R = cb.R[j];
+#pragma unroll
+        for (int l = 0; l < NZ; ++l) {
+            const double2 r = R[(size_t)l * P + p];
+            qv[l].x += c * r.x;
+            qv[l].y += c * r.y;
         }
     }
-    if (want_psi) modal_invert_s<NZ>(mv.proj, mv.back, mv.ev, mv.Htot, nz, k2, p == 0, qv, pv);
+    modal_invert<NZ>(ma.proj, ma.back, ma.ev, ma.Htot, NZ, k2, p == 0, qv, pv);
 #pragma unroll
-    for (int l = 0; l < NZC; ++l) {
-        if (l < nz) {
-            out[(size_t)l * P + p] = qv[l];
-            if (want_psi) psi[(size_t)l * P + p] = pv[l];
-        }
+    for (int l = 0; l < NZ; ++l) {
+        out[(size_t)l * P + p] = qv[l];
+        psi[(size_t)l * P + p] = pv[l];
     }
+}
+
+// without psi, or before a GetPsi of its own (nz > 8): one thread per element
+__global__ void __launch_bounds__(256) k_combo_stream(size_t n, Combo cb, const double2* __restrict__ q,
+                                                      double2* __restrict__ out, const DevScalars* __restrict__ sc) {
+    QGN_PDL_ENTRY();
+    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n) return;
+    const double dt = sc->dt;
+    double2 v = q[e];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j >= cb.n) break;
+        const double c = cb.a[j] * dt;
+        const double2 r = cb.R[j][e];
+        v.x += c * r.x;
+        v.y += c * r.y;
+    }
+    out[e] = v;
 }
 
 // ---- linear combination without q: out = sum_j a_j R_j (error spectra) --------------------
@@ -399,7 +319,9 @@ __global__ void k_lincomb(size_t n, Combo cb, double2* __restrict__ out) {
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n) return;
     double2 v = make_double2(0.0, 0.0);
-    for (int j = 0; j < cb.n; ++j) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j >= cb.n) break;
         const double2 r = cb.R[j][e];
         v.x += cb.a[j] * r.x;
         v.y += cb.a[j] * r.y;
@@ -651,6 +573,21 @@ __global__ void k_set_time(DevScalars* sc, double t, double dt) {
 // ------------------------------------------------------------------------------------------
 // launch wrappers
 // ------------------------------------------------------------------------------------------
+// calls f with the layer count 2..8 as a constant
+template <class F>
+static void dispatch_small_nz(int nz, F&& f) {
+    switch (nz) {
+        case 2: f(std::integral_constant<int, 2>{}); break;
+        case 3: f(std::integral_constant<int, 3>{}); break;
+        case 4: f(std::integral_constant<int, 4>{}); break;
+        case 5: f(std::integral_constant<int, 5>{}); break;
+        case 6: f(std::integral_constant<int, 6>{}); break;
+        case 7: f(std::integral_constant<int, 7>{}); break;
+        case 8: f(std::integral_constant<int, 8>{}); break;
+        default: break;
+    }
+}
+
 static inline unsigned blocks_for(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 template <class T>
@@ -688,12 +625,9 @@ template <int S, int NZ>
 __global__ void __launch_bounds__(256, 2) k_ark_stage_small(Geom g, CombPtrs<double2> cp, const double2* __restrict__ q,
                                                            double2* __restrict__ qout, double2* __restrict__ psi,
                                                            const LayerConst* __restrict__ lc,
-                                                           const __grid_constant__ ModalArg<NZ> ma,
+                                                           const __grid_constant__ ModalParams<NZ> ma,
                                                            const DevScalars* __restrict__ sc) {
     QGN_PDL_ENTRY();
-    QGN_MODAL_SHARED(NZ);
-    const int nz = g.nz;
-    const ModalView mv = modal_view<NZ>(ma, s_proj, s_back, s_ev, nz);
     const size_t P = (size_t)g.nkx * g.nky;
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
@@ -702,11 +636,10 @@ __global__ void __launch_bounds__(256, 2) k_ark_stage_small(Geom g, CombPtrs<dou
     point_k(g, p, kx, m, k2);
     const double k8 = (k2 * k2) * (k2 * k2);
     const double dt = sc->dt;
-    constexpr int NZC = NZ > 0 ? NZ : kMaxNZ;
-    double2 qv[NZC], pv[NZC];
+    double2 qv[NZ], pv[NZ];
 #pragma unroll
-    for (int l = 0; l < NZC; ++l) {
-        if (l < nz) {
+    for (int l = 0; l < NZ; ++l) {
+        {
             const size_t e = (size_t)l * P + p;
             const double D = lc->A2 * k2 + sc->A8L[l] * k8;
             double2 nn[S], qq[S];
@@ -722,10 +655,10 @@ __global__ void __launch_bounds__(256, 2) k_ark_stage_small(Geom g, CombPtrs<dou
             qout[e] = qv[l];
         }
     }
-    modal_invert_s<NZ>(mv.proj, mv.back, mv.ev, mv.Htot, nz, k2, p == 0, qv, pv);
+    modal_invert<NZ>(ma.proj, ma.back, ma.ev, ma.Htot, NZ, k2, p == 0, qv, pv);
 #pragma unroll
-    for (int l = 0; l < NZC; ++l)
-        if (l < nz) psi[(size_t)l * P + p] = pv[l];
+    for (int l = 0; l < NZ; ++l)
+        psi[(size_t)l * P + p] = pv[l];
 }
 
 // grids of at most this many kept mode-layers take the fused stage kernel and the column kernels
@@ -745,11 +678,11 @@ static cudaError_t launch_stage_small_nz(const Geom& g, const Buffers& b, int s,
     const double C = (double)g.csize(), nb = 16.0 * C * (2.0 * s + 2.0);
     double2* qo = b.Qs[s];
     switch (s) {
-        case 1: QGN_LAUNCH(KID_STAGE, nb, st, (::qgn::launch(k_ark_stage_small<1, NZ>, nbk, 256, 0, st, g, cp, b.q, qo, b.psi, b.lc, modal_arg<NZ>(b), b.sc))); break;
-        case 2: QGN_LAUNCH(KID_STAGE, nb, st, (::qgn::launch(k_ark_stage_small<2, NZ>, nbk, 256, 0, st, g, cp, b.q, qo, b.psi, b.lc, modal_arg<NZ>(b), b.sc))); break;
-        case 3: QGN_LAUNCH(KID_STAGE, nb, st, (::qgn::launch(k_ark_stage_small<3, NZ>, nbk, 256, 0, st, g, cp, b.q, qo, b.psi, b.lc, modal_arg<NZ>(b), b.sc))); break;
-        case 4: QGN_LAUNCH(KID_STAGE, nb, st, (::qgn::launch(k_ark_stage_small<4, NZ>, nbk, 256, 0, st, g, cp, b.q, qo, b.psi, b.lc, modal_arg<NZ>(b), b.sc))); break;
-        case 5: QGN_LAUNCH(KID_STAGE, nb, st, (::qgn::launch(k_ark_stage_small<5, NZ>, nbk, 256, 0, st, g, cp, b.q, qo, b.psi, b.lc, modal_arg<NZ>(b), b.sc))); break;
+        case 1: QGN_LAUNCH(KID_STAGE, nb, st, (::qgn::launch(k_ark_stage_small<1, NZ>, nbk, 256, 0, st, g, cp, b.q, qo, b.psi, b.lc, modal_params<NZ>(*b.mc_h), b.sc))); break;
+        case 2: QGN_LAUNCH(KID_STAGE, nb, st, (::qgn::launch(k_ark_stage_small<2, NZ>, nbk, 256, 0, st, g, cp, b.q, qo, b.psi, b.lc, modal_params<NZ>(*b.mc_h), b.sc))); break;
+        case 3: QGN_LAUNCH(KID_STAGE, nb, st, (::qgn::launch(k_ark_stage_small<3, NZ>, nbk, 256, 0, st, g, cp, b.q, qo, b.psi, b.lc, modal_params<NZ>(*b.mc_h), b.sc))); break;
+        case 4: QGN_LAUNCH(KID_STAGE, nb, st, (::qgn::launch(k_ark_stage_small<4, NZ>, nbk, 256, 0, st, g, cp, b.q, qo, b.psi, b.lc, modal_params<NZ>(*b.mc_h), b.sc))); break;
+        case 5: QGN_LAUNCH(KID_STAGE, nb, st, (::qgn::launch(k_ark_stage_small<5, NZ>, nbk, 256, 0, st, g, cp, b.q, qo, b.psi, b.lc, modal_params<NZ>(*b.mc_h), b.sc))); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -783,7 +716,7 @@ template <int S, int NZ, int NY>
 __device__ __forceinline__ void stage_yinv_col(const Geom& g, int kx, const CombPtrs<double2>& cp,
                                                const double2* __restrict__ q, double2* __restrict__ qout,
                                                double2* __restrict__ psi, const LayerConst* __restrict__ lc,
-                                               const ModalView& mv, const DevScalars* __restrict__ sc,
+                                               const ModalParams<NZ>& ma, const DevScalars* __restrict__ sc,
                                                double2* __restrict__ pq, double2* __restrict__ pv,
                                                double2* __restrict__ pu, const double2* __restrict__ twy,
                                                unsigned char* sm_raw) {
@@ -823,7 +756,7 @@ __device__ __forceinline__ void stage_yinv_col(const Geom& g, int kx, const Comb
             }
             qcol[l * nky + m] = qv[l];
         }
-        modal_invert_s<NZ>(mv.proj, mv.back, mv.ev, mv.Htot, NZ, k2, p == 0, qv, pvv);
+        modal_invert<NZ>(ma.proj, ma.back, ma.ev, ma.Htot, NZ, k2, p == 0, qv, pvv);
 #pragma unroll
         for (int l = 0; l < NZ; ++l) {
             psi[(size_t)l * P + p] = pvv[l];
@@ -861,13 +794,12 @@ __device__ __forceinline__ void stage_yinv_col(const Geom& g, int kx, const Comb
 template <int S, int NZ, int NY>
 __global__ void __launch_bounds__(StageYinvCfg<NY, NZ>::THREADS)
     k_stage_yinv(Geom g, CombPtrs<double2> cp, const double2* __restrict__ q, double2* __restrict__ qout,
-                 double2* __restrict__ psi, const LayerConst* __restrict__ lc, const __grid_constant__ ModalArg<NZ> ma,
+                 double2* __restrict__ psi, const LayerConst* __restrict__ lc, const __grid_constant__ ModalParams<NZ> ma,
                  const DevScalars* __restrict__ sc, double2* __restrict__ pq, double2* __restrict__ pv,
                  double2* __restrict__ pu, const double2* __restrict__ twy) {
     QGN_PDL_ENTRY();
     extern __shared__ __align__(16) unsigned char sm_raw[];
-    const ModalView mv = modal_view<NZ>(ma, nullptr, nullptr, nullptr, NZ);
-    stage_yinv_col<S, NZ, NY>(g, blockIdx.x, cp, q, qout, psi, lc, mv, sc, pq, pv, pu, twy, sm_raw);
+    stage_yinv_col<S, NZ, NY>(g, blockIdx.x, cp, q, qout, psi, lc, ma, sc, pq, pv, pu, twy, sm_raw);
 }
 
 // Stages 2..5 without quadratic drag: the y-forward pass that finishes N_{S-1} for column kx
@@ -879,14 +811,13 @@ __global__ void __launch_bounds__(StageYinvCfg<NY, NZ>::THREADS)
     k_yfwd_stage_yinv(Geom g, const double2* __restrict__ pp, const double2* __restrict__ qprev,
                       double2* __restrict__ nout, const double2* __restrict__ extra, CombPtrs<double2> cp,
                       const double2* __restrict__ q, double2* __restrict__ qout, double2* __restrict__ psi,
-                      const LayerConst* __restrict__ lc, const __grid_constant__ ModalArg<NZ> ma,
+                      const LayerConst* __restrict__ lc, const __grid_constant__ ModalParams<NZ> ma,
                       const DevScalars* __restrict__ sc, double2* __restrict__ pq, double2* __restrict__ pv,
                       double2* __restrict__ pu, const double2* __restrict__ twy) {
     QGN_PDL_ENTRY();
     using C = StageYinvCfg<NY, NZ>;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     double2* slots = reinterpret_cast<double2*>(sm_raw);
-    const ModalView mv = modal_view<NZ>(ma, nullptr, nullptr, nullptr, NZ);
     const int tid = threadIdx.x;
     const int kx = blockIdx.x;
     const int nky = g.nky;
@@ -937,7 +868,7 @@ __global__ void __launch_bounds__(StageYinvCfg<NY, NZ>::THREADS)
         }
     }
     __syncthreads();   // N_{S-1} of the column is written; the slots are free
-    stage_yinv_col<S, NZ, NY>(g, kx, cp, q, qout, psi, lc, mv, sc, pq, pv, pu, twy, sm_raw);
+    stage_yinv_col<S, NZ, NY>(g, kx, cp, q, qout, psi, lc, ma, sc, pq, pv, pu, twy, sm_raw);
 }
 
 // the (ny, nz) pairs built: a CTA keeps its registers without spilling
@@ -966,7 +897,7 @@ static cudaError_t stage_yinv_s(const Geom& g, const Buffers& b, cudaStream_t st
     const double Cb = 16.0 * (double)g.csize(), Hb = 16.0 * (double)g.nz * NY * g.nkx;
     const double nb = Cb * (S == 0 ? 2.0 : 2.0 * S + 2.0) + 3.0 * Hb;
     return stage_yinv_launch<NZ, NY>(g, k_stage_yinv<S, NZ, NY>, KID_STAGE, nb, st, g, comb_ptrs<double2>(b), b.q,
-                                     b.Qs[S], b.psi, b.lc, modal_arg<NZ>(b), b.sc, b.hq, b.hp, b.hu, b.twy);
+                                     b.Qs[S], b.psi, b.lc, modal_params<NZ>(*b.mc_h), b.sc, b.hq, b.hp, b.hu, b.twy);
 }
 
 template <int S, int NZ, int NY>
@@ -975,7 +906,7 @@ static cudaError_t yfwd_stage_yinv_s(const Geom& g, const Buffers& b, const doub
     const double nb = 2.0 * Hb + 3.0 * Cb + Cb * (2.0 * S + 2.0) + 3.0 * Hb;
     return stage_yinv_launch<NZ, NY>(g, k_yfwd_stage_yinv<S, NZ, NY>, KID_YFWD, nb, st, g, b.hpp, b.Qs[S - 1],
                                      b.N[S - 1], extra, comb_ptrs<double2>(b), b.q, b.Qs[S], b.psi, b.lc,
-                                     modal_arg<NZ>(b), b.sc, b.hq, b.hp, b.hu, b.twy);
+                                     modal_params<NZ>(*b.mc_h), b.sc, b.hq, b.hp, b.hu, b.twy);
 }
 
 // fused = false: stage s and its y-inverse; true: the y-forward of RHS s-1 as well (s = 2..5)
@@ -1047,20 +978,6 @@ cudaError_t launch_yfwd_stage_yinv(const Geom& g, const Buffers& b, int s, const
     return stage_yinv_dispatch(g, b, s, true, extra, st);
 }
 
-cudaError_t launch_modal_f32(const Geom& g, const Buffers& b, const float2* q, float2* psi, cudaStream_t st) {
-    const size_t P = (size_t)g.nkx * g.nky;
-    dim3 grid(blocks_for(P, 256));
-    const double nb = 16.0 * (double)g.csize();
-    switch (b.mc_h ? g.nz : 0) {
-        case 2: QGN_LAUNCH(KID_MODAL, nb, st, ::qgn::launch(k_modal_f32<2>, grid, 256, 0, st, g, modal_arg<2>(b), q, psi)); break;
-        case 4: QGN_LAUNCH(KID_MODAL, nb, st, ::qgn::launch(k_modal_f32<4>, grid, 256, 0, st, g, modal_arg<4>(b), q, psi)); break;
-        case 8: QGN_LAUNCH(KID_MODAL, nb, st, ::qgn::launch(k_modal_f32<8>, grid, 256, 0, st, g, modal_arg<8>(b), q, psi)); break;
-        case 16: QGN_LAUNCH(KID_MODAL, nb, st, ::qgn::launch(k_modal_f32<16>, grid, 256, 0, st, g, modal_arg<16>(b), q, psi)); break;
-        default: QGN_LAUNCH(KID_MODAL, nb, st, ::qgn::launch(k_modal_f32<0>, grid, 256, 0, st, g, modal_arg<0>(b), q, psi)); break;
-    }
-    return cudaGetLastError();
-}
-
 // stage s of ARK4(3)6L[2]SA: q_s (streaming combination), then psi_s = GetPsi(q_s)
 cudaError_t launch_ark_stage(const Geom& g, const Buffers& b, int s, cudaStream_t st) {
     if (g.csize() <= (size_t)(QGN_FUSED_STAGE_MAX) && b.mc_h) {
@@ -1101,21 +1018,6 @@ cudaError_t launch_ark_update_mixed(const Geom& g, const Buffers& b, cudaStream_
     return cudaGetLastError();
 }
 
-cudaError_t launch_modal_mixed(const Geom& g, const Buffers& b, const double2* q, float2* q32, float2* psi32,
-                               cudaStream_t st) {
-    const size_t P = (size_t)g.nkx * g.nky;
-    dim3 grid(blocks_for(P, 256));
-    const double nb = 32.0 * (double)g.csize();
-    switch (b.mc_h ? g.nz : 0) {
-        case 2: QGN_LAUNCH(KID_MODAL, nb, st, ::qgn::launch(k_modal_mixed<2>, grid, 256, 0, st, g, modal_arg<2>(b), q, q32, psi32)); break;
-        case 4: QGN_LAUNCH(KID_MODAL, nb, st, ::qgn::launch(k_modal_mixed<4>, grid, 256, 0, st, g, modal_arg<4>(b), q, q32, psi32)); break;
-        case 8: QGN_LAUNCH(KID_MODAL, nb, st, ::qgn::launch(k_modal_mixed<8>, grid, 256, 0, st, g, modal_arg<8>(b), q, q32, psi32)); break;
-        case 16: QGN_LAUNCH(KID_MODAL, nb, st, ::qgn::launch(k_modal_mixed<16>, grid, 256, 0, st, g, modal_arg<16>(b), q, q32, psi32)); break;
-        default: QGN_LAUNCH(KID_MODAL, nb, st, ::qgn::launch(k_modal_mixed<0>, grid, 256, 0, st, g, modal_arg<0>(b), q, q32, psi32)); break;
-    }
-    return cudaGetLastError();
-}
-
 cudaError_t launch_f2d(size_t n, const float2* a, double2* b, cudaStream_t st) {
     QGN_LAUNCH(KID_LAYOUT, 24.0 * (double)n, st, ::qgn::launch(k_f2d, blocks_for(n, 256), 256, 0, st, n, a, b));
     return cudaGetLastError();
@@ -1129,20 +1031,24 @@ cudaError_t launch_ark_update(const Geom& g, const Buffers& b, cudaStream_t st) 
     return cudaGetLastError();
 }
 
+// psi in the same launch for nz <= 8, where it saves reading q_tmp back (5 layers on 512 x 256:
+// 41.8 us in the generic form that kept 32 layers per thread in local memory)
 cudaError_t launch_combo(const Geom& g, const Buffers& b, const Combo& cb, const double2* q, double2* out,
                          double2* psi, bool want_psi, cudaStream_t st) {
-    const size_t P = (size_t)g.nkx * g.nky;
-    dim3 grid(blocks_for(P, 256));
-    const int wp = want_psi ? 1 : 0;
-    const double nb = 16.0 * (double)g.csize() * (1.0 + cb.n + 1.0 + wp);
-    switch (b.mc_h ? g.nz : 0) {
-        case 2: QGN_LAUNCH(KID_COMBO, nb, st, ::qgn::launch(k_combo<2>, grid, 256, 0, st, g, cb, q, out, psi, modal_arg<2>(b), b.sc, wp)); break;
-        case 4: QGN_LAUNCH(KID_COMBO, nb, st, ::qgn::launch(k_combo<4>, grid, 256, 0, st, g, cb, q, out, psi, modal_arg<4>(b), b.sc, wp)); break;
-        case 8: QGN_LAUNCH(KID_COMBO, nb, st, ::qgn::launch(k_combo<8>, grid, 256, 0, st, g, cb, q, out, psi, modal_arg<8>(b), b.sc, wp)); break;
-        case 16: QGN_LAUNCH(KID_COMBO, nb, st, ::qgn::launch(k_combo<16>, grid, 256, 0, st, g, cb, q, out, psi, modal_arg<16>(b), b.sc, wp)); break;
-        default: QGN_LAUNCH(KID_COMBO, nb, st, ::qgn::launch(k_combo<0>, grid, 256, 0, st, g, cb, q, out, psi, modal_arg<0>(b), b.sc, wp)); break;
+    const double C = 16.0 * (double)g.csize();
+    auto fused = [&](auto NZc) {
+        constexpr int NZ = decltype(NZc)::value;
+        ::qgn::launch(k_combo<NZ>, blocks_for((size_t)g.nkx * g.nky, 256), 256, 0, st, g, cb, q, out, psi,
+                      modal_params<NZ>(*b.mc_h), b.sc);
+    };
+    if (want_psi && g.nz <= 8) {
+        QGN_LAUNCH(KID_COMBO, C * (cb.n + 3.0), st, dispatch_small_nz(g.nz, fused));
+        return cudaGetLastError();
     }
-    return cudaGetLastError();
+    QGN_LAUNCH(KID_COMBO, C * (cb.n + 2.0), st,
+               ::qgn::launch(k_combo_stream, blocks_for(g.csize(), 256), 256, 0, st, g.csize(), cb, q, out, b.sc));
+    cudaError_t e = cudaGetLastError();
+    return e != cudaSuccess || !want_psi ? e : launch_modal(g, b, out, psi, st);
 }
 
 cudaError_t launch_lincomb(const Geom& g, const Combo& cb, double2* out, cudaStream_t st) {
