@@ -53,21 +53,22 @@ template <int NX, bool DRAG, class CT, int TV = 0>
 __global__ void __launch_bounds__(XCfg<NX, DRAG, CT, TV>::THREADS,
                                   minb(XCfg<NX, DRAG, CT, TV>::THREADS,
                                        XCfg<NX, DRAG, CT, TV>::TP == 32 ? (sizeof(CT) == 16 ? 168 : 112) : regcap<CT>(NX >= 1024 ? 112 : 128, 80)))
-    k_xpass(Geom g, int layer0, const CT* __restrict__ pq, const CT* __restrict__ pv,
+    k_xpass(Geom g, const CT* __restrict__ pq, const CT* __restrict__ pv,
             const CT* __restrict__ pu, CT* __restrict__ pp, CT* __restrict__ pd,
             const CT* __restrict__ twx) {
     QGN_PDL_ENTRY();
-    xpass_tile<NX, DRAG, CT, TV>(g, blockIdx.x, layer0 + blockIdx.y, pq, pv, pu, pp, pd, twx);
+    xpass_tile<NX, DRAG, CT, TV>(g, blockIdx.x, blockIdx.y, pq, pv, pu, pp, pd, twx);
 }
 
 template <int NY, bool DRAG, class CT, int TV = 0>
 __global__ void __launch_bounds__(YFwdCfg<NY, DRAG, CT, TV>::THREADS,
                                   minb(YFwdCfg<NY, DRAG, CT, TV>::THREADS, YFwdCfg<NY, DRAG, CT, TV>::TP == 8 ? 64 : regcap<CT>()))
-    k_yfwd(Geom g, int layer0, const LayerConst* __restrict__ lc, const CT* __restrict__ q,
+    k_yfwd(Geom g, const LayerConst* __restrict__ lc, const CT* __restrict__ q,
            const CT* __restrict__ psi, const CT* __restrict__ pp, const CT* __restrict__ pd,
            CT* __restrict__ out, const CT* __restrict__ twy, const CT* __restrict__ extra) {
     QGN_PDL_ENTRY();
-    yfwd_tile<NY, DRAG, CT, TV>(g, blockIdx.x, layer0 + blockIdx.y, lc, q, psi, pp, pd, out, twy, extra);
+    // with drag, the bottom layer's tiles transform twice: they go first
+    yfwd_tile<NY, DRAG, CT, TV>(g, blockIdx.x, DRAG ? g.nz - 1 - blockIdx.y : blockIdx.y, lc, q, psi, pp, pd, out, twy, extra);
 }
 
 template <int NX, int EPI, int TV = 0, class CT = double2>
@@ -222,15 +223,15 @@ static cudaError_t launch_yinv(const Geom& g, int nf, const CT* q, const CT* psi
 }
 
 template <int NX, bool DRAG, class CT, int TV>
-static cudaError_t xpass_go(const Geom& g, int layer0, int layers, const CT* hq, const CT* hp, const CT* hu, CT* hpp,
-                            CT* hpd, const CT* twx, cudaStream_t s) {
+static cudaError_t xpass_go(const Geom& g, const CT* hq, const CT* hp, const CT* hu, CT* hpp, CT* hpd, const CT* twx,
+                            cudaStream_t s) {
     using C = XCfg<NX, DRAG, CT, TV>;
     cudaError_t e;
     if ((e = set_smem(k_xpass<NX, DRAG, CT, TV>, C::SMEM)) != cudaSuccess) return e;
-    dim3 grid((g.ny / 2 + C::RP - 1) / C::RP, layers);
+    dim3 grid((g.ny / 2 + C::RP - 1) / C::RP, g.nz + (DRAG ? 1 : 0));
     const double es = (double)sizeof(CT);
-    QGN_LAUNCH(KID_XPASS, (DRAG ? 7.0 : 5.0) * es * (double)layers * g.ny * g.nkx, s,
-               ::qgn::launch(k_xpass<NX, DRAG, CT, TV>, grid, C::THREADS, C::SMEM, s, g, layer0, hq, hp, hu, hpp, hpd, twx));
+    QGN_LAUNCH(KID_XPASS, (5.0 * g.nz + (DRAG ? 4.0 : 0.0)) * es * (double)g.ny * g.nkx, s,
+               ::qgn::launch(k_xpass<NX, DRAG, CT, TV>, grid, C::THREADS, C::SMEM, s, g, hq, hp, hu, hpp, hpd, twx));
     return cudaGetLastError();
 }
 
@@ -239,46 +240,30 @@ static cudaError_t launch_xpass(const Geom& g, const CT* hq, const CT* hp, const
                                 bool drag, cudaStream_t s) {
     return dispatch_n(g.nx, [&](auto NXc) -> cudaError_t {
         constexpr int NX = decltype(NXc)::value;
-        cudaError_t e;
-        const int nplain = drag ? g.nz - 1 : g.nz;
-        bool narrow = false;
         if constexpr (has_narrow<NX>()) {
             const long long cd = (long long)((g.ny / 2 + XCfg<NX, false, CT>::RP - 1) / XCfg<NX, false, CT>::RP) * g.nz;
             const long long cn =
                 (long long)((g.ny / 2 + XCfg<NX, false, CT, kNarrowX>::RP - 1) / XCfg<NX, false, CT, kNarrowX>::RP) *
                 g.nz;
-            narrow = narrow_better(cd, cn);
+            if (narrow_better(cd, cn))
+                return drag ? xpass_go<NX, true, CT, kNarrowX>(g, hq, hp, hu, hpp, hpd, twx, s)
+                            : xpass_go<NX, false, CT, kNarrowX>(g, hq, hp, hu, hpp, hpd, twx, s);
         }
-        if (nplain > 0) {
-            if constexpr (has_narrow<NX>())
-                e = narrow ? xpass_go<NX, false, CT, kNarrowX>(g, 0, nplain, hq, hp, hu, hpp, hpd, twx, s)
-                           : xpass_go<NX, false, CT, 0>(g, 0, nplain, hq, hp, hu, hpp, hpd, twx, s);
-            else
-                e = xpass_go<NX, false, CT, 0>(g, 0, nplain, hq, hp, hu, hpp, hpd, twx, s);
-            if (e != cudaSuccess) return e;
-        }
-        if (drag) {
-            if constexpr (has_narrow<NX>())
-                e = narrow ? xpass_go<NX, true, CT, kNarrowX>(g, g.nz - 1, 1, hq, hp, hu, hpp, hpd, twx, s)
-                           : xpass_go<NX, true, CT, 0>(g, g.nz - 1, 1, hq, hp, hu, hpp, hpd, twx, s);
-            else
-                e = xpass_go<NX, true, CT, 0>(g, g.nz - 1, 1, hq, hp, hu, hpp, hpd, twx, s);
-            if (e != cudaSuccess) return e;
-        }
-        return cudaSuccess;
+        return drag ? xpass_go<NX, true, CT, 0>(g, hq, hp, hu, hpp, hpd, twx, s)
+                    : xpass_go<NX, false, CT, 0>(g, hq, hp, hu, hpp, hpd, twx, s);
     });
 }
 
 template <int NY, bool DRAG, class CT, int TV>
-static cudaError_t yfwd_go(const Geom& g, int layer0, int layers, const LayerConst* lc, const CT* q, const CT* psi,
-                           const CT* hpp, const CT* hpd, CT* out, const CT* twy, const CT* extra, cudaStream_t s) {
+static cudaError_t yfwd_go(const Geom& g, const LayerConst* lc, const CT* q, const CT* psi, const CT* hpp, const CT* hpd,
+                           CT* out, const CT* twy, const CT* extra, cudaStream_t s) {
     using C = YFwdCfg<NY, DRAG, CT, TV>;
     cudaError_t e;
     if ((e = set_smem(k_yfwd<NY, DRAG, CT, TV>, C::SMEM)) != cudaSuccess) return e;
-    dim3 grid((g.nkx + C::TKX - 1) / C::TKX, layers);
-    const double lb = (double)sizeof(CT) * (double)layers * g.nkx;
-    QGN_LAUNCH(KID_YFWD, lb * ((DRAG ? 4.0 : 2.0) * NY + 3.0 * g.nky), s,
-               ::qgn::launch(k_yfwd<NY, DRAG, CT, TV>, grid, C::THREADS, C::SMEM, s, g, layer0, lc, q, psi, hpp, hpd, out, twy,
+    dim3 grid((g.nkx + C::TKX - 1) / C::TKX, g.nz);
+    const double lb = (double)sizeof(CT) * g.nkx;
+    QGN_LAUNCH(KID_YFWD, lb * (g.nz * (2.0 * NY + 3.0 * g.nky) + (DRAG ? 2.0 * NY : 0.0)), s,
+               ::qgn::launch(k_yfwd<NY, DRAG, CT, TV>, grid, C::THREADS, C::SMEM, s, g, lc, q, psi, hpp, hpd, out, twy,
                                                                           extra));
     return cudaGetLastError();
 }
@@ -289,32 +274,16 @@ static cudaError_t launch_yfwd(const Geom& g, const LayerConst* lc, const CT* q,
                                const CT* extra = nullptr) {
     return dispatch_n(g.ny, [&](auto NYc) -> cudaError_t {
         constexpr int NY = decltype(NYc)::value;
-        cudaError_t e;
-        const int nplain = drag ? g.nz - 1 : g.nz;
-        bool narrow = false;
         if constexpr (has_narrow<NY>()) {
             using D = YFwdCfg<NY, false, CT>;
             using Nn = YFwdCfg<NY, false, CT, kNarrowY>;
-            narrow = narrow_better((long long)((g.nkx + D::TKX - 1) / D::TKX) * g.nz,
-                                   (long long)((g.nkx + Nn::TKX - 1) / Nn::TKX) * g.nz);
+            if (narrow_better((long long)((g.nkx + D::TKX - 1) / D::TKX) * g.nz,
+                              (long long)((g.nkx + Nn::TKX - 1) / Nn::TKX) * g.nz))
+                return drag ? yfwd_go<NY, true, CT, kNarrowY>(g, lc, q, psi, hpp, hpd, out, twy, extra, s)
+                            : yfwd_go<NY, false, CT, kNarrowY>(g, lc, q, psi, hpp, hpd, out, twy, extra, s);
         }
-        if (nplain > 0) {
-            if constexpr (has_narrow<NY>())
-                e = narrow ? yfwd_go<NY, false, CT, kNarrowY>(g, 0, nplain, lc, q, psi, hpp, hpd, out, twy, extra, s)
-                           : yfwd_go<NY, false, CT, 0>(g, 0, nplain, lc, q, psi, hpp, hpd, out, twy, extra, s);
-            else
-                e = yfwd_go<NY, false, CT, 0>(g, 0, nplain, lc, q, psi, hpp, hpd, out, twy, extra, s);
-            if (e != cudaSuccess) return e;
-        }
-        if (drag) {
-            if constexpr (has_narrow<NY>())
-                e = narrow ? yfwd_go<NY, true, CT, kNarrowY>(g, g.nz - 1, 1, lc, q, psi, hpp, hpd, out, twy, extra, s)
-                           : yfwd_go<NY, true, CT, 0>(g, g.nz - 1, 1, lc, q, psi, hpp, hpd, out, twy, extra, s);
-            else
-                e = yfwd_go<NY, true, CT, 0>(g, g.nz - 1, 1, lc, q, psi, hpp, hpd, out, twy, extra, s);
-            if (e != cudaSuccess) return e;
-        }
-        return cudaSuccess;
+        return drag ? yfwd_go<NY, true, CT, 0>(g, lc, q, psi, hpp, hpd, out, twy, extra, s)
+                    : yfwd_go<NY, false, CT, 0>(g, lc, q, psi, hpp, hpd, out, twy, extra, s);
     });
 }
 

@@ -101,7 +101,7 @@ struct XCfg {
     static constexpr int TP = fft_tp<CT, NX, TV>();
     static constexpr int G = FFTShape<NX, TP>::G;
     static constexpr int RP = (TV == 0 && G == 32) ? QGN_X_ROWPAIRS : cmax(1, (TV == 0 ? 64 : tv_width(TV)) / G);   // row pairs per CTA
-    static constexpr int SP = DRAG ? 4 : 3;             // slots per row pair
+    static constexpr int SP = 3;                        // slots per row pair
     static constexpr int THREADS = SP * RP * G;
     static constexpr int TS = slot_stride(NX, 2, (int)sizeof(CT), TP);
     static constexpr int SMEM = SP * RP * TS * (int)sizeof(CT);
@@ -183,20 +183,9 @@ __device__ __forceinline__ CT pack_hi(CT f1, CT f2) {
 }
 
 // Layout of the forward x transforms P[k] (part 0) and P[nx-k] (part 1) of every row y: the x
-// pass's output, the forward y pass's input.  QGN_P_TILED (default 1): tiles of two kx columns,
-// [nz][nkxp/2][ny][2 parts][2 columns], so that the rows of one column pair are contiguous and a
-// warp of the y-forward pass (8 rows x 2 columns x 2 parts) reads 512 contiguous bytes; the
-// x pass's stores of one row scatter over the tiles instead (stores are not waited for).
-// QGN_P_TILED 0: rows [nz][ny][2 parts][nkxp].  Both hold 2 nz ny nkxp elements.
-#ifndef QGN_P_TILED
-#define QGN_P_TILED 0
-#endif
+// pass's output, the forward y pass's input: rows [nz][ny][2 parts][nkxp], 2 nz ny nkxp elements.
 __host__ __device__ __forceinline__ size_t p_index(const Geom& g, int l, int y, int part, int k) {
-#if QGN_P_TILED
-    return ((size_t)(l * (g.nkxp >> 1) + (k >> 1)) * g.ny + y) * 4 + part * 2 + (k & 1);
-#else
     return ((size_t)l * g.ny + y) * 2 * g.nkxp + (size_t)part * g.nkxp + k;
-#endif
 }
 
 // ------------------------------------------------------------------------------------
@@ -366,9 +355,15 @@ __device__ __forceinline__ void yinv_tile(const Geom g, int bx, int l, const CT*
 // ~1e4 in these units), physical products formed inside the first pass of the forward
 // transforms, r2c of p = uq + i vq per row, whose last pass writes P[k] and P[nx-k] for the
 // kept kx straight to HBM.
+//
+// Quadratic drag (DRAG) adds the transforms of |u|u + i |u|v of the bottom layer (QGN_Module.f90:
+// 284-292).  They are tiles of a layer of their own, l = nz, in the same launch: such a tile
+// transforms u and v of the bottom layer once more (its q slot idles), turns them in place into
+// |u|u and |u|v and runs the same forward transforms.  A second launch for the bottom layer alone,
+// which it replaces, was 15 us of latency per right-hand side (64 CTAs at 512^2).
 // ------------------------------------------------------------------------------------
 template <int NX, bool DRAG, class CT, int TV = 0>
-__device__ __forceinline__ void xpass_tile(const Geom g, int bx, int l, const CT* __restrict__ pq,
+__device__ __forceinline__ void xpass_tile(const Geom g, int bx, int layer, const CT* __restrict__ pq,
                                            const CT* __restrict__ pv, const CT* __restrict__ pu,
                                            CT* __restrict__ pp, CT* __restrict__ pd, const CT* __restrict__ twx) {
     using C = XCfg<NX, DRAG, CT, TV>;
@@ -382,6 +377,8 @@ __device__ __forceinline__ void xpass_tile(const Geom g, int bx, int l, const CT
     const int r_of = slot / C::SP, s_of = slot % C::SP;
     const int rp = bx * C::RP + r_of;
     const bool pair_ok = rp < npairs;
+    const bool drag = DRAG && layer == g.nz;   // this tile makes the drag fields of the bottom layer
+    const int l = drag ? g.nz - 1 : layer;
     CT* base = sm + (r_of * C::SP) * C::TS;
     CT* xs = sm + slot * C::TS;
 
@@ -401,29 +398,33 @@ __device__ __forceinline__ void xpass_tile(const Geom g, int bx, int l, const CT
         plane[x] = v.x;
         plane[C::TS + x] = v.y;
     };
-    fft_fused<NX, +1, SRC_FN, DST_SMEM_STORE, C::TP, (C::G <= 32)>(xs, lane, pair_ok && s_of < 3, twx, ld_inv,
-                                                                     st_inv);
+    fft_fused<NX, +1, SRC_FN, DST_SMEM_STORE, C::TP, (C::G <= 32)>(xs, lane, pair_ok && !(drag && s_of == 0), twx,
+                                                                     ld_inv, st_inv);
 
     // ---- forward: slot 0 = u1 q1 + i v1 q1, 1 = u2 q2 + i v2 q2 (grid/(nx*ny) scaling as in
-    //      QGN_Module.f90:229-235); with drag 2 = |u1|u1 + i|u1|v1, 3 = |u2|u2 + i|u2|v2
+    //      QGN_Module.f90:229-235); a drag tile |u1|u1 + i|u1|v1 and |u2|u2 + i|u2|v2
     const RT sc = (RT)g.inv_nxny;
     const RT sc2 = sc * sc;   // nx, ny are powers of two: u (q sc^2) == (u sc)(q sc) exactly
     // this slot's row in the planes of the q, u, v slots (RT offsets 0, 2 TS, 4 TS)
     const RT* rows = reinterpret_cast<const RT*>(base) + ((s_of & 1) ? C::TS : 0);
-    auto ld_fwd = [&](int x) -> CT {
-        if (s_of < 2) {
-            const RT qs = rows[x] * sc2;
-            return cmk<CT>(rows[2 * C::TS + x] * qs, rows[4 * C::TS + x] * qs);
+    if (drag) {   // u, v -> |u|u, |u|v in place (URMS, QGN_Module.f90:285)
+        for (int e = tid; e < C::RP * 2 * NX; e += C::THREADS) {
+            RT* pl = reinterpret_cast<RT*>(sm + (e / (2 * NX)) * C::SP * C::TS) + ((e / NX) & 1) * C::TS + e % NX;
+            const RT uv = pl[2 * C::TS] * sc, vv = pl[4 * C::TS] * sc;
+            const RT m = sqrt(uv * uv + vv * vv);
+            pl[2 * C::TS] = m * uv;
+            pl[4 * C::TS] = m * vv;
         }
-        const RT uv = rows[2 * C::TS + x] * sc;
-        const RT vv = rows[4 * C::TS + x] * sc;
-        const RT m = sqrt(uv * uv + vv * vv);   // URMS, QGN_Module.f90:285
-        return cmk<CT>(m * uv, m * vv);
+        __syncthreads();
+    }
+    auto ld_fwd = [&](int x) -> CT {
+        const RT qs = drag ? (RT)1 : rows[x] * sc2;
+        return cmk<CT>(rows[2 * C::TS + x] * qs, rows[4 * C::TS + x] * qs);
     };
     const int y = 2 * rp + (s_of & 1);
-    const int ol = (s_of < 2) ? l : 0;                                              // pd holds one layer
-    const size_t olen = (s_of < 2) ? 2 * g.hsize() : (size_t)g.ny * 2 * g.nkxp;   // pp, or pd
-    CT* out = (s_of < 2) ? pp : pd;
+    const int ol = drag ? 0 : l;                                                 // pd holds one layer
+    const size_t olen = drag ? (size_t)g.ny * 2 * g.nkxp : 2 * g.hsize();   // pd, or pp
+    CT* out = drag ? pd : pp;
     auto st_fwd = [&](int k, CT v) {
         if (k < nkx) {
             const size_t i = p_index(g, ol, y, 0, k);
@@ -433,41 +434,7 @@ __device__ __forceinline__ void xpass_tile(const Geom g, int bx, int l, const CT
             if (in_bounds(g, i, olen)) out[i] = v;
         }
     };
-#if QGN_P_TILED
-    // Tiled layout: the last radix pass leaves the kept outputs in the transform's own slot
-    // (P[k] at k, P[nx-k] at nkxp + k; the dealiased band's outputs on the slot's last element),
-    // and the whole CTA then writes each kx column pair's values of its rows as one contiguous
-    // run: with one row pair per CTA, rows 2p and 2p+1 of a tile are adjacent, 8 values = 128 B.
-    if (2 * g.nkxp < C::TS - 1) {   // the kept outputs fit below the spare element (uniform)
-        auto omap = [&](int k) -> int {
-            if (k < nkx) return k;
-            if (k > NX - nkx) return g.nkxp + (NX - k);
-            return C::TS - 1;
-        };
-        fft_fused<NX, -1, SRC_FN_SMEM, DST_SMEM_MAP, C::TP, (C::G <= 32)>(xs, lane, pair_ok && s_of < (DRAG ? 4 : 2),
-                                                                             twx, ld_fwd, omap);
-        // fft_fused ended with a block-wide barrier: every slot holds its row's outputs
-        const int T = g.nkxp >> 1;
-        for (int dr = 0; dr < (DRAG ? 2 : 1); ++dr) {   // dr 0: uq + i vq into pp; 1: drag fields into pd
-            CT* o = dr == 0 ? pp : pd;
-            const int ol2 = dr == 0 ? l : 0;
-            const size_t olen2 = dr == 0 ? 2 * g.hsize() : (size_t)g.ny * 2 * g.nkxp;
-            for (int e = tid; e < C::RP * T * 8; e += C::THREADS) {
-                const int r = e / (T * 8), rem = e % (T * 8);
-                const int t = rem >> 3, w = rem & 7;
-                const int rr = w >> 2, part = (w >> 1) & 1, k = 2 * t + (w & 1);
-                const int rpp = bx * C::RP + r;
-                if (rpp >= npairs || k >= nkx || (part == 1 && k == 0)) continue;
-                const CT* src = sm + (r * C::SP + 2 * dr + rr) * C::TS;
-                const size_t i = p_index(g, ol2, 2 * rpp + rr, part, k);
-                if (in_bounds(g, i, olen2)) o[i] = src[part * g.nkxp + k];
-            }
-        }
-        return;
-    }
-#endif
-    fft_fused<NX, -1, SRC_FN_SMEM, DST_FN, C::TP, (C::G <= 32)>(xs, lane, pair_ok && s_of < (DRAG ? 4 : 2), twx, ld_fwd,
-                                                                   st_fwd);
+    fft_fused<NX, -1, SRC_FN_SMEM, DST_FN, C::TP, (C::G <= 32)>(xs, lane, pair_ok && s_of < 2, twx, ld_fwd, st_fwd);
 }
 
 // ------------------------------------------------------------------------------------
@@ -523,7 +490,7 @@ __device__ __forceinline__ void yfwd_tile(const Geom g, int bx, int l, const Lay
     // would split across one bank group twice
     auto omap = [](int y) { return y; };
 
-    if (DRAG) {
+    if (DRAG && bottom) {
         // drag_hat = i ky (|u|u)^ - i kx (|u|v)^ on the bottom layer (QGN_Module.f90:284-292)
         auto ldd = [&](int y) -> CT {
             const size_t i = p_index(g, 0, y, fld, kx0 + c);
