@@ -12,9 +12,9 @@
 //
 // Kernels (one CTA = 8 warps = 128 consecutive pixels of one image row, persistent over rows):
 //   k_conv<CIN,COUT,EPI>  implicit GEMM  out[p, n] = sum_{tap, k} in[p + tap, k] w[tap, n, k]
-//                         EPI_GELU:      Z = acc + bias (FP32), A = bf16(GELU(Z))
+//                         EPI_GELU:      A = bf16(GELU(Z)), D = GELU'(Z) (FP32), Z = acc + bias
 //                         EPI_LINEAR:    Y = acc + bias (FP32)
-//                         EPI_GELU_GRAD: G = bf16(acc * GELU'(Z))   (backward through a layer)
+//                         EPI_GELU_GRAD: G = bf16(acc * D)   (backward through a layer)
 //   k_wgrad<CIN,COUT>     dW[tap, n, k] partials = sum_p G[p, n] in[p + tap, k] per row chunk
 //   k_reduce_*            deterministic chunk sums of dW and the bias gradient
 //   k_mse                 loss and dL/dY = 2 (Y - T)/count, as BF16 G of the last layer
@@ -43,17 +43,22 @@ namespace cnn {
 constexpr int kTileP = 128;          // pixels per CTA tile (one row segment)
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
-// Warps of the tcgen05 convolutions (one CTA per SM either way: shared memory).  The fused
-// small-batch inference has one tile per CTA and per layer, with nothing to overlap its epilogue
-// (TMEM loads, bias, GELU, BF16 packing, staged stores), so 16 warps each drain 16 accumulator
-// columns: the 128^2 batch-1 inference ran 58.2 -> 53.7 us on B200.  The persistent layer kernel
-// overlaps each tile's epilogue with the next tile's MMAs and stays at 8 warps (16 made the
-// batch-32 forward 231 -> 228 TFLOP/s and a training step 3.92 -> 4.06 ms).
-constexpr int kTcWarps = 8;
-constexpr int kTcThreads = kTcWarps * 32;
+// Warps of the fused small-batch inference (one CTA per SM: shared memory).  It has one tile per
+// CTA and per layer, with nothing to overlap its epilogue (TMEM loads, bias, GELU, BF16 packing,
+// staged stores), so 16 warps each drain 16 accumulator columns: the 128^2 batch-1 inference ran
+// 58.2 -> 53.7 us on B200.
 constexpr int kFusedWarps = 16;
 constexpr int kFusedThreads = kFusedWarps * 32;
-constexpr int kWChunkRows = 16;      // image rows per weight-gradient partial
+// Warps of the layer kernels k_conv_tc and k_wgrad_tc, by role: accumulator drain, row loads, and
+// one that issues the MMAs.  Twelve in all, three per sub-partition: up to 168 registers a thread
+// (a thirteenth would leave 128).
+constexpr int kEpiWarps = 8;
+constexpr int kLoadWarps = 3;
+constexpr int kLoadThreads = kLoadWarps * 32;
+constexpr int kRoleThreads = (kEpiWarps + kLoadWarps + 1) * 32;
+constexpr int kMseThreads = 1024;
+constexpr int kWChunkRows = 16;      // image rows summed in the accumulators before they are added up in FP32
+constexpr int kWgChunks = 49;        // row ranges of the tcgen05 weight gradient: 3 x 49 CTAs
 
 // EPI_PLANAR: as EPI_LINEAR but the FP32 output is planar, out[n][pixel] (the closure's input
 // to its forward transform)
@@ -117,7 +122,7 @@ template <int CIN, int COUT, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
     k_conv(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wt, const float* __restrict__ bias,
            int B, int H, int W, float* __restrict__ outf, __nv_bfloat16* __restrict__ outb,
-           const float* __restrict__ zin) {
+           const float* __restrict__ dact) {
     QGN_PDL_ENTRY();
     static_assert(CIN % 16 == 0 && COUT % 16 == 0, "channel counts are padded to 16");
     constexpr int LDI = RowPad<CIN>::LD;
@@ -184,17 +189,21 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const size_t np = (size_t)B * H * W;
                     outf[(size_t)n * np + p] = v0 + bias[n];
                     outf[(size_t)(n + 1) * np + p] = v1 + bias[n + 1];
-                } else if (EPI == EPI_GELU || EPI == EPI_LINEAR) {
+                } else if (EPI == EPI_GELU || EPI == EPI_LINEAR || EPI == EPI_GELU_ACT) {
                     v0 += bias[n];
                     v1 += bias[n + 1];
-                    *reinterpret_cast<float2*>(outf + p * COUT + n) = make_float2(v0, v1);
-                    if (EPI == EPI_GELU)
+                    if (EPI == EPI_GELU || EPI == EPI_GELU_ACT) {
+                        if (EPI == EPI_GELU)
+                            *reinterpret_cast<float2*>(outf + p * COUT + n) =
+                                make_float2(gelu_grad(v0), gelu_grad(v1));
                         *reinterpret_cast<__nv_bfloat162*>(outb + p * COUT + n) =
                             __floats2bfloat162_rn(gelu(v0), gelu(v1));
+                    } else {
+                        *reinterpret_cast<float2*>(outf + p * COUT + n) = make_float2(v0, v1);
+                    }
                 } else {
-                    const float2 z = *reinterpret_cast<const float2*>(zin + p * COUT + n);
-                    *reinterpret_cast<__nv_bfloat162*>(outb + p * COUT + n) =
-                        __floats2bfloat162_rn(v0 * gelu_grad(z.x), v1 * gelu_grad(z.y));
+                    const float2 d = *reinterpret_cast<const float2*>(dact + p * COUT + n);
+                    *reinterpret_cast<__nv_bfloat162*>(outb + p * COUT + n) = __floats2bfloat162_rn(v0 * d.x, v1 * d.y);
                 }
             }
         }
@@ -283,6 +292,7 @@ __global__ void k_reduce_wgrad(const float* __restrict__ part, int nchunks, int 
     QGN_PDL_ENTRY();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float s = 0.f;
+#pragma unroll 8
         for (int c = 0; c < nchunks; ++c) s += part[(size_t)c * n + i];
         dw[i] = s;
     }
@@ -301,22 +311,31 @@ __global__ void k_bias_part(const __nv_bfloat16* __restrict__ gr, long long npix
     }
 }
 
-// MSE over the real output channels; G = bf16(2 (Y - T) / count), zero in padded channels
-__global__ void k_mse(const float* __restrict__ y, const float* __restrict__ tgt, long long npix, int C, int creal,
+// MSE over the real output channels; G = bf16(2 (Y - T) / count), zero in padded channels.  One
+// thread per four channels of a pixel: 16-byte loads, none of them for padded groups.
+__global__ void __launch_bounds__(kMseThreads) k_mse(const float* __restrict__ y, const float* __restrict__ tgt, long long npix, int C, int creal,
                       double inv_count, __nv_bfloat16* __restrict__ g, double* __restrict__ loss_part) {
     QGN_PDL_ENTRY();
-    __shared__ double red[kThreads / 32];
+    __shared__ double red[kMseThreads / 32];
     double s = 0.0;
-    const long long n = npix * C;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % C);
-        float gv = 0.f;
-        if (c < creal) {
-            const float d = y[i] - tgt[i];
-            s += (double)d * (double)d;
-            gv = (float)(2.0 * inv_count) * d;
+    const float gs = (float)(2.0 * inv_count);
+    const long long n4 = npix * (C / 4);
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+        const int c0 = 4 * (int)((unsigned long long)i % (unsigned)(C / 4));
+        float gv[4] = {0.f, 0.f, 0.f, 0.f};
+        if (c0 < creal) {
+            const float4 a = reinterpret_cast<const float4*>(y)[i], b = reinterpret_cast<const float4*>(tgt)[i];
+            const float d[4] = {a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (c0 + k < creal) {
+                    s += (double)d[k] * (double)d[k];
+                    gv[k] = gs * d[k];
+                }
+            }
         }
-        g[i] = __float2bfloat16_rn(gv);
+        __nv_bfloat162 o[2] = {__floats2bfloat162_rn(gv[0], gv[1]), __floats2bfloat162_rn(gv[2], gv[3])};
+        reinterpret_cast<uint2*>(g)[i] = *reinterpret_cast<const uint2*>(o);
     }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = s;
@@ -399,15 +418,14 @@ __global__ void k_gather(const unsigned char* __restrict__ src, const int* __res
 //               (dh, dw) starts at pixel dw of the slot holding row h+dh-1: rows (pixels) 16 B
 //               apart, 8-row groups 128 B apart (SBO), the two halves of a K step 130*16 B apart (LBO);
 //   weights     [9 taps][CIN/8 chunks][COUT][8]: SBO 128 B, LBO COUT*16 B.
-// Each CTA takes a contiguous range of tiles ordered row-fastest, so consecutive tiles share two
-// of their three input rows: one new row per tile, fetched with cp.async into the free ring slot
-// while the current tile's MMAs run.  Completion is signalled by tcgen05.commit on an mbarrier;
-// every wait is bounded, and a wait that runs out records an error, waits once more, frees the
-// TMEM and returns.
+// Each CTA takes a contiguous range of tiles ordered row-fastest, so consecutive tiles of a column
+// of rows share two of their three input rows: one new row per tile.  Completion is signalled by
+// tcgen05.commit on mbarriers; every wait is bounded, and a wait that runs out records an error,
+// waits once more for the MMAs in flight, frees the TMEM and returns.
 namespace tc {
 
 constexpr int kPixS = kTileP + 2;        // staged pixels per input row (periodic halo)
-constexpr int kSlots = 6;                // input-row ring: rows of the tile in flight and the next
+constexpr int kSlots = 6;                // input-row ring of the layer kernel
 constexpr long long kWaitLimit = 1LL << 22;
 
 constexpr int imax(int a, int b) { return a > b ? a : b; }
@@ -426,10 +444,9 @@ struct Lay {
     static constexpr int B_LAST = W_OFF + (8 * (CIN / 8) + CIN / 8 - 2) * COUT * 16;
     static constexpr int A_END = A_LAST + imax(kPixS * 16 + 15 * 128, 15 * kPixS * 16 + 128) + 128;
     static constexpr int B_END = B_LAST + imax(COUT * 16 + (COUT / 8 - 1) * 128, (COUT / 8 - 1) * COUT * 16 + 128) + 128;
-    static constexpr int OPS_END = (imax(BAR_OFF + 64, imax(A_END, B_END)) + 1023) / 1024 * 1024;
-    static constexpr int STF_OFF = OPS_END;                         // FP32 output staging [128][COUT]
-    static constexpr int STB_OFF = STF_OFF + kTileP * COUT * 4;     // BF16 output staging [128][COUT]
-    static constexpr int SMEM = STB_OFF + kTileP * COUT * 2;
+    static constexpr int OPS_END = (imax(BAR_OFF + 256, imax(A_END, B_END)) + 1023) / 1024 * 1024;
+    static constexpr int STG_OFF = OPS_END;                 // output staging, 4 KB per epilogue warp
+    static constexpr int SMEM = STG_OFF + kEpiWarps * 4096;
     static constexpr int TMEM_COLS = COUT < 32 ? 64 : 2 * COUT;   // two accumulator tiles, power of two
 };
 
@@ -463,6 +480,34 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
         if (ok) return true;
     }
     return false;
+}
+
+// bounded wait of one role of a layer kernel; gives up at once when another role has.  False: the
+// role leaves its loop (and so, through the flag, do the others).
+__device__ __forceinline__ bool role_wait(uint32_t bar, uint32_t parity, volatile int* gave_up) {
+    for (long long i = 0; i < kWaitLimit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if (*gave_up) return false;
+    }
+    *gave_up = 1;
+    return false;
+}
+__device__ __forceinline__ void arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void bar_init(uint32_t bar, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
 }
 
 __device__ __forceinline__ void cp16(uint32_t saddr, const void* g) {
@@ -507,8 +552,7 @@ __device__ __forceinline__ void issue_tile(uint32_t dacc, const uint32_t* ra, ui
                 idesc<COUT>(), (tap | kc) ? 1u : 0u);
         }
     }
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar)
-                 : "memory");
+    commit(bar);
 }
 
 // a layer's weights [9][COUT][CIN] (BF16) into the K-major operand layout [9][CIN/8][COUT][8];
@@ -526,9 +570,9 @@ __device__ __forceinline__ void fetch_weights(const __nv_bfloat16* __restrict__ 
 // one input row (image b, row hh, pixels w0-1 .. w0+128 periodic) into a ring slot, asynchronously
 template <int CIN, int NT>
 __device__ __forceinline__ void fetch_row(const __nv_bfloat16* __restrict__ x, int b, int hh, int H, int W, int w0,
-                                         uint32_t slot_addr) {
+                                         uint32_t slot_addr, int tid) {
     const size_t row = ((size_t)b * H + hh) * W;
-    for (int i = threadIdx.x; i < kPixS * (CIN / 8); i += NT) {
+    for (int i = tid; i < kPixS * (CIN / 8); i += NT) {
         const int c8 = i % (CIN / 8), px = i / (CIN / 8);
         int ww = w0 - 1 + px;   // in [-1, W]: one periodic wrap at either end
         ww = ww < 0 ? ww + W : (ww >= W ? ww - W : ww);
@@ -538,7 +582,7 @@ __device__ __forceinline__ void fetch_row(const __nv_bfloat16* __restrict__ x, i
 
 }  // namespace tc
 
-// Epilogue of one tile: warp w reads TMEM lanes 32 (w % 4).. (one pixel per thread) and a block
+// Epilogue of one tile of the fused inference: warp w reads TMEM lanes 32 (w % 4).. (one pixel per thread) and a block
 // of columns, applies bias + GELU (or GELU' for the backward pass), and writes the tile through
 // XOR-swizzled shared-memory staging so that the global stores are contiguous 16-byte pieces.
 // The tile's outputs are contiguous in global memory: pixels p0 .. p0+127, COUT channels each.
@@ -552,8 +596,7 @@ __device__ __forceinline__ int epi_n0(int warp) { return COUT == 64 ? epi_ncol<C
 template <int CIN, int COUT, int EPI, int NW>
 __device__ __forceinline__ void conv_tc_epilogue(uint32_t tacc, size_t p0, const float* breg,
                                                  float* __restrict__ outf, __nv_bfloat16* __restrict__ outb,
-                                                 const float* __restrict__ zin, unsigned char* stf, unsigned char* stb,
-                                                 size_t npix) {
+                                                 unsigned char* stf, unsigned char* stb, size_t npix) {
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     constexpr int NCOL = epi_ncol<COUT, NW>();
     constexpr int NT = NW * 32;
@@ -562,14 +605,6 @@ __device__ __forceinline__ void conv_tc_epilogue(uint32_t tacc, size_t p0, const
     const bool reads = COUT == 64 || warp < 4;
     const int px = 32 * (warp % 4) + lane;
     const int n0 = epi_n0<COUT, NW>(warp);
-    if (EPI == EPI_GELU_GRAD) {   // the tile's pre-activations, read contiguously
-        for (int i = threadIdx.x; i < kTileP * CF; i += NT) {
-            const int r = i / CF, c = i % CF;
-            *reinterpret_cast<float4*>(stf + (r * CF + (c ^ (r % CF))) * 16) =
-                *reinterpret_cast<const float4*>(zin + (p0 + r) * COUT + c * 4);
-        }
-        __syncthreads();
-    }
     if (reads) {
         float v[NCOL];
         tc::tmem_ld<NCOL>(tacc + ((uint32_t)(32 * (warp % 4)) << 16) + (uint32_t)n0, v);
@@ -578,25 +613,19 @@ __device__ __forceinline__ void conv_tc_epilogue(uint32_t tacc, size_t p0, const
             const int c = (n0 + j) / 4;
             float4* fz = reinterpret_cast<float4*>(stf + (px * CF + (c ^ (px % CF))) * 16);
             uint2* fb = reinterpret_cast<uint2*>(stb + (px * CB + (((n0 + j) / 8) ^ (px % CB))) * 16 + ((n0 + j) % 8) * 2);
-            if (EPI == EPI_GELU || EPI == EPI_LINEAR || EPI == EPI_PLANAR || EPI == EPI_GELU_ACT) {
-                const float4 z = make_float4(v[j] + breg[j], v[j + 1] + breg[j + 1], v[j + 2] + breg[j + 2],
-                                             v[j + 3] + breg[j + 3]);
-                if (EPI != EPI_GELU_ACT) *fz = z;
-                if (EPI == EPI_GELU || EPI == EPI_GELU_ACT) {
-                    __nv_bfloat162 g2[2] = {__floats2bfloat162_rn(gelu(z.x), gelu(z.y)),
-                                            __floats2bfloat162_rn(gelu(z.z), gelu(z.w))};
-                    *fb = *reinterpret_cast<const uint2*>(g2);
-                }
-            } else {
-                const float4 z = *fz;
-                __nv_bfloat162 g2[2] = {__floats2bfloat162_rn(v[j] * gelu_grad(z.x), v[j + 1] * gelu_grad(z.y)),
-                                        __floats2bfloat162_rn(v[j + 2] * gelu_grad(z.z), v[j + 3] * gelu_grad(z.w))};
+            const float4 z = make_float4(v[j] + breg[j], v[j + 1] + breg[j + 1], v[j + 2] + breg[j + 2],
+                                         v[j + 3] + breg[j + 3]);
+            if (EPI == EPI_GELU_ACT) {
+                __nv_bfloat162 g2[2] = {__floats2bfloat162_rn(gelu(z.x), gelu(z.y)),
+                                        __floats2bfloat162_rn(gelu(z.z), gelu(z.w))};
                 *fb = *reinterpret_cast<const uint2*>(g2);
+            } else {
+                *fz = z;
             }
         }
     }
     __syncthreads();
-    if (EPI == EPI_GELU || EPI == EPI_LINEAR) {
+    if (EPI == EPI_LINEAR) {
         for (int i = threadIdx.x; i < kTileP * CF; i += NT) {
             const int r = i / CF, c = i % CF;
             *reinterpret_cast<float4*>(outf + (p0 + r) * COUT + c * 4) =
@@ -611,7 +640,7 @@ __device__ __forceinline__ void conv_tc_epilogue(uint32_t tacc, size_t p0, const
                 reinterpret_cast<const float*>(stf + (r * CF + (c ^ (r % CF))) * 16)[n % 4];
         }
     }
-    if (EPI == EPI_GELU || EPI == EPI_GELU_GRAD || EPI == EPI_GELU_ACT) {
+    if (EPI == EPI_GELU_ACT) {
         for (int i = threadIdx.x; i < kTileP * CB; i += NT) {
             const int r = i / CB, c = i % CB;
             *reinterpret_cast<uint4*>(outb + (p0 + r) * COUT + c * 8) =
@@ -620,25 +649,46 @@ __device__ __forceinline__ void conv_tc_epilogue(uint32_t tacc, size_t p0, const
     }
 }
 
-// Pipelined over the CTA's tiles: the MMAs of tile t run into TMEM buffer t&1 while the
-// epilogue drains tile t-1 from the other buffer, and the next tile's new input row is fetched
-// meanwhile.  Input rows live in a 6-slot ring.
+// One layer for a batch, persistent over the CTA's tiles, with the warps split by role so that the
+// row loads, the MMAs and the epilogue of different tiles overlap:
+//   loaders   stream the input rows of the CTA's tiles into the ring (cp.async, two rows in flight
+//             behind the one being issued), one 'full' barrier per slot;
+//   issuer    one thread: waits for a tile's rows and a free accumulator, issues the tile's MMAs,
+//             and commits them to the accumulator's barrier and to the 'empty' barriers of the
+//             slots that no later tile reads;
+//   epilogue  eight warps, each 32 pixels x 32 channels: accumulator to registers, bias, GELU, BF16
+//             packing, and stores through a 4 KB staging block of the warp's own (XOR-swizzled, so
+//             that the global stores are whole 64- and 128-byte pieces): no block-wide barrier.
+// Bound by the epilogue's arithmetic: 8192 GELUs per tile are about 2000 cycles of the SM's issue
+// slots, the 36 MMAs 1200, the tile's traffic 850.  With one role after another in the same warps a
+// 64 -> 64 layer at batch 32 on 128^2 took 152 us with its FP32 second output; split, 118 us with it
+// and 92 us without (inference needs none), of which the loaders alone are 57 (B200, ncu).
+// EPI_GELU stores GELU'(z) in FP32 beside the activation, where the backward pass only multiplies by
+// it: the error function is evaluated once per training step instead of twice.
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(kTcThreads, 1)
+__global__ void __launch_bounds__(kRoleThreads, 1)
     k_conv_tc(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wt, const float* __restrict__ bias,
               int B, int H, int W, float* __restrict__ outf, __nv_bfloat16* __restrict__ outb,
-              const float* __restrict__ zin, int* __restrict__ err) {
+              const float* __restrict__ dact, int* __restrict__ err) {
     QGN_PDL_ENTRY();
     using L = tc::Lay<CIN, COUT>;
     static_assert(COUT == 16 || COUT == 64, "N of the MMA");
+    static_assert(COUT == 64 || EPI == EPI_LINEAR || EPI == EPI_PLANAR, "narrow outputs are the last layer's");
     constexpr int NACC = COUT < 32 ? 32 : COUT;           // TMEM columns per accumulator tile
+    constexpr int NCOL = COUT == 64 ? 32 : 16;            // channels per epilogue thread
+    constexpr int EW = COUT == 64 ? kEpiWarps : 4;        // epilogue warps with work
+    constexpr int NS = tc::kSlots;
     extern __shared__ __align__(1024) unsigned char smtc[];
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smtc + L::BAR_OFF);   // bar[0], bar[1]
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(smtc + L::BAR_OFF + 32);
-    const int warp = threadIdx.x / 32;
-    const uint32_t bar_a = smem_u32(bar), in_a = smem_u32(smtc), w_a = smem_u32(smtc + L::W_OFF);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(smtc + L::BAR_OFF + 192);
+    volatile int* gave_up = reinterpret_cast<volatile int*>(smtc + L::BAR_OFF + 200);
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const uint32_t in_a = smem_u32(smtc), w_a = smem_u32(smtc + L::W_OFF);
+    const uint32_t full = smem_u32(smtc + L::BAR_OFF), empty = full + 8 * NS, accf = empty + 8 * NS, acce = accf + 16,
+                   drained = acce + 16;
 
-    // this CTA's tiles: a contiguous range of t = ((b * segs + seg) * H + h), rows fastest
+    // this CTA's tiles: a contiguous range of t = ((b * segs + seg) * H + h), rows fastest.  Its
+    // maximal runs of consecutive rows of one (b, seg) read cnt + 2 rows each; loaders and issuer
+    // count the rows of all runs in the same order, row n in slot n % NS.
     const int segs = W / kTileP;
     const int ntiles = B * H * segs;
     const int per = (ntiles + gridDim.x - 1) / gridDim.x;
@@ -650,124 +700,183 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_a));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_a + 8));
+        *gave_up = 0;
+        for (int i = 0; i < NS; ++i) {
+            tc::bar_init(full + 8 * i, kLoadThreads);
+            tc::bar_init(empty + 8 * i, 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            tc::bar_init(accf + 8 * i, 1);
+            tc::bar_init(acce + 8 * i, EW);
+        }
+        tc::bar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    tc::fetch_weights<kTcThreads>(wt, CIN, COUT, w_a);
+    tc::fetch_weights<kRoleThreads>(wt, CIN, COUT, w_a);
     tc::cp_commit();
+    tc::cp_wait_all();
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tslot;
-    unsigned char* stf = smtc + L::STF_OFF;
-    unsigned char* stb = smtc + L::STB_OFF;
-    // this thread's bias values (its columns are the same in every tile)
-    constexpr int NCOL = epi_ncol<COUT, kTcWarps>();
-    float breg[NCOL];
-    {
-        const int n0 = epi_n0<COUT, kTcWarps>(warp);
+
+    if (warp < EW) {   // ---- epilogue
+        const int pw = 32 * (warp % 4);                   // first pixel of the warp
+        const int n0 = NCOL * (warp / 4);                 // first channel
+        float breg[NCOL];
+        if constexpr (EPI != EPI_GELU_GRAD) {
 #pragma unroll
-        for (int j = 0; j < NCOL; ++j) breg[j] = (EPI == EPI_GELU_GRAD) ? 0.f : bias[n0 + j];
-    }
-    // Ring slots are handed out round-robin, so the last six rows fetched sit in distinct slots.
-    // A tile that continues the previous one (same image and segment, next row) reuses two of
-    // its rows and needs one new row, usually prefetched during the previous tile; otherwise
-    // all three rows are fetched.  Live rows (previous tile, this tile, the prefetch) are at
-    // most the last five fetched, so no slot that an MMA in flight reads is overwritten.
-    int next_slot = 0;
-    int sl[3] = {0, 0, 0};                  // this tile's slots (rows h-1, h, h+1)
-    int pre_slot = -1;                      // slot of the row prefetched for this tile, or -1
-    int pbs = -1;
-    uint32_t phase[2] = {0u, 0u};
-    int pb = 0, ph = 0, pw0 = 0;            // coordinates of the previous tile
-    bool failed = false;
-    for (int t = t0; t < t1 && !failed; ++t) {
-        const int h = t % H, bs = t / H;
-        const int seg = bs % segs, b = bs / segs;
-        const int w0 = seg * kTileP;
-        const bool cont = t > t0 && bs == pbs && h == ph + 1 && H >= 3;
-        if (cont) {
-            sl[0] = sl[1];
-            sl[1] = sl[2];
-            if (pre_slot >= 0) {
-                sl[2] = pre_slot;
-            } else {
-                sl[2] = next_slot;
-                next_slot = (next_slot + 1) % tc::kSlots;
-                tc::fetch_row<CIN, kTcThreads>(x, b, (h + 1) % H, H, W, w0, in_a + (uint32_t)(sl[2] * L::SLOT_BYTES));
+            for (int j = 0; j < NCOL; ++j) breg[j] = bias[n0 + j];
+        }
+        unsigned char* stg = smtc + L::STG_OFF + warp * 4096;
+        for (int t = t0, i = 0; t < t1; ++t, ++i) {
+            const int h = t % H, bs = t / H;
+            const size_t p0 = ((size_t)(bs / segs) * H + h) * W + (bs % segs) * kTileP + pw;
+            const int buf = i & 1;
+            float4 dv[8];   // EPI_GELU_GRAD: the tile's GELU', 128 bytes of four pixels per load
+            if constexpr (EPI == EPI_GELU_GRAD) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    dv[k] = *reinterpret_cast<const float4*>(dact + (p0 + 4 * k + lane / 8) * COUT + n0 + 4 * (lane % 8));
             }
-        } else {
+            const bool ok = tc::role_wait(accf + 8 * buf, (i >> 1) & 1, gave_up);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            float v[NCOL];
+            tc::tmem_ld<NCOL>(tmem + ((uint32_t)pw << 16) + (uint32_t)(buf * NACC + n0), v);
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc::arrive(acce + 8 * buf);
+            if constexpr (EPI != EPI_GELU_GRAD) {
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                sl[k] = next_slot;
-                next_slot = (next_slot + 1) % tc::kSlots;
-                tc::fetch_row<CIN, kTcThreads>(x, b, (h + k - 1 + H) % H, H, W, w0, in_a + (uint32_t)(sl[k] * L::SLOT_BYTES));
+                for (int j = 0; j < NCOL; ++j) v[j] += breg[j];
+            }
+            if constexpr (EPI == EPI_PLANAR) {   // out[n][pixel]: 128 bytes per channel and warp
+                const size_t npix = (size_t)B * H * W;
+#pragma unroll
+                for (int j = 0; j < NCOL; ++j) outf[(size_t)(n0 + j) * npix + p0 + lane] = v[j];
+            } else if constexpr (EPI == EPI_LINEAR) {   // 16 channels: 64 bytes per pixel
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    *reinterpret_cast<float4*>(stg + lane * 64 + ((c ^ ((lane >> 1) & 3)) * 16)) =
+                        make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int px = 8 * k + lane / 4, c = lane % 4;
+                    *reinterpret_cast<float4*>(outf + (p0 + px) * COUT + 4 * c) =
+                        *reinterpret_cast<const float4*>(stg + px * 64 + ((c ^ ((px >> 1) & 3)) * 16));
+                }
+                __syncwarp();
+            } else {
+                __nv_bfloat162 o[NCOL / 2];
+                if constexpr (EPI == EPI_GELU_GRAD) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const int px = 4 * k + lane / 8, c = lane % 8;
+                        *reinterpret_cast<float4*>(stg + px * 128 + ((c ^ (px & 7)) * 16)) = dv[k];
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const float4 d = *reinterpret_cast<const float4*>(stg + lane * 128 + ((c ^ (lane & 7)) * 16));
+                        o[2 * c] = __floats2bfloat162_rn(v[4 * c] * d.x, v[4 * c + 1] * d.y);
+                        o[2 * c + 1] = __floats2bfloat162_rn(v[4 * c + 2] * d.z, v[4 * c + 3] * d.w);
+                    }
+                    __syncwarp();
+                } else {
+#pragma unroll
+                    for (int k = 0; k < NCOL / 2; ++k) {
+                        const float a = v[2 * k], b = v[2 * k + 1];
+                        o[k] = __floats2bfloat162_rn(gelu(a), gelu(b));
+                        if constexpr (EPI == EPI_GELU) {
+                            v[2 * k] = gelu_grad(a);
+                            v[2 * k + 1] = gelu_grad(b);
+                        }
+                    }
+                }
+                if constexpr (EPI == EPI_GELU) {   // GELU', 128 bytes per pixel
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        *reinterpret_cast<float4*>(stg + lane * 128 + ((c ^ (lane & 7)) * 16)) =
+                            make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+                    __syncwarp();
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const int px = 4 * k + lane / 8, c = lane % 8;
+                        *reinterpret_cast<float4*>(outf + (p0 + px) * COUT + n0 + 4 * c) =
+                            *reinterpret_cast<const float4*>(stg + px * 128 + ((c ^ (px & 7)) * 16));
+                    }
+                    __syncwarp();
+                }
+                // BF16 output, 64 bytes per pixel
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    *reinterpret_cast<uint4*>(stg + lane * 64 + ((c ^ ((lane >> 1) & 3)) * 16)) =
+                        *reinterpret_cast<const uint4*>(&o[4 * c]);
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int px = 8 * k + lane / 4, c = lane % 4;
+                    *reinterpret_cast<uint4*>(outb + (p0 + px) * COUT + n0 + 8 * c) =
+                        *reinterpret_cast<const uint4*>(stg + px * 64 + ((c ^ ((px >> 1) & 3)) * 16));
+                }
+                __syncwarp();
             }
         }
-        pre_slot = -1;
-        tc::cp_commit();
+    } else if (warp >= kEpiWarps && warp < kEpiWarps + kLoadWarps) {   // ---- loaders
+        const int tid = threadIdx.x - kEpiWarps * 32;
+        int n = 0;             // rows issued
+        bool ok = true;
+        for (int t = t0; t < t1 && ok;) {
+            const int h0 = t % H, bs = t / H;
+            const int cnt = min(t1 - t, H - h0);
+            const int b = bs / segs, w0 = (bs % segs) * kTileP;
+            for (int i = 0; i < cnt + 2; ++i, ++n) {
+                if (!(ok = tc::role_wait(empty + 8 * (n % NS), ((n / NS) & 1) ^ 1, gave_up))) break;
+                tc::fetch_row<CIN, kLoadThreads>(x, b, (h0 - 1 + i + H) % H, H, W, w0,
+                                                 in_a + (uint32_t)((n % NS) * L::SLOT_BYTES), tid);
+                tc::cp_commit();
+                if (n >= 2) {   // row n - 2 has landed
+                    asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    tc::arrive(full + 8 * ((n - 2) % NS));
+                }
+            }
+            t += cnt;
+        }
         tc::cp_wait_all();
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        __syncthreads();
-        const int buf = (t - t0) & 1;
-        if (threadIdx.x == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const uint32_t ra[3] = {in_a + (uint32_t)(sl[0] * L::SLOT_BYTES), in_a + (uint32_t)(sl[1] * L::SLOT_BYTES),
-                                    in_a + (uint32_t)(sl[2] * L::SLOT_BYTES)};
-            tc::issue_tile<CIN, COUT>(tmem + (uint32_t)(buf * NACC), ra, w_a, bar_a + 8u * (uint32_t)buf);
-        }
-        // the next tile's new row, if it continues this one.  Only when this tile continued the
-        // previous one (or is the first): after a fresh three-row fetch the six slots hold the
-        // previous tile's rows, whose MMAs may still be running, and this tile's.
-        if ((cont || t == t0) && t + 1 < t1 && (t + 1) / H == bs && h + 1 < H && H >= 3) {
-            pre_slot = next_slot;
-            next_slot = (next_slot + 1) % tc::kSlots;
-            tc::fetch_row<CIN, kTcThreads>(x, b, (h + 2) % H, H, W, w0, in_a + (uint32_t)(pre_slot * L::SLOT_BYTES));
-            tc::cp_commit();
-        }
-        // drain the previous tile while this one's MMAs run
-        if (t > t0) {
-            const int pbuf = buf ^ 1;
-            const bool ok = tc::bar_wait(bar_a + 8u * (uint32_t)pbuf, phase[pbuf]);
-            phase[pbuf] ^= 1u;
-            if (__syncthreads_or(!ok)) {
-                if (threadIdx.x == 0) atomicOr(err, 1);
-                failed = true;
-            } else {
+        for (int k = n >= 2 ? n - 2 : 0; k < n; ++k) tc::arrive(full + 8 * (k % NS));
+    } else if (warp == kEpiWarps + kLoadWarps && lane == 0) {   // ---- MMA issuer
+        int n = 0, i = 0;      // first row of the run, tile count
+        bool ok = true;
+        for (int t = t0; t < t1 && ok;) {
+            const int cnt = min(t1 - t, H - t % H);
+            for (int j = 0; j < cnt; ++j, ++i) {
+                for (int r = j == 0 ? 0 : 2; r < 3 && ok; ++r)
+                    ok = tc::role_wait(full + 8 * ((n + j + r) % NS), ((n + j + r) / NS) & 1, gave_up);
+                const int buf = i & 1;
+                ok = ok && tc::role_wait(acce + 8 * buf, ((i >> 1) & 1) ^ 1, gave_up);
+                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                conv_tc_epilogue<CIN, COUT, EPI, kTcWarps>(tmem + (uint32_t)(pbuf * NACC), ((size_t)pb * H + ph) * W + pw0, breg,
-                                                 outf, outb, zin, stf, stb, (size_t)B * H * W);
+                uint32_t ra[3];
+#pragma unroll
+                for (int r = 0; r < 3; ++r) ra[r] = in_a + (uint32_t)(((n + j + r) % NS) * L::SLOT_BYTES);
+                tc::issue_tile<CIN, COUT>(tmem + (uint32_t)(buf * NACC), ra, w_a, accf + 8 * buf);
+                for (int r = 0; r < (j == cnt - 1 ? 3 : 1); ++r) tc::commit(empty + 8 * ((n + j + r) % NS));
             }
+            n += cnt + 2;
+            t += cnt;
         }
-        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-        __syncthreads();   // the drained buffer and the previous tile's slots are free again
-        pbs = bs;
-        pb = b;
-        ph = h;
-        pw0 = w0;
+        tc::commit(drained);   // every MMA issued, also after a wait that ran out
+        tc::bar_wait(drained, 0);
     }
-    // the last tile
-    if (t1 > t0 && !failed) {
-        const int lbuf = (t1 - 1 - t0) & 1;
-        const bool ok = tc::bar_wait(bar_a + 8u * (uint32_t)lbuf, phase[lbuf]);
-        phase[lbuf] ^= 1u;
-        if (__syncthreads_or(!ok)) {
-            if (threadIdx.x == 0) atomicOr(err, 1);
-            failed = true;
-        } else {
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            conv_tc_epilogue<CIN, COUT, EPI, kTcWarps>(tmem + (uint32_t)(lbuf * NACC), ((size_t)pb * H + ph) * W + pw0, breg,
-                                             outf, outb, zin, stf, stb, (size_t)B * H * W);
-        }
-    }
-    if (failed) {   // once more, bounded, for MMAs still in flight, before the TMEM is freed
-        tc::bar_wait(bar_a, phase[0]);
-        tc::bar_wait(bar_a + 8u, phase[1]);
-    }
-    tc::cp_wait_all();
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
+    if (threadIdx.x == 0 && *gave_up) atomicOr(err, 1);
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t)L::TMEM_COLS));
@@ -842,7 +951,7 @@ __device__ __forceinline__ bool fused_layer(const FusedArgs& a, int l, int t, in
     const int H = a.H, W = a.W;
     const __nv_bfloat16* src = l == 0 ? a.x : a.act[l];
     // the own row needs no wait: it is this CTA's previous output (or the input)
-    tc::fetch_row<CIN, kFusedThreads>(src, b, h, H, W, w0, in_a + (uint32_t)FL::SLOT_BYTES);
+    tc::fetch_row<CIN, kFusedThreads>(src, b, h, H, W, w0, in_a + (uint32_t)FL::SLOT_BYTES, threadIdx.x);
     tc::cp_commit();
     // the epilogue's bias columns, loaded while the rows and the MMAs are in flight
     const int warp = threadIdx.x / 32;
@@ -861,8 +970,8 @@ __device__ __forceinline__ bool fused_layer(const FusedArgs& a, int l, int t, in
         tc::cp_wait_all();
         return false;
     }
-    tc::fetch_row<CIN, kFusedThreads>(src, b, (h - 1 + H) % H, H, W, w0, in_a);
-    tc::fetch_row<CIN, kFusedThreads>(src, b, (h + 1) % H, H, W, w0, in_a + 2u * (uint32_t)FL::SLOT_BYTES);
+    tc::fetch_row<CIN, kFusedThreads>(src, b, (h - 1 + H) % H, H, W, w0, in_a, threadIdx.x);
+    tc::fetch_row<CIN, kFusedThreads>(src, b, (h + 1) % H, H, W, w0, in_a + 2u * (uint32_t)FL::SLOT_BYTES, threadIdx.x);
     tc::cp_commit();
     tc::cp_wait_all();   // the rows and this layer's weights
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -887,7 +996,7 @@ __device__ __forceinline__ bool fused_layer(const FusedArgs& a, int l, int t, in
     }
     const size_t p0 = ((size_t)b * H + h) * W + w0;
     conv_tc_epilogue<CIN, COUT, EPI, kFusedWarps>(tmem, p0, breg, a.y, EPI == EPI_GELU_ACT ? a.act[l + 1] : nullptr,
-                                               nullptr, stf, stb, (size_t)a.B * H * W);
+                                                  stf, stb, (size_t)a.B * H * W);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     if (l + 1 < a.L) {   // publish the row
         __threadfence();
@@ -971,34 +1080,43 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_cnn_fused(FusedArgs a) {
 
 // ---- weight gradient on tcgen05 -------------------------------------------------------------
 // dW[tap][n][k] = sum_p G[p][n] X[p + tap][k] as MMAs with M = 64 (the 64-channel side: G when
-// COUT = 64, else X, whose channels are then padded to 64 with zero rows), N = the other side's
-// channels and K = 16 pixels.  Both operands are read MN-major (channels contiguous), straight
-// from the NHWC rows staged in the [channel group][pixel][16 B] layout of the forward pass, so a
-// tap's horizontal shift is a 16-byte offset of the descriptor's start address.  One CTA covers
-// a chunk of image rows for one tap row dh and keeps the three taps dw in TMEM; each stage (one
-// image row segment of 128 pixels: X row h + dh with its periodic halo, G row h) is fetched into
-// a three-buffer ring while the previous stage's 24 MMAs run.  On B200 an M = 64 accumulator
-// holds row m in TMEM lane 32 (m / 16) + m % 16, and an MN-major no-swizzle descriptor takes the
-// stride between 8-pixel (K) groups as its leading byte offset and the stride between 8-channel
-// groups as its stride byte offset (both measured with known operands).
+// COUT = 64, else X), N = the other side's channels and K = 16 pixels.  Both operands are read
+// MN-major (channels contiguous), straight from the NHWC rows staged in the [channel group][pixel]
+// [16 B] layout of the forward pass, so a tap's horizontal shift is a 16-byte offset of the
+// descriptor's start address.  One CTA covers a range of image rows for one tap row dh and keeps the
+// three taps dw in TMEM; a stage is one image row segment of 128 pixels (X row h + dh with its
+// periodic halo, G row h), 24 MMAs.  On B200 an M = 64 accumulator holds row m in TMEM lane
+// 32 (m / 16) + m % 16, and an MN-major no-swizzle descriptor takes the stride between 8-pixel (K)
+// groups as its leading byte offset and the stride between 8-channel groups as its stride byte
+// offset (both measured with known operands).
+// The warps have the roles of k_conv_tc: loaders fill a six-stage ring, one thread issues the MMAs,
+// and eight warps add the accumulators up in FP32 registers every kWChunkRows image rows (two
+// accumulator sets, so the MMAs go on meanwhile; the sums in TMEM stay as short as when each range
+// of 16 rows was a partial in memory).  In the CTAs of the middle tap row these warps also sum G
+// over the staged pixels: the bias gradient, without a pass of its own over G.
+// The three CTAs of a row range are neighbours in the grid, so the rows that one has fetched are in
+// L2 for the others.  A 64 -> 64 layer at batch 32 on 128^2: 195 us with one stage in flight and one
+// partial per 16 rows, 146 us now; its MMAs alone are about 35 us.
 namespace tc {
 template <int CIN, int COUT>
 struct WgLay {
     static constexpr bool A_IS_G = COUT == 64;
+    static_assert(A_IS_G || CIN == 64, "one side has the 64 rows of the MMA");
     static constexpr int N = A_IS_G ? CIN : COUT;           // MMA N
-    static constexpr int XG = A_IS_G ? CIN / 8 : 8;        // channel groups of an X slot
-    static constexpr int GG = A_IS_G ? 8 : COUT / 8;       // channel groups of a G slot
+    static constexpr int XG = CIN / 8, GG = COUT / 8;       // channel groups
     static constexpr int X_BYTES = XG * kPixS * 16;
-    static constexpr int G_BYTES = GG * kTileP * 16;
+    static constexpr int G_BYTES = GG * kPixS * 16;         // 128 of the 130 pixels: the loads of eight
+                                                            // groups then spread over the banks
     static constexpr int STAGE = (X_BYTES + G_BYTES + 1023) / 1024 * 1024;
-    static constexpr int NST = 3;                          // ring buffers
+    static constexpr int NST = 6;                          // ring stages
     static constexpr int BAR_OFF = NST * STAGE;
-    static constexpr int SMEM = BAR_OFF + 64;
-    static constexpr int TMEM_COLS = 3 * N <= 64 ? 64 : (3 * N <= 128 ? 128 : 256);
+    static constexpr int SMEM = BAR_OFF + 256;
+    static constexpr int TMEM_COLS = 6 * N <= 128 ? 128 : 512;   // two sets of three taps
     // every byte an MMA reads lies inside its stage, under either reading of LBO/SBO: the
     // furthest is the last pixel group of the last channel group at the largest start offset
     static_assert((16 * 7 + 2) * 16 + (XG - 1) * kPixS * 16 + 2 * 128 <= X_BYTES, "X reads stay in the slot");
-    static_assert(16 * 7 * 16 + (GG - 1) * kTileP * 16 + 2 * 128 <= G_BYTES, "G reads stay in the slot");
+    static_assert(16 * 7 * 16 + (GG - 1) * kPixS * 16 + 2 * 128 <= G_BYTES, "G reads stay in the slot");
+    static_assert(6 * N <= TMEM_COLS, "two accumulator sets");
 };
 
 // M = 64, N, BF16 x BF16 -> F32, both operands MN-major
@@ -1008,14 +1126,14 @@ __host__ __device__ constexpr uint32_t idesc_mn() {
            ((uint32_t)(64 >> 4) << 24);
 }
 
-// one G row segment (image b, row h, pixels w0 .. w0+127) into a slot [C/8][128][16 B]
+// one G row segment (image b, row h, pixels w0 .. w0+127) into a slot [C/8][kPixS][16 B]
 template <int C, int NT>
 __device__ __forceinline__ void fetch_grow(const __nv_bfloat16* __restrict__ g, int b, int h, int H, int W, int w0,
-                                          uint32_t slot_addr) {
+                                          uint32_t slot_addr, int tid) {
     const size_t row = ((size_t)b * H + h) * W + w0;
-    for (int i = threadIdx.x; i < kTileP * (C / 8); i += NT) {
+    for (int i = tid; i < kTileP * (C / 8); i += NT) {
         const int c8 = i % (C / 8), px = i / (C / 8);
-        cp16(slot_addr + (uint32_t)((c8 * kTileP + px) * 16), g + (row + px) * C + c8 * 8);
+        cp16(slot_addr + (uint32_t)((c8 * kPixS + px) * 16), g + (row + px) * C + c8 * 8);
     }
 }
 
@@ -1030,23 +1148,30 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
 }
 }  // namespace tc
 
-// partial[chunk][tap][n][k] over the chunk's rows for taps 3 dh' + 0..2 (dh' = blockIdx.y)
+// part[c][tap][n][k]: row range c of gridDim.x / 3, taps 3 dh' + 0..2 (dh' = blockIdx.x % 3);
+// bpart[c][n]: the sum of G over the range
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kRoleThreads, 1)
     k_wgrad_tc(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gr, int B, int H, int W,
-               float* __restrict__ part, int* __restrict__ err) {
+               float* __restrict__ part, float* __restrict__ bpart, int* __restrict__ err) {
     QGN_PDL_ENTRY();
     using L = tc::WgLay<CIN, COUT>;
-    constexpr int N = L::N;
+    constexpr int N = L::N, NST = L::NST;
     extern __shared__ __align__(1024) unsigned char smw[];
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(smw + L::BAR_OFF + 32);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(smw + L::BAR_OFF + 192);
+    volatile int* gave_up = reinterpret_cast<volatile int*>(smw + L::BAR_OFF + 200);
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const uint32_t base_a = smem_u32(smw), bar_a = smem_u32(smw + L::BAR_OFF);
-    const int dhi = blockIdx.y, dh = dhi - 1;
-    const int chunk = blockIdx.x;
+    const uint32_t base_a = smem_u32(smw);
+    const uint32_t full = smem_u32(smw + L::BAR_OFF), empty = full + 8 * NST, accf = empty + 8 * NST,
+                   acce = accf + 16, drained = acce + 16;
+    const int dhi = blockIdx.x % 3, dh = dhi - 1;
+    const int chunk = blockIdx.x / 3, chunks = gridDim.x / 3;
     const int segs = W / kTileP;
-    const int r0 = chunk * kWChunkRows, r1 = min(B * H, r0 + kWChunkRows);
-    const int S = (r1 - r0) * segs;
+    const int rows = B * H;
+    const int r0 = (int)((long long)rows * chunk / chunks), r1 = (int)((long long)rows * (chunk + 1) / chunks);
+    const int S = (r1 - r0) * segs;                     // stages
+    const int F = kWChunkRows * segs;                   // stages per accumulator set
+    const bool sums_g = dhi == 1;                       // the bias gradient's CTAs
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tslot)),
@@ -1054,109 +1179,152 @@ __global__ void __launch_bounds__(kThreads, 1)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
     if (threadIdx.x == 0) {
-        for (int i = 0; i < L::NST; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_a + 8u * i));
+        *gave_up = 0;
+        for (int i = 0; i < NST; ++i) {
+            tc::bar_init(full + 8 * i, kLoadThreads);
+            tc::bar_init(empty + 8 * i, sums_g ? 1 + kEpiWarps : 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            tc::bar_init(accf + 8 * i, 1);
+            tc::bar_init(acce + 8 * i, kEpiWarps);
+        }
+        tc::bar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    if constexpr (!L::A_IS_G && CIN < 64) {   // X as M: channel groups CIN/8 .. 7 are zero rows
-        constexpr int P = tc::kPixS;
-        for (int i = threadIdx.x; i < L::NST * (8 - CIN / 8) * P; i += kThreads) {
-            const int st = i / ((8 - CIN / 8) * P), r = i % ((8 - CIN / 8) * P);
-            *reinterpret_cast<uint4*>(smw + st * L::STAGE + (CIN / 8) * P * 16 + r * 16) = make_uint4(0, 0, 0, 0);
-        }
-    }
-    auto fetch = [&](int s, int buf) {
-        const int row = r0 + s / segs, w0 = (s % segs) * kTileP;
-        const int b = row / H, h = row % H;
-        const uint32_t xs = base_a + (uint32_t)(buf * L::STAGE), gs = xs + (uint32_t)L::X_BYTES;
-        tc::fetch_row<CIN, kThreads>(x, b, (h + dh + H) % H, H, W, w0, xs);
-        tc::fetch_grow<COUT, kThreads>(gr, b, h, H, W, w0, gs);
-        tc::cp_commit();
-    };
-    fetch(0, 0);
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tslot;
 
-    bool failed = false;
-    int issued = 0;   // stages whose MMAs were issued
-    for (int s = 0; s < S; ++s) {
-        const int buf = s % L::NST;
-        if (s + 1 < S) {
-            const int nb = (s + 1) % L::NST;
-            if (s + 1 >= L::NST) {   // the MMAs of stage s+1-NST read buffer nb
-                const bool ok = tc::bar_wait(bar_a + 8u * (uint32_t)nb, (uint32_t)(((s + 1 - L::NST) / L::NST) & 1));
-                if (__syncthreads_or(!ok)) {
-                    failed = true;
-                    break;
+    if (warp < kEpiWarps) {   // ---- accumulator drain and the bias sums
+        // warp w reads TMEM lanes 32 (w % 4) ..: its threads 0..15 hold rows m = 16 (w % 4) + lane,
+        // and the two warps of a sub-partition split the N columns
+        const int m = 16 * (warp % 4) + lane;
+        const int c0 = (warp / 4) * (N / 2);
+        float acc[3][N / 2];
+#pragma unroll
+        for (int dw = 0; dw < 3; ++dw)
+#pragma unroll
+            for (int c = 0; c < N / 2; ++c) acc[dw][c] = 0.f;
+        // bias sums: channel group tid % GG, every (256 / GG)-th pixel
+        constexpr int GG = L::GG, PX = kEpiWarps * 32 / GG;
+        float bs[8] = {};
+        bool ok = true;
+        for (int s0 = 0, e = 0; s0 < S && ok; s0 += F, ++e) {
+            if (sums_g) {
+                for (int s = s0; s < min(S, s0 + F) && ok; ++s) {
+                    ok = __all_sync(0xffffffffu, tc::role_wait(full + 8 * (s % NST), (s / NST) & 1, gave_up));
+                    if (!ok) break;
+                    const unsigned char* gs = smw + (s % NST) * L::STAGE + L::X_BYTES +
+                                              (threadIdx.x % GG) * tc::kPixS * 16 + (threadIdx.x / GG) * 16;
+#pragma unroll
+                    for (int px = 0; px < kTileP; px += PX) {
+                        const uint4 v = *reinterpret_cast<const uint4*>(gs + px * 16);
+                        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const float2 f = __bfloat1622float2(p[k]);
+                            bs[2 * k] += f.x;
+                            bs[2 * k + 1] += f.y;
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) tc::arrive(empty + 8 * (s % NST));
+                }
+                if (!ok) break;
+            }
+            ok = __all_sync(0xffffffffu, tc::role_wait(accf + 8 * (e & 1), (e >> 1) & 1, gave_up));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+            for (int dw = 0; dw < 3; ++dw) {
+#pragma unroll
+                for (int c = 0; c < N / 2; c += 8) {
+                    float v[8];
+                    tc::tmem_ld8(tmem + ((uint32_t)(32 * (warp % 4)) << 16) +
+                                     (uint32_t)((e & 1) * 3 * N + dw * N + c0 + c), v);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc[dw][c + j] += v[j];
                 }
             }
-            fetch(s + 1, nb);
-            asm volatile("cp.async.wait_group 1;\n" ::: "memory");   // stage s has landed
-        } else {
-            tc::cp_wait_all();
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc::arrive(acce + 8 * (e & 1));
         }
+        if (ok && lane < 16) {
+#pragma unroll
+            for (int dw = 0; dw < 3; ++dw) {
+                float* out = part + ((size_t)chunk * 9 + 3 * dhi + dw) * COUT * CIN;
+#pragma unroll
+                for (int c = 0; c < N / 2; ++c) {
+                    if constexpr (L::A_IS_G) out[(size_t)m * CIN + c0 + c] = acc[dw][c];          // D[n][k]
+                    else out[(size_t)(c0 + c) * CIN + m] = acc[dw][c];                            // D[k][n]
+                }
+            }
+        }
+        if (sums_g) {   // the threads of a channel group in a fixed order; every stage has been read
+            asm volatile("bar.sync 1, %0;\n" ::"r"(kEpiWarps * 32) : "memory");
+            float* sb = reinterpret_cast<float*>(smw);   // [256][8]
+#pragma unroll
+            for (int k = 0; k < 8; ++k) sb[threadIdx.x * 8 + k] = bs[k];
+            asm volatile("bar.sync 1, %0;\n" ::"r"(kEpiWarps * 32) : "memory");
+            if (threadIdx.x < COUT) {
+                float t = 0.f;
+                for (int q = 0; q < PX; ++q) t += sb[(q * GG + threadIdx.x / 8) * 8 + threadIdx.x % 8];
+                bpart[(size_t)chunk * COUT + threadIdx.x] = t;
+            }
+        }
+    } else if (warp < kEpiWarps + kLoadWarps) {   // ---- loaders
+        const int tid = threadIdx.x - kEpiWarps * 32;
+        int s = 0;
+        for (; s < S; ++s) {
+            if (!tc::role_wait(empty + 8 * (s % NST), ((s / NST) & 1) ^ 1, gave_up)) break;
+            const int row = r0 + s / segs, w0 = (s % segs) * kTileP;
+            const int b = row / H, h = row % H;
+            const uint32_t xs = base_a + (uint32_t)((s % NST) * L::STAGE), gs = xs + (uint32_t)L::X_BYTES;
+            tc::fetch_row<CIN, kLoadThreads>(x, b, (h + dh + H) % H, H, W, w0, xs, tid);
+            tc::fetch_grow<COUT, kLoadThreads>(gr, b, h, H, W, w0, gs, tid);
+            tc::cp_commit();
+            if (s >= 2) {   // stage s - 2 has landed
+                asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                tc::arrive(full + 8 * ((s - 2) % NST));
+            }
+        }
+        tc::cp_wait_all();
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        __syncthreads();
-        if (threadIdx.x == 0) {
+        for (int k = s >= 2 ? s - 2 : 0; k < s; ++k) tc::arrive(full + 8 * (k % NST));
+    } else if (lane == 0) {   // ---- MMA issuer
+        bool ok = true;
+        for (int s = 0; s < S && ok; ++s) {
+            const int e = s / F;
+            ok = tc::role_wait(full + 8 * (s % NST), (s / NST) & 1, gave_up);
+            if (ok && s % F == 0) ok = tc::role_wait(acce + 8 * (e & 1), ((e >> 1) & 1) ^ 1, gave_up);
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const uint32_t xs = base_a + (uint32_t)(buf * L::STAGE), gs = xs + (uint32_t)L::X_BYTES;
+            const uint32_t xs = base_a + (uint32_t)((s % NST) * L::STAGE), gs = xs + (uint32_t)L::X_BYTES;
+            const uint32_t d = tmem + (uint32_t)((e & 1) * 3 * N);
 #pragma unroll
             for (int dw = 0; dw < 3; ++dw) {
 #pragma unroll
                 for (int kc = 0; kc < kTileP / 16; ++kc) {
                     const uint32_t xa = xs + (uint32_t)((16 * kc + dw) * 16);   // slot pixel 0 is w0 - 1
                     const uint32_t ga = gs + (uint32_t)(16 * kc * 16);
-                    const uint64_t xd = tc::sdesc(xa, 128, tc::kPixS * 16), gd = tc::sdesc(ga, 128, kTileP * 16);
-                    tc::mma(tmem + (uint32_t)(dw * N), L::A_IS_G ? gd : xd, L::A_IS_G ? xd : gd, tc::idesc_mn<N>(),
-                            (s > 0 || kc > 0) ? 1u : 0u);
+                    const uint64_t xd = tc::sdesc(xa, 128, tc::kPixS * 16), gd = tc::sdesc(ga, 128, tc::kPixS * 16);
+                    tc::mma(d + (uint32_t)(dw * N), L::A_IS_G ? gd : xd, L::A_IS_G ? xd : gd, tc::idesc_mn<N>(),
+                            (s % F > 0 || kc > 0) ? 1u : 0u);
                 }
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                             bar_a + 8u * (uint32_t)buf)
-                         : "memory");
+            tc::commit(empty + 8 * (s % NST));
+            if (s % F == F - 1 || s == S - 1) tc::commit(accf + 8 * (e & 1));
         }
-        issued = s + 1;
+        tc::commit(drained);   // every MMA issued, also after a wait that ran out
+        tc::bar_wait(drained, 0);
     }
-    // the last issued stage's commit covers every earlier MMA of this thread
-    bool ok = true;
-    if (issued > 0) {
-        const int ls = issued - 1;
-        ok = tc::bar_wait(bar_a + 8u * (uint32_t)(ls % L::NST), (uint32_t)((ls / L::NST) & 1));
-    }
-    if (__syncthreads_or(!ok) || failed) {
-        if (threadIdx.x == 0) atomicOr(err, 4);
-        failed = true;
-    }
-    if (!failed) {
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        // warp w reads TMEM lanes 32 (w % 4) ..; its threads 0..15 hold rows m = 16 (w % 4) + lane,
-        // and the two warps of a sub-partition split the N columns
-        const int m = 16 * (warp % 4) + lane;
-        const int c0 = (warp / 4) * (N / 2);
-#pragma unroll
-        for (int dw = 0; dw < 3; ++dw) {
-            const int tap = 3 * dhi + dw;
-            float* out = part + ((size_t)chunk * 9 + tap) * COUT * CIN;
-#pragma unroll
-            for (int c = 0; c < N / 2; c += 8) {
-                float v[8];
-                tc::tmem_ld8(tmem + ((uint32_t)(32 * (warp % 4)) << 16) + (uint32_t)(dw * N + c0 + c), v);
-                if (lane < 16) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const int col = c0 + c + j;
-                        if constexpr (L::A_IS_G) out[(size_t)m * CIN + col] = v[j];          // D[n][k]
-                        else if (m < CIN) out[(size_t)col * CIN + m] = v[j];                 // D[k][n]
-                    }
-                }
-            }
-        }
-    }
-    tc::cp_wait_all();
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
+    if (threadIdx.x == 0 && *gave_up) atomicOr(err, 4);
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t)L::TMEM_COLS));
@@ -1186,11 +1354,13 @@ struct qgn_cnn {
     std::vector<int> ci, co;                         // padded channel counts per layer
     std::vector<float*> w, bias, mw, vw, mb, vb, gw, gb;
     std::vector<__nv_bfloat16*> wf, wb;
-    std::vector<float*> z;                           // pre-activations (FP32) per layer
+    std::vector<float*> z;                           // per layer (FP32): GELU'(pre-activation); last: the output
     std::vector<__nv_bfloat16*> act;                 // act[0] = input batch, act[l+1] = GELU(z[l])
     __nv_bfloat16* gA = nullptr;                     // backward: G of the current layer
     __nv_bfloat16* gB = nullptr;
+    float* grads = nullptr;                          // gw and gb of every layer, as in qgn_cnn_get_weights
     float* part = nullptr;                           // weight-gradient partials
+    float* bpart = nullptr;                          // bias-gradient partials
     size_t part_elems = 0;
     double* loss_part = nullptr;
     double* loss_host = nullptr;
@@ -1241,72 +1411,81 @@ int conv_grid(const qgn_cnn* n, int batch) {
 
 template <int CIN, int COUT, int EPI>
 cudaError_t launch_conv_t(qgn_cnn* n, const __nv_bfloat16* x, const __nv_bfloat16* wt, const float* bias, int batch,
-                          float* outf, __nv_bfloat16* outb, const float* zin) {
-    if (n->engine == 0) {
+                          float* outf, __nv_bfloat16* outb, const float* dact) {
+    if (n->engine != 1) {
         constexpr int SM = tc::Lay<CIN, COUT>::SMEM;
         if (cudaError_t e = smem_opt_in(k_conv_tc<CIN, COUT, EPI>, SM); e != cudaSuccess) return e;
-        ::qgn::launch(k_conv_tc<CIN, COUT, EPI>, conv_grid(n, batch), kTcThreads, SM, n->stream, x, wt, bias, batch, n->H, n->W,
-                                                                                    outf, outb, zin, n->d_err);
+        ::qgn::launch(k_conv_tc<CIN, COUT, EPI>, conv_grid(n, batch), kRoleThreads, SM, n->stream, x, wt, bias, batch, n->H,
+                      n->W, outf, outb, dact, n->d_err);
         return cudaGetLastError();
     }
     constexpr int SM = conv_smem<CIN, COUT>();
     if (cudaError_t e = smem_opt_in(k_conv<CIN, COUT, EPI>, SM); e != cudaSuccess) return e;
     ::qgn::launch(k_conv<CIN, COUT, EPI>, conv_grid(n, batch), kThreads, SM, n->stream, x, wt, bias, batch, n->H, n->W, outf,
-                                                                             outb, zin);
+                                                                             outb, dact);
     return cudaGetLastError();
 }
 
+// the layers of a network of width 64: 16 or 64 channels in and 64 out, or (the last) 64 in, 16 out
 template <int EPI>
 cudaError_t launch_conv(qgn_cnn* n, int cin, int cout, const __nv_bfloat16* x, const __nv_bfloat16* wt,
-                        const float* bias, int batch, float* outf, __nv_bfloat16* outb, const float* zin) {
-    if (cin == 16 && cout == 64) return launch_conv_t<16, 64, EPI>(n, x, wt, bias, batch, outf, outb, zin);
-    if (cin == 64 && cout == 64) return launch_conv_t<64, 64, EPI>(n, x, wt, bias, batch, outf, outb, zin);
-    if (cin == 64 && cout == 16) return launch_conv_t<64, 16, EPI>(n, x, wt, bias, batch, outf, outb, zin);
-    if (cin == 16 && cout == 16) return launch_conv_t<16, 16, EPI>(n, x, wt, bias, batch, outf, outb, zin);
+                        const float* bias, int batch, float* outf, __nv_bfloat16* outb, const float* dact) {
+    if constexpr (EPI == EPI_LINEAR || EPI == EPI_PLANAR) {
+        if (cin == 64 && cout == 16) return launch_conv_t<64, 16, EPI>(n, x, wt, bias, batch, outf, outb, dact);
+    } else {
+        if (cin == 16 && cout == 64) return launch_conv_t<16, 64, EPI>(n, x, wt, bias, batch, outf, outb, dact);
+        if (cin == 64 && cout == 64) return launch_conv_t<64, 64, EPI>(n, x, wt, bias, batch, outf, outb, dact);
+    }
     return cudaErrorInvalidValue;
 }
 
+// weight- and bias-gradient partials of one layer: *nchunks of the first in part, *nbias of the
+// second in bpart (the tcgen05 kernel) or, with the mma.sync engine, in part after the first are
+// reduced (see backward)
 template <int CIN, int COUT>
-cudaError_t launch_wgrad_t(qgn_cnn* n, const __nv_bfloat16* x, const __nv_bfloat16* g, int batch, float* part,
-                           int* nchunks) {
-    const int chunks = (batch * n->H + kWChunkRows - 1) / kWChunkRows;
-    *nchunks = chunks;
-    if (n->engine != 1) {   // tcgen05: one CTA per (row chunk, tap row), the three taps in TMEM
+cudaError_t launch_wgrad_t(qgn_cnn* n, const __nv_bfloat16* x, const __nv_bfloat16* g, int batch, int* nchunks) {
+    if (n->engine != 1) {   // one CTA per (row range, tap row), the three taps in TMEM
+        const int chunks = std::min(batch * n->H, kWgChunks);
+        *nchunks = chunks;
         constexpr int SM = tc::WgLay<CIN, COUT>::SMEM;
         if (cudaError_t e = smem_opt_in(k_wgrad_tc<CIN, COUT>, SM); e != cudaSuccess) return e;
-        ::qgn::launch(k_wgrad_tc<CIN, COUT>, dim3(chunks, 3), kThreads, SM, n->stream, x, g, batch, n->H, n->W, part,
-                      n->d_err);
+        ::qgn::launch(k_wgrad_tc<CIN, COUT>, 3 * chunks, kRoleThreads, SM, n->stream, x, g, batch, n->H, n->W, n->part,
+                      n->bpart, n->d_err);
         return cudaGetLastError();
     }
+    const int chunks = (batch * n->H + kWChunkRows - 1) / kWChunkRows;
+    *nchunks = chunks;
     constexpr int SM = wgrad_smem<CIN, COUT>();
     if (cudaError_t e = smem_opt_in(k_wgrad<CIN, COUT>, SM); e != cudaSuccess) return e;
-    ::qgn::launch(k_wgrad<CIN, COUT>, dim3(chunks, 9), kThreads, SM, n->stream, x, g, batch, n->H, n->W, part);
+    ::qgn::launch(k_wgrad<CIN, COUT>, dim3(chunks, 9), kThreads, SM, n->stream, x, g, batch, n->H, n->W, n->part);
     return cudaGetLastError();
 }
 
 cudaError_t launch_wgrad(qgn_cnn* n, int cin, int cout, const __nv_bfloat16* x, const __nv_bfloat16* g, int batch,
-                         float* part, int* nchunks) {
-    if (cin == 16 && cout == 64) return launch_wgrad_t<16, 64>(n, x, g, batch, part, nchunks);
-    if (cin == 64 && cout == 64) return launch_wgrad_t<64, 64>(n, x, g, batch, part, nchunks);
-    if (cin == 64 && cout == 16) return launch_wgrad_t<64, 16>(n, x, g, batch, part, nchunks);
-    if (cin == 16 && cout == 16) return launch_wgrad_t<16, 16>(n, x, g, batch, part, nchunks);
+                         int* nchunks) {
+    if (cin == 16 && cout == 64) return launch_wgrad_t<16, 64>(n, x, g, batch, nchunks);
+    if (cin == 64 && cout == 64) return launch_wgrad_t<64, 64>(n, x, g, batch, nchunks);
+    if (cin == 64 && cout == 16) return launch_wgrad_t<64, 16>(n, x, g, batch, nchunks);
     return cudaErrorInvalidValue;
 }
 
 // forward of a batch: layer 0 reads x0 (default act[0]); the last layer's FP32 output goes
-// to ylast (default z[L-1])
-int forward(qgn_cnn* net, int batch, const __nv_bfloat16* x0 = nullptr, float* ylast = nullptr, bool planar = false) {
+// to ylast (default z[L-1]).  grads: the hidden layers' GELU' go to z[l] for the backward pass.
+int forward(qgn_cnn* net, int batch, bool grads, const __nv_bfloat16* x0 = nullptr, float* ylast = nullptr,
+            bool planar = false) {
     const int L = net->layers;
     for (int l = 0; l < L; ++l) {
         const bool last = l == L - 1;
         const __nv_bfloat16* in = (l == 0 && x0) ? x0 : net->act[l];
-        cudaError_t e = (last && planar)
-                            ? launch_conv<EPI_PLANAR>(net, net->ci[l], net->co[l], in, net->wf[l], net->bias[l], batch,
-                                                      ylast ? ylast : net->z[l], nullptr, nullptr)
-                        : last ? launch_conv<EPI_LINEAR>(net, net->ci[l], net->co[l], in, net->wf[l], net->bias[l],
-                                                       batch, ylast ? ylast : net->z[l], nullptr, nullptr)
-                             : launch_conv<EPI_GELU>(net, net->ci[l], net->co[l], in, net->wf[l], net->bias[l],
-                                                     batch, net->z[l], net->act[l + 1], nullptr);
+        float* y = ylast ? ylast : net->z[l];
+        const int ci = net->ci[l], co = net->co[l];
+        cudaError_t e =
+            last && planar ? launch_conv<EPI_PLANAR>(net, ci, co, in, net->wf[l], net->bias[l], batch, y, nullptr, nullptr)
+            : last    ? launch_conv<EPI_LINEAR>(net, ci, co, in, net->wf[l], net->bias[l], batch, y, nullptr, nullptr)
+            : grads   ? launch_conv<EPI_GELU>(net, ci, co, in, net->wf[l], net->bias[l], batch, net->z[l],
+                                              net->act[l + 1], nullptr)
+                      : launch_conv<EPI_GELU_ACT>(net, ci, co, in, net->wf[l], net->bias[l], batch, nullptr,
+                                                  net->act[l + 1], nullptr);
         NCK(e);
     }
     return QGN_OK;
@@ -1320,15 +1499,20 @@ int backward(qgn_cnn* net, int batch) {
     const long long np = (long long)npix(net, batch);
     for (int l = L - 1; l >= 0; --l) {
         int chunks = 0;
-        NCK(launch_wgrad(net, net->ci[l], net->co[l], net->act[l], gcur, batch, net->part, &chunks));
+        NCK(launch_wgrad(net, net->ci[l], net->co[l], net->act[l], gcur, batch, &chunks));
         const int nw = 9 * net->co[l] * net->ci[l];
         ::qgn::launch(k_reduce_wgrad, (nw + 255) / 256, 256, 0, net->stream, net->part, chunks, nw, net->gw[l]);
         NCK(cudaGetLastError());
-        const int ppb = 1024;
-        const int nbp = (int)((np + ppb - 1) / ppb);
-        ::qgn::launch(k_bias_part, nbp, 64, 0, net->stream, gcur, np, net->co[l], ppb, net->part);
-        NCK(cudaGetLastError());
-        ::qgn::launch(k_reduce_wgrad, 1, 64, 0, net->stream, net->part, nbp, net->co[l], net->gb[l]);
+        const float* bpart = net->bpart;
+        int nbias = chunks;
+        if (net->engine == 1) {
+            const int ppb = 1024;
+            nbias = (int)((np + ppb - 1) / ppb);
+            ::qgn::launch(k_bias_part, nbias, 64, 0, net->stream, gcur, np, net->co[l], ppb, net->part);
+            NCK(cudaGetLastError());
+            bpart = net->part;
+        }
+        ::qgn::launch(k_reduce_wgrad, 1, 64, 0, net->stream, bpart, nbias, net->co[l], net->gb[l]);
         NCK(cudaGetLastError());
         if (l > 0) {
             NCK(launch_conv<EPI_GELU_GRAD>(net, net->co[l], net->ci[l], gcur, net->wb[l], nullptr, batch, nullptr,
@@ -1344,7 +1528,7 @@ int mse(qgn_cnn* net, int batch, const float* tgt) {
     const long long np = (long long)npix(net, batch);
     const int C = net->co[L - 1];
     const double inv = 1.0 / ((double)np * net->cout);
-    ::qgn::launch(k_mse, 148, kThreads, 0, net->stream, net->z[L - 1], tgt, np, C, net->cout, inv, net->gA, net->loss_part);
+    ::qgn::launch(k_mse, 148, kMseThreads, 0, net->stream, net->z[L - 1], tgt, np, C, net->cout, inv, net->gA, net->loss_part);
     NCK(cudaGetLastError());
     return QGN_OK;
 }
@@ -1445,7 +1629,7 @@ int infer(qgn_cnn* net, const void* x, float* y, int batch, cudaStream_t stream,
     cudaStream_t own = net->stream;
     net->stream = stream;
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
-    const int rc = fused_ok(net, batch) ? forward_fused(net, batch, xb, y, planar) : forward(net, batch, xb, y, planar);
+    const int rc = fused_ok(net, batch) ? forward_fused(net, batch, xb, y, planar) : forward(net, batch, false, xb, y, planar);
     net->stream = own;
     return rc;
 }
@@ -1486,14 +1670,24 @@ int qgn_cnn_create(int cin, int width, int cout, int layers, int H, int W, int m
     net->mb.resize(layers); net->vb.resize(layers); net->gw.resize(layers); net->gb.resize(layers);
     net->wf.resize(layers); net->wb.resize(layers); net->z.resize(layers); net->act.resize(layers + 1);
     size_t part = 0;
+    // gradients in one allocation, in the order of qgn_cnn_get_weights: one copy reads them back
+    size_t np = 0;
+    for (int l = 0; l < layers; ++l) np += 9ull * net->co[l] * net->ci[l] + net->co[l];
+    if (nalloc(net, &net->grads, np)) return fail(QGN_ERR_CUDA);
+    np = 0;
+    for (int l = 0; l < layers; ++l) {
+        net->gw[l] = net->grads + np;
+        np += 9ull * net->co[l] * net->ci[l];
+        net->gb[l] = net->grads + np;
+        np += net->co[l];
+    }
     std::mt19937_64 rng(seed);
     for (int l = 0; l < layers; ++l) {
         const int nw = 9 * net->co[l] * net->ci[l];
         if (nalloc(net, &net->w[l], nw) || nalloc(net, &net->mw[l], nw) || nalloc(net, &net->vw[l], nw) ||
-            nalloc(net, &net->gw[l], nw) || nalloc(net, &net->wf[l], nw) || nalloc(net, &net->wb[l], nw) ||
+            nalloc(net, &net->wf[l], nw) || nalloc(net, &net->wb[l], nw) ||
             nalloc(net, &net->bias[l], net->co[l]) || nalloc(net, &net->mb[l], net->co[l]) ||
-            nalloc(net, &net->vb[l], net->co[l]) || nalloc(net, &net->gb[l], net->co[l]) ||
-            nalloc(net, &net->z[l], NP * net->co[l]) || nalloc(net, &net->act[l], NP * net->ci[l]))
+            nalloc(net, &net->vb[l], net->co[l]) || nalloc(net, &net->z[l], NP * net->co[l]) || nalloc(net, &net->act[l], NP * net->ci[l]))
             return fail(QGN_ERR_CUDA);
         // He initialisation over the real fan-in, zeros in padded channels
         const int real_in = l == 0 ? cin : width, real_out = l == layers - 1 ? cout : width;
@@ -1509,10 +1703,10 @@ int qgn_cnn_create(int cin, int width, int cout, int layers, int H, int W, int m
         ::qgn::launch(k_weights_bf16, (nw + 255) / 256, 256, 0, net->stream, net->w[l], nw, net->co[l], net->ci[l], net->wf[l],
                                                                   net->wb[l]);
         const size_t chunks = (size_t)((max_batch * H + kWChunkRows - 1) / kWChunkRows);
-        part = std::max(part, chunks * nw);
+        part = std::max(part, std::max(chunks, (size_t)kWgChunks) * nw);
         part = std::max(part, ((NP + 1023) / 1024) * (size_t)net->co[l]);
     }
-    if (nalloc(net, &net->act[layers], 16) || nalloc(net, &net->gA, NP * net->width) ||
+    if (nalloc(net, &net->bpart, (size_t)kWgChunks * net->width) || nalloc(net, &net->act[layers], 16) || nalloc(net, &net->gA, NP * net->width) ||
         nalloc(net, &net->gB, NP * net->width) || nalloc(net, &net->part, part) ||
         nalloc(net, &net->loss_part, 148) || nalloc(net, &net->ytgt, NP * pad16(cout)) ||
         nalloc(net, &net->d_err, 1) || nalloc(net, &net->flags, 1024))
@@ -1595,21 +1789,14 @@ int qgn_cnn_gradients(qgn_cnn* net, const void* x, const float* y, int batch, fl
     if (!net || !x || !y || batch < 1 || batch > net->max_batch) return QGN_ERR_ARG;
     const size_t xb = npix(net, batch) * net->ci[0] * sizeof(__nv_bfloat16);
     NCK(cudaMemcpyAsync(net->act[0], x, xb, cudaMemcpyDeviceToDevice, net->stream));
-    int rc = forward(net, batch);
+    int rc = forward(net, batch, true);
     if (rc == QGN_OK) rc = mse(net, batch, y);
     if (rc == QGN_OK) rc = backward(net, batch);
     if (rc == QGN_OK) rc = read_loss(net, loss);
     if (rc != QGN_OK) return rc;
     if (grads_host) {
-        size_t off = 0;
-        for (int l = 0; l < net->layers; ++l) {
-            const size_t nw = 9ull * net->co[l] * net->ci[l];
-            NCK(cudaMemcpyAsync(grads_host + off, net->gw[l], sizeof(float) * nw, cudaMemcpyDeviceToHost, net->stream));
-            off += nw;
-            NCK(cudaMemcpyAsync(grads_host + off, net->gb[l], sizeof(float) * net->co[l], cudaMemcpyDeviceToHost,
-                                net->stream));
-            off += net->co[l];
-        }
+        NCK(cudaMemcpyAsync(grads_host, net->grads, sizeof(float) * (size_t)qgn_cnn_num_params(net),
+                            cudaMemcpyDeviceToHost, net->stream));
         NCK(cudaStreamSynchronize(net->stream));
     }
     return QGN_OK;
@@ -1630,7 +1817,7 @@ int qgn_cnn_train_step(qgn_cnn* net, const void* x_all, const float* y_all, cons
     ::qgn::launch(k_gather, 148 * 4, 256, 0, net->stream, reinterpret_cast<const unsigned char*>(y_all), idx, batch, ys,
                                               reinterpret_cast<unsigned char*>(net->ytgt));
     NCK(cudaGetLastError());
-    int rc = forward(net, batch);
+    int rc = forward(net, batch, true);
     if (rc == QGN_OK) rc = mse(net, batch, net->ytgt);
     if (rc == QGN_OK) rc = backward(net, batch);
     if (rc != QGN_OK) return rc;
