@@ -25,6 +25,7 @@
 #include "qgn_internal.cuh"
 #include "cnn.cuh"
 
+#include <cuda.h>        // CUtensorMap (types only: the encoder is looked up at run time)
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -49,16 +50,14 @@ constexpr int kThreads = kWarps * 32;
 // 58.2 -> 53.7 us on B200.
 constexpr int kFusedWarps = 16;
 constexpr int kFusedThreads = kFusedWarps * 32;
-// Warps of the layer kernels k_conv_tc and k_wgrad_tc, by role: accumulator drain, row loads, and
-// one that issues the MMAs.  Twelve in all, three per sub-partition: up to 168 registers a thread
-// (a thirteenth would leave 128).
-constexpr int kEpiWarps = 8;
-constexpr int kLoadWarps = 3;
-constexpr int kLoadThreads = kLoadWarps * 32;
-constexpr int kRoleThreads = (kEpiWarps + kLoadWarps + 1) * 32;
+// Warps of the layer kernels k_conv_tc and k_wgrad_tc by role: these drain accumulators, one more
+// loads rows, one issues the MMAs
+constexpr int kEpiWarps = 16;        // k_conv_tc
+constexpr int kDrainWarps = 8;       // k_wgrad_tc
+constexpr int kConvThreads = (kEpiWarps + 2) * 32;
+constexpr int kWgThreads = (kDrainWarps + 2) * 32;
 constexpr int kMseThreads = 1024;
-constexpr int kWChunkRows = 16;      // image rows summed in the accumulators before they are added up in FP32
-constexpr int kWgChunks = 49;        // row ranges of the tcgen05 weight gradient: 3 x 49 CTAs
+constexpr int kWChunkRows = 16;      // image rows per weight-gradient partial of the mma.sync engine
 
 // EPI_PLANAR: as EPI_LINEAR but the FP32 output is planar, out[n][pixel] (the closure's input
 // to its forward transform)
@@ -288,14 +287,34 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
-__global__ void k_reduce_wgrad(const float* __restrict__ part, int nchunks, int n, float* __restrict__ dw) {
+// dw[i] = sum of nchunks partials of n weights, db likewise of nb biases: a block sums 64 outputs, its
+// four groups of threads a quarter of the partials each, then the quarters in order.  (One thread per
+// output ran 147 dependent loads deep, 15.8 us for 64 x 64 x 9, and the biases' one block 12.5 us more.)
+constexpr int kRedOut = 64;
+__global__ void __launch_bounds__(4 * kRedOut)
+    k_reduce_wgrad(const float* __restrict__ part, int nchunks, int n, float* __restrict__ dw,
+                   const float* __restrict__ bpart, int nbchunks, int nb, float* __restrict__ db) {
     QGN_PDL_ENTRY();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float s = 0.f;
-#pragma unroll 8
-        for (int c = 0; c < nchunks; ++c) s += part[(size_t)c * n + i];
-        dw[i] = s;
+    __shared__ float sm[4][kRedOut];
+    const int o = threadIdx.x % kRedOut, q = threadIdx.x / kRedOut;
+    int i = blockIdx.x * kRedOut + o;
+    const int wblocks = (n + kRedOut - 1) / kRedOut;   // (the blocks of the weights; one more for the biases)
+    if ((int)blockIdx.x >= wblocks) {
+        part = bpart;
+        nchunks = nbchunks;
+        dw = db;
+        n = nb;
+        i = o;
     }
+    const int c0 = nchunks * q / 4, c1 = nchunks * (q + 1) / 4;
+    float s = 0.f;
+    if (i < n) {
+#pragma unroll 8
+        for (int c = c0; c < c1; ++c) s += part[(size_t)c * n + i];
+    }
+    sm[q][o] = s;
+    __syncthreads();
+    if (q == 0 && i < n) dw[i] = ((s + sm[1][o]) + sm[2][o]) + sm[3][o];
 }
 
 // bias gradient: per-block column sums of G, then a chunk reduction
@@ -410,14 +429,17 @@ __global__ void k_gather(const unsigned char* __restrict__ src, const int* __res
 
 // ---- the same convolution on the 5th-generation tensor cores (tcgen05, accumulator in TMEM) ----
 // One tile = 128 consecutive pixels of an image row (GEMM M = 128) x all COUT output channels
-// (N = COUT) with K = 9 taps x CIN, issued as 9*CIN/16 tcgen05.mma (kind::f16, BF16 in, FP32
-// accumulate) by one thread; the FP32 tile lives in TMEM (COUT columns, one lane per pixel) and
-// the epilogue reads it back with tcgen05.ld.  Operands sit in shared memory in the canonical
-// K-major no-swizzle layout (core matrices of 8 rows x 16 bytes):
-//   input rows  ring of 4 slots [CIN/8 chunks][130 pixels][8 channels]; the A tile of tap
-//               (dh, dw) starts at pixel dw of the slot holding row h+dh-1: rows (pixels) 16 B
-//               apart, 8-row groups 128 B apart (SBO), the two halves of a K step 130*16 B apart (LBO);
-//   weights     [9 taps][CIN/8 chunks][COUT][8]: SBO 128 B, LBO COUT*16 B.
+// with K = 9 taps x CIN (kind::f16, BF16 in, FP32 accumulate); the FP32 tile lives in TMEM (COUT columns, one lane per pixel) and
+// the epilogue reads it back with tcgen05.ld.  Operands sit in shared memory:
+//   input rows of 64 channels   [pixel][128 B] in the 128-byte swizzle (16-byte piece c of a pixel at
+//               c ^ (address / 128 % 8)), as one tensor-map copy of 128 pixels writes them, with the
+//               two pixels of the periodic halo on either side.  The A tile of tap (dh, dw) starts
+//               at pixel dw - 1: the swizzle goes by address, so a shift by whole pixels (128 B) is a
+//               shift of the start address.  Eight-pixel groups 1024 B apart (SBO);
+//   input rows of 16 channels   canonical K-major no-swizzle layout (core matrices of 8 rows x 16
+//               bytes): [2 channel groups][130 pixels][8 channels], pixels 16 B apart, 8-pixel
+//               groups 128 B apart (SBO), the two halves of a K step 130*16 B apart (LBO);
+//   weights     no-swizzle, chunks of eight input channels: SBO 128 B, LBO one chunk.
 // Each CTA takes a contiguous range of tiles ordered row-fastest, so consecutive tiles of a column
 // of rows share two of their three input rows: one new row per tile.  Completion is signalled by
 // tcgen05.commit on mbarriers; every wait is bounded, and a wait that runs out records an error,
@@ -426,33 +448,47 @@ namespace tc {
 
 constexpr int kPixS = kTileP + 2;        // staged pixels per input row (periodic halo)
 constexpr int kSlots = 6;                // input-row ring of the layer kernel
+constexpr int kAccSlots = 8;             // accumulator ring of the layer kernel
 constexpr long long kWaitLimit = 1LL << 22;
 
 constexpr int imax(int a, int b) { return a > b ? a : b; }
 
-// Shared-memory plan.  SMEM also covers the bytes an MMA would read if the hardware took the
-// two descriptor strides the other way round (8-row groups LBO apart, K halves SBO apart):
-// every operand read of the kernel stays inside the CTA's allocation under either reading.
-template <int CIN, int COUT>
-struct Lay {
-    static constexpr int SLOT_BYTES = (CIN / 8) * kPixS * 16;
-    static constexpr int IN_BYTES = kSlots * SLOT_BYTES;
-    static constexpr int W_OFF = (IN_BYTES + 1023) / 1024 * 1024;
-    static constexpr int W_BYTES = 9 * (CIN / 8) * COUT * 16;
-    static constexpr int BAR_OFF = (W_OFF + W_BYTES + 1023) / 1024 * 1024;
-    static constexpr int A_LAST = (kSlots - 1) * SLOT_BYTES + ((CIN / 8 - 2) * kPixS + 2) * 16;
-    static constexpr int B_LAST = W_OFF + (8 * (CIN / 8) + CIN / 8 - 2) * COUT * 16;
-    static constexpr int A_END = A_LAST + imax(kPixS * 16 + 15 * 128, 15 * kPixS * 16 + 128) + 128;
-    static constexpr int B_END = B_LAST + imax(COUT * 16 + (COUT / 8 - 1) * 128, (COUT / 8 - 1) * COUT * 16 + 128) + 128;
-    static constexpr int OPS_END = (imax(BAR_OFF + 256, imax(A_END, B_END)) + 1023) / 1024 * 1024;
-    static constexpr int STG_OFF = OPS_END;                 // output staging, 4 KB per epilogue warp
-    static constexpr int SMEM = STG_OFF + kEpiWarps * 4096;
-    static constexpr int TMEM_COLS = COUT < 32 ? 64 : 2 * COUT;   // two accumulator tiles, power of two
+// a staged row of C channels: 64 channels swizzled, halo pixels in the eight-pixel blocks before and
+// after the 128 pixels at MAIN; 16 channels in two planes
+template <int C>
+struct Row {
+    static constexpr bool SWZ = C == 64;
+    static constexpr int MAIN = SWZ ? 1024 : 0;
+    static constexpr int BYTES = SWZ ? 1024 + kTileP * 128 + 1024 : ((C / 8) * kPixS * 16 + 1023) / 1024 * 1024;
 };
 
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);   // version 1, no swizzle
+// Shared-memory plan of the layer kernel
+template <int CIN, int COUT>
+struct Lay {
+    static constexpr int SLOT_BYTES = Row<CIN>::BYTES;
+    static constexpr int W_OFF = kSlots * SLOT_BYTES;
+    static constexpr int W_BYTES = 9 * (CIN / 8) * COUT * 16;
+    static constexpr int BAR_OFF = (W_OFF + W_BYTES + 1023) / 1024 * 1024;
+    static constexpr int NB = 3 * COUT;                      // operand rows: the three tap rows
+    static constexpr int OPS_END = BAR_OFF + 1024;
+    static constexpr int STG_OFF = OPS_END;                 // output staging, 2 KB per epilogue warp
+    static constexpr int SMEM = STG_OFF + kEpiWarps * 2048;
+    static constexpr int TMEM_COLS = kAccSlots * COUT;       // the accumulators of eight output rows
+};
+
+// Shared-memory operand descriptors, version 1: the low word holds the start address and the leading
+// byte offset, the high word the stride byte offset and the swizzle.  Addresses and offsets are in
+// 16-byte units below 2^14, so a later start address is a sum on the low word.
+struct Desc {
+    uint32_t lo, hi;
+    __device__ __forceinline__ Desc at(uint32_t bytes) const { return Desc{lo + (bytes >> 4), hi}; }
+};
+__device__ __forceinline__ Desc sdesc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {   // no swizzle
+    return Desc{(saddr >> 4) | ((lbo >> 4) << 16), (sbo >> 4) | (1u << 14)};
+}
+// an operand in the 128-byte swizzle, groups of eight 128-byte rows 1024 B apart
+__device__ __forceinline__ Desc sdesc128(uint32_t saddr) {
+    return Desc{(saddr >> 4) | (64u << 16), 64u | (1u << 14) | (2u << 29)};
 }
 
 // M = 128, N = COUT, BF16 x BF16 -> F32, both operands K-major
@@ -461,11 +497,25 @@ __host__ __device__ constexpr uint32_t idesc() {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma(uint32_t tmem, uint64_t a, uint64_t b, uint32_t id, uint32_t accumulate) {
+// the same with N at run time (a multiple of 16, at most 256)
+__device__ __forceinline__ uint32_t idesc_n(int n) { return idesc<0>() | ((uint32_t)(n >> 3) << 17); }
+
+__device__ __forceinline__ void mma(uint32_t tmem, Desc a, Desc b, uint32_t id, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-        "l"(a), "l"(b), "r"(id), "r"(accumulate));
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}\n" ::"r"(tmem),
+        "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(id), "r"(accumulate));
+}
+
+// One lane of a converged warp, always the same one.  The MMAs are issued under it and not under
+// `lane == 0`: their operands live in uniform registers, and only this form tells the compiler that
+// what one thread computes is the warp's -- under a lane test every MMA moved its descriptors there
+// by itself and took about 110 cycles to issue, whatever its size.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
 }
 
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
@@ -516,6 +566,15 @@ __device__ __forceinline__ void cp16(uint32_t saddr, const void* g) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
 template <int NC>
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, float* v);
 template <>
@@ -540,17 +599,14 @@ __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, float* v) {
 // slots holding input rows h-1, h, h+1; w: the layer's weights.  One thread issues.
 template <int CIN, int COUT>
 __device__ __forceinline__ void issue_tile(uint32_t dacc, const uint32_t* ra, uint32_t w, uint32_t bar) {
-    // descriptors without their start address; per MMA the address is added in
-    const uint64_t da0 = sdesc(0u, kPixS * 16, 128), db0 = sdesc(0u, COUT * 16, 128);
+    const Desc b0 = sdesc(w, COUT * 16, 128);
+    const Desc a0[3] = {sdesc(ra[0], kPixS * 16, 128), sdesc(ra[1], kPixS * 16, 128), sdesc(ra[2], kPixS * 16, 128)};
 #pragma unroll
     for (int tap = 0; tap < 9; ++tap) {
 #pragma unroll
-        for (int kc = 0; kc < CIN / 16; ++kc) {
-            const uint32_t a_addr = ra[tap / 3] + (uint32_t)((2 * kc * kPixS + tap % 3) * 16);
-            const uint32_t b_addr = w + (uint32_t)((tap * (CIN / 8) + 2 * kc) * COUT * 16);
-            mma(dacc, da0 | (uint64_t)((a_addr >> 4) & 0x3FFFu), db0 | (uint64_t)((b_addr >> 4) & 0x3FFFu),
+        for (int kc = 0; kc < CIN / 16; ++kc)
+            mma(dacc, a0[tap / 3].at((2 * kc * kPixS + tap % 3) * 16), b0.at((tap * (CIN / 8) + 2 * kc) * COUT * 16),
                 idesc<COUT>(), (tap | kc) ? 1u : 0u);
-        }
     }
     commit(bar);
 }
@@ -567,6 +623,18 @@ __device__ __forceinline__ void fetch_weights(const __nv_bfloat16* __restrict__ 
     }
 }
 
+// the same into the layer kernel's operand layout [3 dw][CIN/8][3 COUT][8]: for one horizontal tap the
+// three tap rows stacked, dh = +1 first
+template <int CIN, int COUT, int NT>
+__device__ __forceinline__ void fetch_weights_stacked(const __nv_bfloat16* __restrict__ wt, uint32_t w) {
+    constexpr int C8 = CIN / 8;
+    for (int i = threadIdx.x; i < 9 * COUT * C8; i += NT) {
+        const int c8 = i % C8, n = (i / C8) % COUT, tap = i / (C8 * COUT);
+        const int dh = tap / 3, dw = tap % 3;
+        cp16(w + (uint32_t)(((dw * C8 + c8) * 3 * COUT + (2 - dh) * COUT + n) * 16), wt + ((size_t)tap * COUT + n) * CIN + c8 * 8);
+    }
+}
+
 // one input row (image b, row hh, pixels w0-1 .. w0+128 periodic) into a ring slot, asynchronously
 template <int CIN, int NT>
 __device__ __forceinline__ void fetch_row(const __nv_bfloat16* __restrict__ x, int b, int hh, int H, int W, int w0,
@@ -579,6 +647,46 @@ __device__ __forceinline__ void fetch_row(const __nv_bfloat16* __restrict__ x, i
         cp16(slot_addr + (uint32_t)((c8 * kPixS + px) * 16), x + (row + ww) * CIN + c8 * 8);
     }
 }
+
+// 128 pixels of 64 channels (row `row` of the map, pixels w0 ..) into swizzled shared memory; the
+// copy's bytes complete on bar
+__device__ __forceinline__ void tma_row(uint32_t dst, const CUtensorMap* map, int w0, int row, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+        "[%5];\n" ::"r"(dst),
+        "l"(map), "r"(0), "r"(w0), "r"(row), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void arrive_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+// One warp loads a row with its periodic halo (image row `row`, pixels w0-1 .. w0+128) into the slot
+// at `slot` and commits its cp.async group.  64 channels: the 128 pixels by tensor-map copy (its 16 KB
+// are an arrival on `full` of their own, made here) and the two halo pixels by cp.async; 16 channels:
+// all by cp.async.  The caller arrives once more when the group has completed.
+template <int C>
+__device__ __forceinline__ void load_row_warp(const CUtensorMap* map, const __nv_bfloat16* __restrict__ x, int row, int W,
+                                              int w0, uint32_t slot, uint32_t full, int lane) {
+    if constexpr (Row<C>::SWZ) {
+        const uint32_t main = slot + Row<C>::MAIN;
+        if (lane == 0) {
+            arrive_tx(full, kTileP * 128);
+            tma_row(main, map, w0, row, full);
+        }
+        if (lane < 16) {   // pixel w0-1 in the last row of the block before, w0+128 in the first one after
+            const int side = lane / 8, c = lane % 8;
+            const int ww = side ? (w0 + kTileP == W ? 0 : w0 + kTileP) : (w0 == 0 ? W - 1 : w0 - 1);
+            cp16(main + (side ? kTileP * 128 + c * 16 : -128 + ((c ^ 7) * 16)), x + ((size_t)row * W + ww) * C + c * 8);
+        }
+    } else {
+        fetch_row<C, 32>(x, 0, row, 0, W, w0, slot, lane);   // (b = 0: `row` counts all images' rows)
+    }
+    cp_commit();
+}
+// arrivals per use of a row's full barrier
+template <int C>
+__host__ __device__ constexpr int row_arrivals() { return Row<C>::SWZ ? 2 : 1; }
 
 }  // namespace tc
 
@@ -651,40 +759,44 @@ __device__ __forceinline__ void conv_tc_epilogue(uint32_t tacc, size_t p0, const
 
 // One layer for a batch, persistent over the CTA's tiles, with the warps split by role so that the
 // row loads, the MMAs and the epilogue of different tiles overlap:
-//   loaders   stream the input rows of the CTA's tiles into the ring (cp.async, two rows in flight
+//   loader    one warp: streams the input rows of the CTA's tiles into the ring (two rows in flight
 //             behind the one being issued), one 'full' barrier per slot;
-//   issuer    one thread: waits for a tile's rows and a free accumulator, issues the tile's MMAs,
-//             and commits them to the accumulator's barrier and to the 'empty' barriers of the
-//             slots that no later tile reads;
-//   epilogue  eight warps, each 32 pixels x 32 channels: accumulator to registers, bias, GELU, BF16
-//             packing, and stores through a 4 KB staging block of the warp's own (XOR-swizzled, so
-//             that the global stores are whole 64- and 128-byte pieces): no block-wide barrier.
-// Bound by the epilogue's arithmetic: 8192 GELUs per tile are about 2000 cycles of the SM's issue
-// slots, the 36 MMAs 1200, the tile's traffic 850.  With one role after another in the same warps a
-// 64 -> 64 layer at batch 32 on 128^2 took 152 us with its FP32 second output; split, 118 us with it
-// and 92 us without (inference needs none), of which the loaders alone are 57 (B200, ncu).
+//   issuer    one thread: multiplies each input row by the weights of all three tap rows at once, N =
+//             3 COUT, into the accumulators of the three output rows that it belongs to, which are
+//             neighbours in a ring of eight in TMEM; commits the row's slot to its 'empty' barrier
+//             and the output row that it completes to its 'full' one;
+//   epilogue  sixteen warps, each 32 pixels x 16 channels: accumulator to registers, bias, GELU, BF16
+//             packing, and stores through a 2 KB staging block of the warp's own (XOR-swizzled, so
+//             that the global stores are whole 32- and 64-byte sectors): no block-wide barrier.
+// An MMA here costs the shared-memory bytes of its operands (128 B per clock): 4 KB of pixels and 2 KB
+// of weights per 16 channels when each tap row was an MMA of its own with N = 64 (63 cycles measured,
+// 36 of them per tile), 4 + 6 KB for the three together.  The sum of an output is formed in the same
+// order either way (dh, dw, channels).
+// The epilogue's arithmetic is what is left: 8192 GELUs per tile, 32 instructions each.  64 -> 64 at
+// batch 32 on 128^2 (B200, ncu): loads, MMAs and epilogue one after another in the same warps 152 us
+// with an FP32 second output; the split in roles 118 us, 92 us without it (inference); this form 86 and
+// 69 us.
 // EPI_GELU stores GELU'(z) in FP32 beside the activation, where the backward pass only multiplies by
 // it: the error function is evaluated once per training step instead of twice.
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(kRoleThreads, 1)
-    k_conv_tc(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wt, const float* __restrict__ bias,
+__global__ void __launch_bounds__(kConvThreads, 1)
+    k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wt, const float* __restrict__ bias,
               int B, int H, int W, float* __restrict__ outf, __nv_bfloat16* __restrict__ outb,
               const float* __restrict__ dact, int* __restrict__ err) {
     QGN_PDL_ENTRY();
     using L = tc::Lay<CIN, COUT>;
     static_assert(COUT == 16 || COUT == 64, "N of the MMA");
     static_assert(COUT == 64 || EPI == EPI_LINEAR || EPI == EPI_PLANAR, "narrow outputs are the last layer's");
-    constexpr int NACC = COUT < 32 ? 32 : COUT;           // TMEM columns per accumulator tile
-    constexpr int NCOL = COUT == 64 ? 32 : 16;            // channels per epilogue thread
+    constexpr int NCOL = 16;                              // channels per epilogue thread
     constexpr int EW = COUT == 64 ? kEpiWarps : 4;        // epilogue warps with work
-    constexpr int NS = tc::kSlots;
+    constexpr int NS = tc::kSlots, NA = tc::kAccSlots;
     extern __shared__ __align__(1024) unsigned char smtc[];
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(smtc + L::BAR_OFF + 192);
-    volatile int* gave_up = reinterpret_cast<volatile int*>(smtc + L::BAR_OFF + 200);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(smtc + L::BAR_OFF + 240);
+    volatile int* gave_up = reinterpret_cast<volatile int*>(smtc + L::BAR_OFF + 248);
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const uint32_t in_a = smem_u32(smtc), w_a = smem_u32(smtc + L::W_OFF);
-    const uint32_t full = smem_u32(smtc + L::BAR_OFF), empty = full + 8 * NS, accf = empty + 8 * NS, acce = accf + 16,
-                   drained = acce + 16;
+    const uint32_t full = smem_u32(smtc + L::BAR_OFF), empty = full + 8 * NS, accf = empty + 8 * NS, acce = accf + 8 * NA,
+                   drained = acce + 8 * NA;
 
     // this CTA's tiles: a contiguous range of t = ((b * segs + seg) * H + h), rows fastest.  Its
     // maximal runs of consecutive rows of one (b, seg) read cnt + 2 rows each; loaders and issuer
@@ -702,17 +814,17 @@ __global__ void __launch_bounds__(kRoleThreads, 1)
     if (threadIdx.x == 0) {
         *gave_up = 0;
         for (int i = 0; i < NS; ++i) {
-            tc::bar_init(full + 8 * i, kLoadThreads);
+            tc::bar_init(full + 8 * i, tc::row_arrivals<CIN>());
             tc::bar_init(empty + 8 * i, 1);
         }
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < NA; ++i) {
             tc::bar_init(accf + 8 * i, 1);
             tc::bar_init(acce + 8 * i, EW);
         }
         tc::bar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    tc::fetch_weights<kRoleThreads>(wt, CIN, COUT, w_a);
+    tc::fetch_weights_stacked<CIN, COUT, kConvThreads>(wt, w_a);
     tc::cp_commit();
     tc::cp_wait_all();
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -729,22 +841,22 @@ __global__ void __launch_bounds__(kRoleThreads, 1)
 #pragma unroll
             for (int j = 0; j < NCOL; ++j) breg[j] = bias[n0 + j];
         }
-        unsigned char* stg = smtc + L::STG_OFF + warp * 4096;
+        unsigned char* stg = smtc + L::STG_OFF + warp * 2048;
         for (int t = t0, i = 0; t < t1; ++t, ++i) {
             const int h = t % H, bs = t / H;
             const size_t p0 = ((size_t)(bs / segs) * H + h) * W + (bs % segs) * kTileP + pw;
-            const int buf = i & 1;
-            float4 dv[8];   // EPI_GELU_GRAD: the tile's GELU', 128 bytes of four pixels per load
+            const int buf = i % NA;
+            float4 dv[4];   // EPI_GELU_GRAD: the tile's GELU', 64 bytes of eight pixels per load
             if constexpr (EPI == EPI_GELU_GRAD) {
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    dv[k] = *reinterpret_cast<const float4*>(dact + (p0 + 4 * k + lane / 8) * COUT + n0 + 4 * (lane % 8));
+                for (int k = 0; k < 4; ++k)
+                    dv[k] = *reinterpret_cast<const float4*>(dact + (p0 + 8 * k + lane / 4) * COUT + n0 + 4 * (lane % 4));
             }
-            const bool ok = tc::role_wait(accf + 8 * buf, (i >> 1) & 1, gave_up);
+            const bool ok = tc::role_wait(accf + 8 * buf, (i / NA) & 1, gave_up);
             if (!__all_sync(0xffffffffu, ok)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             float v[NCOL];
-            tc::tmem_ld<NCOL>(tmem + ((uint32_t)pw << 16) + (uint32_t)(buf * NACC + n0), v);
+            tc::tmem_ld<NCOL>(tmem + ((uint32_t)pw << 16) + (uint32_t)(buf * COUT + n0), v);
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
             if (lane == 0) tc::arrive(acce + 8 * buf);
@@ -756,77 +868,67 @@ __global__ void __launch_bounds__(kRoleThreads, 1)
                 const size_t npix = (size_t)B * H * W;
 #pragma unroll
                 for (int j = 0; j < NCOL; ++j) outf[(size_t)(n0 + j) * npix + p0 + lane] = v[j];
-            } else if constexpr (EPI == EPI_LINEAR) {   // 16 channels: 64 bytes per pixel
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    *reinterpret_cast<float4*>(stg + lane * 64 + ((c ^ ((lane >> 1) & 3)) * 16)) =
-                        make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-                __syncwarp();
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int px = 8 * k + lane / 4, c = lane % 4;
-                    *reinterpret_cast<float4*>(outf + (p0 + px) * COUT + 4 * c) =
-                        *reinterpret_cast<const float4*>(stg + px * 64 + ((c ^ ((px >> 1) & 3)) * 16));
-                }
-                __syncwarp();
             } else {
-                __nv_bfloat162 o[NCOL / 2];
-                if constexpr (EPI == EPI_GELU_GRAD) {
+                // FP32 staging: 64 bytes per pixel; lane = pixel, or four lanes per pixel
+                auto fpiece = [&](int px, int c) {
+                    return reinterpret_cast<float4*>(stg + px * 64 + ((c ^ ((px >> 1) & 3)) * 16));
+                };
+                auto put_f32 = [&]() {   // v -> outf
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const int px = 4 * k + lane / 8, c = lane % 8;
-                        *reinterpret_cast<float4*>(stg + px * 128 + ((c ^ (px & 7)) * 16)) = dv[k];
-                    }
+                    for (int c = 0; c < 4; ++c)
+                        *fpiece(lane, c) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
                     __syncwarp();
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const float4 d = *reinterpret_cast<const float4*>(stg + lane * 128 + ((c ^ (lane & 7)) * 16));
-                        o[2 * c] = __floats2bfloat162_rn(v[4 * c] * d.x, v[4 * c + 1] * d.y);
-                        o[2 * c + 1] = __floats2bfloat162_rn(v[4 * c + 2] * d.z, v[4 * c + 3] * d.w);
+                    for (int k = 0; k < 4; ++k) {
+                        const int px = 8 * k + lane / 4, c = lane % 4;
+                        *reinterpret_cast<float4*>(outf + (p0 + px) * COUT + n0 + 4 * c) = *fpiece(px, c);
                     }
                     __syncwarp();
+                };
+                if constexpr (EPI == EPI_LINEAR) {
+                    put_f32();
                 } else {
+                    __nv_bfloat162 o[NCOL / 2];
+                    if constexpr (EPI == EPI_GELU_GRAD) {
 #pragma unroll
-                    for (int k = 0; k < NCOL / 2; ++k) {
-                        const float a = v[2 * k], b = v[2 * k + 1];
-                        o[k] = __floats2bfloat162_rn(gelu(a), gelu(b));
-                        if constexpr (EPI == EPI_GELU) {
-                            v[2 * k] = gelu_grad(a);
-                            v[2 * k + 1] = gelu_grad(b);
+                        for (int k = 0; k < 4; ++k) *fpiece(8 * k + lane / 4, lane % 4) = dv[k];
+                        __syncwarp();
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const float4 d = *fpiece(lane, c);
+                            o[2 * c] = __floats2bfloat162_rn(v[4 * c] * d.x, v[4 * c + 1] * d.y);
+                            o[2 * c + 1] = __floats2bfloat162_rn(v[4 * c + 2] * d.z, v[4 * c + 3] * d.w);
+                        }
+                        __syncwarp();
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < NCOL / 2; ++k) {
+                            const float a = v[2 * k], b = v[2 * k + 1];
+                            o[k] = __floats2bfloat162_rn(gelu(a), gelu(b));
+                            if constexpr (EPI == EPI_GELU) {
+                                v[2 * k] = gelu_grad(a);
+                                v[2 * k + 1] = gelu_grad(b);
+                            }
                         }
                     }
-                }
-                if constexpr (EPI == EPI_GELU) {   // GELU', 128 bytes per pixel
+                    if constexpr (EPI == EPI_GELU) put_f32();
+                    // BF16 output, 32 bytes per pixel
+                    auto bpiece = [&](int px, int c) {
+                        return reinterpret_cast<uint4*>(stg + px * 32 + ((c ^ ((px >> 2) & 1)) * 16));
+                    };
 #pragma unroll
-                    for (int c = 0; c < 8; ++c)
-                        *reinterpret_cast<float4*>(stg + lane * 128 + ((c ^ (lane & 7)) * 16)) =
-                            make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+                    for (int c = 0; c < 2; ++c) *bpiece(lane, c) = *reinterpret_cast<const uint4*>(&o[4 * c]);
                     __syncwarp();
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const int px = 4 * k + lane / 8, c = lane % 8;
-                        *reinterpret_cast<float4*>(outf + (p0 + px) * COUT + n0 + 4 * c) =
-                            *reinterpret_cast<const float4*>(stg + px * 128 + ((c ^ (px & 7)) * 16));
+                    for (int k = 0; k < 2; ++k) {
+                        const int px = 16 * k + lane / 2, c = lane % 2;
+                        *reinterpret_cast<uint4*>(outb + (p0 + px) * COUT + n0 + 8 * c) = *bpiece(px, c);
                     }
                     __syncwarp();
                 }
-                // BF16 output, 64 bytes per pixel
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    *reinterpret_cast<uint4*>(stg + lane * 64 + ((c ^ ((lane >> 1) & 3)) * 16)) =
-                        *reinterpret_cast<const uint4*>(&o[4 * c]);
-                __syncwarp();
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int px = 8 * k + lane / 4, c = lane % 4;
-                    *reinterpret_cast<uint4*>(outb + (p0 + px) * COUT + n0 + 8 * c) =
-                        *reinterpret_cast<const uint4*>(stg + px * 64 + ((c ^ ((px >> 1) & 3)) * 16));
-                }
-                __syncwarp();
             }
         }
-    } else if (warp >= kEpiWarps && warp < kEpiWarps + kLoadWarps) {   // ---- loaders
-        const int tid = threadIdx.x - kEpiWarps * 32;
+    } else if (warp == kEpiWarps) {   // ---- loader
         int n = 0;             // rows issued
         bool ok = true;
         for (int t = t0; t < t1 && ok;) {
@@ -834,44 +936,89 @@ __global__ void __launch_bounds__(kRoleThreads, 1)
             const int cnt = min(t1 - t, H - h0);
             const int b = bs / segs, w0 = (bs % segs) * kTileP;
             for (int i = 0; i < cnt + 2; ++i, ++n) {
-                if (!(ok = tc::role_wait(empty + 8 * (n % NS), ((n / NS) & 1) ^ 1, gave_up))) break;
-                tc::fetch_row<CIN, kLoadThreads>(x, b, (h0 - 1 + i + H) % H, H, W, w0,
-                                                 in_a + (uint32_t)((n % NS) * L::SLOT_BYTES), tid);
-                tc::cp_commit();
-                if (n >= 2) {   // row n - 2 has landed
+                ok = __all_sync(0xffffffffu, tc::role_wait(empty + 8 * (n % NS), ((n / NS) & 1) ^ 1, gave_up));
+                if (!ok) break;
+                tc::load_row_warp<CIN>(&xmap, x, b * H + (h0 - 1 + i + H) % H, W, w0,
+                                       in_a + (uint32_t)((n % NS) * L::SLOT_BYTES), full + 8 * (n % NS), lane);
+                if (n >= 2) {   // the cp.async part of row n - 2 has landed
                     asm volatile("cp.async.wait_group 2;\n" ::: "memory");
                     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                    tc::arrive(full + 8 * ((n - 2) % NS));
+                    __syncwarp();
+                    if (lane == 0) tc::arrive(full + 8 * ((n - 2) % NS));
                 }
             }
             t += cnt;
         }
         tc::cp_wait_all();
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        for (int k = n >= 2 ? n - 2 : 0; k < n; ++k) tc::arrive(full + 8 * (k % NS));
-    } else if (warp == kEpiWarps + kLoadWarps && lane == 0) {   // ---- MMA issuer
-        int n = 0, i = 0;      // first row of the run, tile count
+        __syncwarp();
+        if (lane == 0) {
+            for (int k = n >= 2 ? n - 2 : 0; k < n; ++k) tc::arrive(full + 8 * (k % NS));
+            // after a wait that ran out, the tensor-map copies in flight still write this CTA's memory
+            if (!ok)
+                for (int k = n > NS ? n - NS : 0; k < n; ++k) tc::bar_wait(full + 8 * (k % NS), (k / NS) & 1);
+        }
+    } else if (warp == kEpiWarps + 1) {   // ---- MMA issuer (one lane; the warp waits with it)
+        int n = 0, o = 0;      // input rows, and output rows of the earlier runs
         bool ok = true;
         for (int t = t0; t < t1 && ok;) {
             const int cnt = min(t1 - t, H - t % H);
-            for (int j = 0; j < cnt; ++j, ++i) {
-                for (int r = j == 0 ? 0 : 2; r < 3 && ok; ++r)
-                    ok = tc::role_wait(full + 8 * ((n + j + r) % NS), ((n + j + r) / NS) & 1, gave_up);
-                const int buf = i & 1;
-                ok = ok && tc::role_wait(acce + 8 * buf, ((i >> 1) & 1) ^ 1, gave_up);
+            // input row i of the run belongs to its output rows i - 2 (dh = +1), i - 1 and i (dh = -1)
+            for (int i = 0; i < cnt + 2; ++i, ++n) {
+                ok = tc::role_wait(full + 8 * (n % NS), (n / NS) & 1, gave_up);
+                if (i < cnt)   // output row i starts here: its accumulator has been read
+                    ok = ok && tc::role_wait(acce + 8 * ((o + i) % NA), (((o + i) / NA) & 1) ^ 1, gave_up);
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                uint32_t ra[3];
+                if (tc::elect_one()) {
+                    constexpr bool SWZ = tc::Row<CIN>::SWZ;
+                    const uint32_t ra = in_a + (uint32_t)((n % NS) * L::SLOT_BYTES + tc::Row<CIN>::MAIN);
+                    const tc::Desc a0 = SWZ ? tc::sdesc128(ra - 128) : tc::sdesc(ra, tc::kPixS * 16, 128);
+                    const tc::Desc b0 = tc::sdesc(w_a, L::NB * 16, 128);
+                    // output rows jlo .. jhi; the ring's end may split them.  Everything that an MMA needs
+                    // beyond a sum per descriptor is formed here, once per row: this thread shares its
+                    // scheduler with the epilogue's warps (with the split worked out per MMA, a row's
+                    // MMAs took 190 cycles each to issue)
+                    const int jlo = max(i - 2, 0), jhi = min(i, cnt - 1);
+                    const int s1 = (o + jlo) % NA, c1 = min(jhi - jlo + 1, NA - s1), c2 = jhi - jlo + 1 - c1;
+                    const tc::Desc b1 = b0.at((jlo - (i - 2)) * COUT * 16), b2 = b1.at(c1 * COUT * 16);
+                    const uint32_t d1 = tmem + (uint32_t)(s1 * COUT);   // the second part starts at slot 0
+                    const uint32_t id1 = tc::idesc_n(c1 * COUT), id2 = tc::idesc_n(c2 * COUT);
+                    // the first product starts output row i (an accumulator of its own, the last one)
+                    if (i < cnt) {
+                        const int sn = (o + i) % NA;
+                        tc::mma(tmem + (uint32_t)(sn * COUT), a0, b0.at(2 * COUT * 16), tc::idesc<COUT>(), 0u);
+                        const int m1 = c2 > 0 ? c1 : c1 - 1;            // earlier rows in each part
+                        if (m1 > 0) tc::mma(d1, a0, b1, tc::idesc_n(m1 * COUT), 1u);
+                        if (c2 > 1) tc::mma(tmem, a0, b2, tc::idesc<COUT>(), 1u);
+                    } else {
+                        tc::mma(d1, a0, b1, id1, 1u);
+                        if (c2 > 0) tc::mma(tmem, a0, b2, id2, 1u);
+                    }
 #pragma unroll
-                for (int r = 0; r < 3; ++r) ra[r] = in_a + (uint32_t)(((n + j + r) % NS) * L::SLOT_BYTES);
-                tc::issue_tile<CIN, COUT>(tmem + (uint32_t)(buf * NACC), ra, w_a, accf + 8 * buf);
-                for (int r = 0; r < (j == cnt - 1 ? 3 : 1); ++r) tc::commit(empty + 8 * ((n + j + r) % NS));
+                    for (int dw = 0; dw < 3; ++dw) {
+#pragma unroll
+                        for (int kc = 0; kc < CIN / 16; ++kc) {
+                            if (dw == 0 && kc == 0) continue;
+                            const tc::Desc a = a0.at(SWZ ? dw * 128 + kc * 32 : (2 * kc * tc::kPixS + dw) * 16);
+                            const int bo = (dw * (CIN / 8) + 2 * kc) * L::NB * 16;
+                            tc::mma(d1, a, b1.at(bo), id1, 1u);
+                            if (c2 > 0) tc::mma(tmem, a, b2.at(bo), id2, 1u);
+                        }
+                    }
+                    tc::commit(empty + 8 * (n % NS));
+                    if (i >= 2) tc::commit(accf + 8 * ((o + i - 2) % NA));
+                }
+                __syncwarp();
             }
-            n += cnt + 2;
+            o += cnt;
             t += cnt;
         }
-        tc::commit(drained);   // every MMA issued, also after a wait that ran out
-        tc::bar_wait(drained, 0);
+        if (tc::elect_one()) {
+            tc::commit(drained);   // every MMA issued, also after a wait that ran out
+            tc::bar_wait(drained, 0);
+        }
     }
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -976,11 +1123,12 @@ __device__ __forceinline__ bool fused_layer(const FusedArgs& a, int l, int t, in
     tc::cp_wait_all();   // the rows and this layer's weights
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0 && tc::elect_one()) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t ra[3] = {in_a, in_a + (uint32_t)FL::SLOT_BYTES, in_a + 2u * (uint32_t)FL::SLOT_BYTES};
         tc::issue_tile<CIN, COUT>(tmem, ra, w_a, bar_a);
     }
+    __syncwarp();
     ok = tc::bar_wait(bar_a, phase);
     phase ^= 1u;
     if (__syncthreads_or(!ok)) {
@@ -1079,99 +1227,81 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_cnn_fused(FusedArgs a) {
 }
 
 // ---- weight gradient on tcgen05 -------------------------------------------------------------
-// dW[tap][n][k] = sum_p G[p][n] X[p + tap][k] as MMAs with M = 64 (the 64-channel side: G when
-// COUT = 64, else X), N = the other side's channels and K = 16 pixels.  Both operands are read
-// MN-major (channels contiguous), straight from the NHWC rows staged in the [channel group][pixel]
-// [16 B] layout of the forward pass, so a tap's horizontal shift is a 16-byte offset of the
-// descriptor's start address.  One CTA covers a range of image rows for one tap row dh and keeps the
-// three taps dw in TMEM; a stage is one image row segment of 128 pixels (X row h + dh with its
-// periodic halo, G row h), 24 MMAs.  On B200 an M = 64 accumulator holds row m in TMEM lane
-// 32 (m / 16) + m % 16, and an MN-major no-swizzle descriptor takes the stride between 8-pixel (K)
-// groups as its leading byte offset and the stride between 8-channel groups as its stride byte
-// offset (both measured with known operands).
-// The warps have the roles of k_conv_tc: loaders fill a six-stage ring, one thread issues the MMAs,
-// and eight warps add the accumulators up in FP32 registers every kWChunkRows image rows (two
-// accumulator sets, so the MMAs go on meanwhile; the sums in TMEM stay as short as when each range
-// of 16 rows was a partial in memory).  In the CTAs of the middle tap row these warps also sum G
-// over the staged pixels: the bias gradient, without a pass of its own over G.
-// The three CTAs of a row range are neighbours in the grid, so the rows that one has fetched are in
-// L2 for the others.  A 64 -> 64 layer at batch 32 on 128^2: 195 us with one stage in flight and one
-// partial per 16 rows, 146 us now; its MMAs alone are about 35 us.
+// dW[dh, dw][n][k] = sum_p G[p][n] X[p + (dh, dw)][k] as MMAs over K = 16 pixels, both operands read
+// MN-major (channels contiguous) straight from the NHWC rows staged as for the forward pass.  The M
+// side G has 64 channels, X 16 or 64.  For the last layer (64 -> 16) the two change places: with q = p
+// + tap the sum is over X[q] G[q - tap], the same with all taps mirrored (SWAP).
+// An input row r of X belongs to the taps dh = +1, 0, -1 of the G rows r - 1, r, r + 1, so one CTA makes
+// all nine taps from one pass over its rows: for every 16 pixels
+//   [G row r-1; G row r] x X row r    M = 128: two rows of G as the two 64-channel blocks of the A
+//                                     operand, their distance in the ring being the block stride (LBO);
+//                                     zero blocks before and after the ring stand in for a row that is
+//                                     not the CTA's, and for the second row where the ring wraps
+//   G row r+1 x X row r               M = 64
+// and, when X has 64 channels, its three horizontal taps are the three 64-column blocks of one B
+// operand with N = 192, one pixel (128 bytes of the swizzled row) apart.  Operand bytes in shared memory
+// are what an MMA costs: 18 KB per 16 pixels for the nine taps, 36 KB as nine products with M = N = 64.
+// On B200 an M = 64 accumulator holds row m in TMEM lane 32 (m / 16) + m % 16; an MN-major no-swizzle
+// descriptor takes the stride between 8-pixel (K) groups as its leading byte offset and the stride
+// between 8-channel groups as its stride byte offset, a swizzled one the stride between 64-channel
+// blocks and the stride between 8-pixel groups (measured with known operands).
+// Roles as in k_conv_tc: a loader (one ring of X rows, one of G rows), an MMA issuer, and eight warps
+// that sum G over the staged pixels (the bias gradient) while the MMAs run, then write the accumulators
+// as one partial per chunk of at most kWgRows rows, which bounds the length of the FP32 sums in TMEM.
+// 64 -> 64 at batch 32 on 128^2 (B200, ncu): one CTA per tap row 195 us with one stage in flight, 146 us
+// with the roles split, 89 us with swizzled tensor-map rows and MMAs issued from uniform registers;
+// this form 51 us, its traffic alone 20.
+constexpr int kWgRows = 32;          // most row segments per partial
 namespace tc {
-template <int CIN, int COUT>
+template <int CX>
 struct WgLay {
-    static constexpr bool A_IS_G = COUT == 64;
-    static_assert(A_IS_G || CIN == 64, "one side has the 64 rows of the MMA");
-    static constexpr int N = A_IS_G ? CIN : COUT;           // MMA N
-    static constexpr int XG = CIN / 8, GG = COUT / 8;       // channel groups
-    static constexpr int X_BYTES = XG * kPixS * 16;
-    static constexpr int G_BYTES = GG * kPixS * 16;         // 128 of the 130 pixels: the loads of eight
-                                                            // groups then spread over the banks
-    static constexpr int STAGE = (X_BYTES + G_BYTES + 1023) / 1024 * 1024;
-    static constexpr int NST = 6;                          // ring stages
-    static constexpr int BAR_OFF = NST * STAGE;
+    static constexpr int NX = 4, NG = 6;                   // ring slots
+    static constexpr int XB = Row<CX>::BYTES, GB = kTileP * 128;
+    static constexpr int Z1_OFF = 0;                       // zeros, below every G slot
+    static constexpr int G_OFF = GB;
+    static constexpr int Z2_OFF = G_OFF + NG * GB;         // zeros, above every G slot
+    static constexpr int X_OFF = Z2_OFF + GB;
+    static constexpr int SUM_OFF = X_OFF + NX * XB;        // bias sums [256][8]
+    static constexpr int BAR_OFF = SUM_OFF + kDrainWarps * 32 * 8 * 4;
     static constexpr int SMEM = BAR_OFF + 256;
-    static constexpr int TMEM_COLS = 6 * N <= 128 ? 128 : 512;   // two sets of three taps
-    // every byte an MMA reads lies inside its stage, under either reading of LBO/SBO: the
-    // furthest is the last pixel group of the last channel group at the largest start offset
-    static_assert((16 * 7 + 2) * 16 + (XG - 1) * kPixS * 16 + 2 * 128 <= X_BYTES, "X reads stay in the slot");
-    static_assert(16 * 7 * 16 + (GG - 1) * kPixS * 16 + 2 * 128 <= G_BYTES, "G reads stay in the slot");
-    static_assert(6 * N <= TMEM_COLS, "two accumulator sets");
+    static constexpr int N = 3 * CX;                       // accumulator columns of the three dw
+    static constexpr int TMEM_COLS = 2 * N <= 128 ? 128 : 512;
+    static_assert(Z2_OFF / 16 < (1 << 14), "block strides fit the descriptor");
+    // reads of a no-swizzle X slot, under either reading of LBO/SBO
+    static_assert(Row<CX>::SWZ || (16 * 7 + 2) * 16 + (CX / 8 - 1) * kPixS * 16 + 2 * 128 <= XB, "X reads");
 };
 
-// M = 64, N, BF16 x BF16 -> F32, both operands MN-major
-template <int N>
-__host__ __device__ constexpr uint32_t idesc_mn() {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(N >> 3) << 17) |
-           ((uint32_t)(64 >> 4) << 24);
+// BF16 x BF16 -> F32, both operands MN-major
+__host__ __device__ constexpr uint32_t idesc_mn(int m, int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(n >> 3) << 17) |
+           ((uint32_t)(m >> 4) << 24);
 }
-
-// one G row segment (image b, row h, pixels w0 .. w0+127) into a slot [C/8][kPixS][16 B]
-template <int C, int NT>
-__device__ __forceinline__ void fetch_grow(const __nv_bfloat16* __restrict__ g, int b, int h, int H, int W, int w0,
-                                          uint32_t slot_addr, int tid) {
-    const size_t row = ((size_t)b * H + h) * W + w0;
-    for (int i = tid; i < kTileP * (C / 8); i += NT) {
-        const int c8 = i % (C / 8), px = i / (C / 8);
-        cp16(slot_addr + (uint32_t)((c8 * kPixS + px) * 16), g + (row + px) * C + c8 * 8);
-    }
-}
-
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+// an MN-major operand in the 128-byte swizzle: 64-channel blocks `block` bytes apart
+__device__ __forceinline__ Desc sdesc128_mn(uint32_t saddr, uint32_t block) {
+    return Desc{(saddr >> 4) | ((block >> 4) << 16), 64u | (1u << 14) | (2u << 29)};
 }
 }  // namespace tc
 
-// part[c][tap][n][k]: row range c of gridDim.x / 3, taps 3 dh' + 0..2 (dh' = blockIdx.x % 3);
-// bpart[c][n]: the sum of G over the range
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(kRoleThreads, 1)
-    k_wgrad_tc(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gr, int B, int H, int W,
+// part[chunk][tap][n][k] and bpart[chunk][n] over the chunk's row segments (ordered as the tiles of
+// k_conv_tc), chunk = blockIdx.x, + gridDim.x, ...  SWAP: x is the 16-channel gradient, gr the
+// 64-channel input, and part is [8 - tap][k][n] of what the kernel forms.
+template <int CX, bool SWAP>
+__global__ void __launch_bounds__(kWgThreads, 1)
+    k_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap gmap,
+               const __nv_bfloat16* __restrict__ x, int B, int H, int W, int rows_per_chunk, int chunks,
                float* __restrict__ part, float* __restrict__ bpart, int* __restrict__ err) {
     QGN_PDL_ENTRY();
-    using L = tc::WgLay<CIN, COUT>;
-    constexpr int N = L::N, NST = L::NST;
+    using L = tc::WgLay<CX>;
+    constexpr int N = L::N, NX = L::NX, NG = L::NG;
     extern __shared__ __align__(1024) unsigned char smw[];
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(smw + L::BAR_OFF + 192);
-    volatile int* gave_up = reinterpret_cast<volatile int*>(smw + L::BAR_OFF + 200);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(smw + L::BAR_OFF + 240);
+    volatile int* gave_up = reinterpret_cast<volatile int*>(smw + L::BAR_OFF + 248);
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const uint32_t base_a = smem_u32(smw);
-    const uint32_t full = smem_u32(smw + L::BAR_OFF), empty = full + 8 * NST, accf = empty + 8 * NST,
-                   acce = accf + 16, drained = acce + 16;
-    const int dhi = blockIdx.x % 3, dh = dhi - 1;
-    const int chunk = blockIdx.x / 3, chunks = gridDim.x / 3;
+    const uint32_t fullx = smem_u32(smw + L::BAR_OFF), emptyx = fullx + 8 * NX, fullg = emptyx + 8 * NX,
+                   emptyg = fullg + 8 * NG, accf = emptyg + 8 * NG, acce = accf + 8, drained = acce + 8;
     const int segs = W / kTileP;
-    const int rows = B * H;
-    const int r0 = (int)((long long)rows * chunk / chunks), r1 = (int)((long long)rows * (chunk + 1) / chunks);
-    const int S = (r1 - r0) * segs;                     // stages
-    const int F = kWChunkRows * segs;                   // stages per accumulator set
-    const bool sums_g = dhi == 1;                       // the bias gradient's CTAs
+    const int ntiles = B * H * segs;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tslot)),
@@ -1180,146 +1310,232 @@ __global__ void __launch_bounds__(kRoleThreads, 1)
     }
     if (threadIdx.x == 0) {
         *gave_up = 0;
-        for (int i = 0; i < NST; ++i) {
-            tc::bar_init(full + 8 * i, kLoadThreads);
-            tc::bar_init(empty + 8 * i, sums_g ? 1 + kEpiWarps : 1);
+        for (int i = 0; i < NX; ++i) {
+            tc::bar_init(fullx + 8 * i, tc::row_arrivals<CX>());
+            tc::bar_init(emptyx + 8 * i, SWAP ? 1 + kDrainWarps : 1);
         }
-        for (int i = 0; i < 2; ++i) {
-            tc::bar_init(accf + 8 * i, 1);
-            tc::bar_init(acce + 8 * i, kEpiWarps);
+        for (int i = 0; i < NG; ++i) {
+            tc::bar_init(fullg + 8 * i, 1);
+            tc::bar_init(emptyg + 8 * i, SWAP ? 1 : 1 + kDrainWarps);
         }
+        tc::bar_init(accf, 1);
+        tc::bar_init(acce, kDrainWarps);
         tc::bar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    for (int i = threadIdx.x; i < L::GB / 16; i += kWgThreads) {
+        *reinterpret_cast<uint4*>(smw + L::Z1_OFF + i * 16) = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4*>(smw + L::Z2_OFF + i * 16) = make_uint4(0, 0, 0, 0);
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tslot;
 
-    if (warp < kEpiWarps) {   // ---- accumulator drain and the bias sums
-        // warp w reads TMEM lanes 32 (w % 4) ..: its threads 0..15 hold rows m = 16 (w % 4) + lane,
-        // and the two warps of a sub-partition split the N columns
-        const int m = 16 * (warp % 4) + lane;
-        const int c0 = (warp / 4) * (N / 2);
-        float acc[3][N / 2];
-#pragma unroll
-        for (int dw = 0; dw < 3; ++dw)
-#pragma unroll
-            for (int c = 0; c < N / 2; ++c) acc[dw][c] = 0.f;
-        // bias sums: channel group tid % GG, every (256 / GG)-th pixel
-        constexpr int GG = L::GG, PX = kEpiWarps * 32 / GG;
-        float bs[8] = {};
-        bool ok = true;
-        for (int s0 = 0, e = 0; s0 < S && ok; s0 += F, ++e) {
-            if (sums_g) {
-                for (int s = s0; s < min(S, s0 + F) && ok; ++s) {
-                    ok = __all_sync(0xffffffffu, tc::role_wait(full + 8 * (s % NST), (s / NST) & 1, gave_up));
+    // Every role walks the same rows: the chunk's runs of consecutive rows of one (b, seg), cnt G rows
+    // and cnt + 2 X rows each; X row i of a run goes with the G rows i - 2, i - 1 and i.
+    bool ok = true;
+    if (warp < kDrainWarps) {   // ---- bias sums, then the accumulators
+        // sums: channel group tid % GROUPS, every PX-th pixel of the staged gradient rows
+        constexpr int GROUPS = SWAP ? CX / 8 : 8, PX = kDrainWarps * 32 / GROUPS;
+        const int c8 = threadIdx.x % GROUPS, pq = threadIdx.x / GROUPS;
+        int n = 0, e = 0;      // rows summed, chunks done
+        for (int c = blockIdx.x; c < chunks && ok; c += gridDim.x, ++e) {
+            float bs[8] = {};
+            const int t1 = min(ntiles, (c + 1) * rows_per_chunk);
+            for (int t = c * rows_per_chunk; t < t1 && ok;) {
+                const int cnt = min(t1 - t, H - t % H);
+                for (int i = 0; i < (SWAP ? cnt + 2 : cnt); ++i, ++n) {
+                    const uint32_t f = SWAP ? fullx + 8 * (n % NX) : fullg + 8 * (n % NG);
+                    ok = __all_sync(0xffffffffu, tc::role_wait(f, (n / (SWAP ? NX : NG)) & 1, gave_up));
                     if (!ok) break;
-                    const unsigned char* gs = smw + (s % NST) * L::STAGE + L::X_BYTES +
-                                              (threadIdx.x % GG) * tc::kPixS * 16 + (threadIdx.x / GG) * 16;
+                    if (!SWAP || (i >= 1 && i <= cnt)) {   // (the halo rows are other rows' gradients)
+                        const unsigned char* s = SWAP ? smw + L::X_OFF + (n % NX) * L::XB : smw + L::G_OFF + (n % NG) * L::GB;
 #pragma unroll
-                    for (int px = 0; px < kTileP; px += PX) {
-                        const uint4 v = *reinterpret_cast<const uint4*>(gs + px * 16);
-                        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
+                        for (int p0 = 0; p0 < kTileP; p0 += PX) {
+                            const int px = p0 + pq;
+                            const uint4 v = *reinterpret_cast<const uint4*>(
+                                s + (SWAP ? (c8 * tc::kPixS + px + 1) * 16 : px * 128 + ((c8 ^ (px & 7)) * 16)));
+                            const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const float2 f = __bfloat1622float2(p[k]);
-                            bs[2 * k] += f.x;
-                            bs[2 * k + 1] += f.y;
+                            for (int k = 0; k < 4; ++k) {
+                                const float2 q = __bfloat1622float2(p[k]);
+                                bs[2 * k] += q.x;
+                                bs[2 * k + 1] += q.y;
+                            }
                         }
                     }
                     __syncwarp();
-                    if (lane == 0) tc::arrive(empty + 8 * (s % NST));
+                    if (lane == 0) tc::arrive(SWAP ? emptyx + 8 * (n % NX) : emptyg + 8 * (n % NG));
                 }
-                if (!ok) break;
+                t += cnt;
             }
-            ok = __all_sync(0xffffffffu, tc::role_wait(accf + 8 * (e & 1), (e >> 1) & 1, gave_up));
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            ok = ok && __all_sync(0xffffffffu, tc::role_wait(accf, e & 1, gave_up));
+            if (ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                // warp w reads TMEM lanes 32 (w % 4) .. and half of the columns.  First accumulator: rows
+                // 0..63 dh = +1, 64..127 dh = 0; second (M = 64, lanes 0..15 of each quarter): dh = -1
+                constexpr int HALF = N / 2, STEP = HALF % 16 == 0 ? 16 : 8;
+                const int q4 = warp % 4, c0 = (warp / 4) * HALF;
+                float* out = part + (size_t)c * 9 * 64 * CX;
 #pragma unroll
-            for (int dw = 0; dw < 3; ++dw) {
+                for (int d = 0; d < 2; ++d) {
+                    const int m = d == 0 ? (32 * q4 + lane) % 64 : 16 * q4 + lane;
+                    const int dh = d == 0 ? (q4 < 2 ? 1 : 0) : -1;
+                    for (int cc = 0; cc < HALF; cc += STEP) {
+                        float v[STEP];
+                        const uint32_t ta = tmem + ((uint32_t)(32 * q4) << 16) + (uint32_t)(d * N + c0 + cc);
+                        if constexpr (STEP == 16) tc::tmem_ld<16>(ta, v);
+                        else tc::tmem_ld8(ta, v);
+                        if (d == 0 || lane < 16) {
+                            const int dw = (c0 + cc) / CX, k = (c0 + cc) % CX;   // (a step stays in one tap)
+                            const int tap = 3 * (dh + 1) + dw;
+                            if constexpr (SWAP) {
 #pragma unroll
-                for (int c = 0; c < N / 2; c += 8) {
-                    float v[8];
-                    tc::tmem_ld8(tmem + ((uint32_t)(32 * (warp % 4)) << 16) +
-                                     (uint32_t)((e & 1) * 3 * N + dw * N + c0 + c), v);
+                                for (int j = 0; j < STEP; ++j) out[((size_t)(8 - tap) * CX + k + j) * 64 + m] = v[j];
+                            } else {
+                                float4* o = reinterpret_cast<float4*>(out + ((size_t)tap * 64 + m) * CX + k);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[dw][c + j] += v[j];
+                                for (int j = 0; j < STEP / 4; ++j)
+                                    o[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                            }
+                        }
+                    }
                 }
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tc::arrive(acce);
             }
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            __syncwarp();
-            if (lane == 0) tc::arrive(acce + 8 * (e & 1));
-        }
-        if (ok && lane < 16) {
-#pragma unroll
-            for (int dw = 0; dw < 3; ++dw) {
-                float* out = part + ((size_t)chunk * 9 + 3 * dhi + dw) * COUT * CIN;
-#pragma unroll
-                for (int c = 0; c < N / 2; ++c) {
-                    if constexpr (L::A_IS_G) out[(size_t)m * CIN + c0 + c] = acc[dw][c];          // D[n][k]
-                    else out[(size_t)(c0 + c) * CIN + m] = acc[dw][c];                            // D[k][n]
-                }
-            }
-        }
-        if (sums_g) {   // the threads of a channel group in a fixed order; every stage has been read
-            asm volatile("bar.sync 1, %0;\n" ::"r"(kEpiWarps * 32) : "memory");
-            float* sb = reinterpret_cast<float*>(smw);   // [256][8]
+            // the channels' sums over the warps' threads, in a fixed order (every warp comes here, also
+            // after a wait that ran out: `ok` then ends the loop)
+            float* sb = reinterpret_cast<float*>(smw + L::SUM_OFF);
 #pragma unroll
             for (int k = 0; k < 8; ++k) sb[threadIdx.x * 8 + k] = bs[k];
-            asm volatile("bar.sync 1, %0;\n" ::"r"(kEpiWarps * 32) : "memory");
-            if (threadIdx.x < COUT) {
-                float t = 0.f;
-                for (int q = 0; q < PX; ++q) t += sb[(q * GG + threadIdx.x / 8) * 8 + threadIdx.x % 8];
-                bpart[(size_t)chunk * COUT + threadIdx.x] = t;
+            asm volatile("bar.sync 1, %0;\n" ::"r"(kDrainWarps * 32) : "memory");
+            if (threadIdx.x < GROUPS * 8) {
+                float s = 0.f;
+                for (int q = 0; q < PX; ++q) s += sb[(q * GROUPS + threadIdx.x / 8) * 8 + threadIdx.x % 8];
+                bpart[(size_t)c * GROUPS * 8 + threadIdx.x] = s;
             }
+            uint32_t any;           // the warps leave the loop together
+            asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 1, %2, q;\n\t"
+                         "selp.u32 %0, 1, 0, p;\n\t}\n"
+                         : "=r"(any)
+                         : "r"(ok ? 0u : 1u), "r"(kDrainWarps * 32)
+                         : "memory");
+            ok = any == 0;
         }
-    } else if (warp < kEpiWarps + kLoadWarps) {   // ---- loaders
-        const int tid = threadIdx.x - kEpiWarps * 32;
-        int s = 0;
-        for (; s < S; ++s) {
-            if (!tc::role_wait(empty + 8 * (s % NST), ((s / NST) & 1) ^ 1, gave_up)) break;
-            const int row = r0 + s / segs, w0 = (s % segs) * kTileP;
-            const int b = row / H, h = row % H;
-            const uint32_t xs = base_a + (uint32_t)((s % NST) * L::STAGE), gs = xs + (uint32_t)L::X_BYTES;
-            tc::fetch_row<CIN, kLoadThreads>(x, b, (h + dh + H) % H, H, W, w0, xs, tid);
-            tc::fetch_grow<COUT, kLoadThreads>(gr, b, h, H, W, w0, gs, tid);
-            tc::cp_commit();
-            if (s >= 2) {   // stage s - 2 has landed
-                asm volatile("cp.async.wait_group 2;\n" ::: "memory");
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                tc::arrive(full + 8 * ((s - 2) % NST));
+    } else if (warp == kDrainWarps) {   // ---- loader
+        int n = 0, ng = 0;     // X rows and G rows issued
+        for (int c = blockIdx.x; c < chunks && ok; c += gridDim.x) {
+            const int t1 = min(ntiles, (c + 1) * rows_per_chunk);
+            for (int t = c * rows_per_chunk; t < t1 && ok;) {
+                const int h0 = t % H, bs = t / H;
+                const int cnt = min(t1 - t, H - h0);
+                const int b = bs / segs, w0 = (bs % segs) * kTileP;
+                for (int i = 0; i < cnt + 2; ++i, ++n) {
+                    ok = tc::role_wait(emptyx + 8 * (n % NX), ((n / NX) & 1) ^ 1, gave_up);
+                    if (i < cnt) ok = ok && tc::role_wait(emptyg + 8 * (ng % NG), ((ng / NG) & 1) ^ 1, gave_up);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    if (i < cnt) {
+                        if (lane == 0) {
+                            tc::arrive_tx(fullg + 8 * (ng % NG), L::GB);
+                            tc::tma_row(base_a + (uint32_t)(L::G_OFF + (ng % NG) * L::GB), &gmap, w0, b * H + h0 + i,
+                                        fullg + 8 * (ng % NG));
+                        }
+                        ++ng;
+                    }
+                    tc::load_row_warp<CX>(&xmap, x, b * H + (h0 - 1 + i + H) % H, W, w0,
+                                          base_a + (uint32_t)(L::X_OFF + (n % NX) * L::XB), fullx + 8 * (n % NX), lane);
+                    if (n >= 2) {   // the cp.async part of row n - 2 has landed
+                        asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+                        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) tc::arrive(fullx + 8 * ((n - 2) % NX));
+                    }
+                }
+                t += cnt;
             }
         }
         tc::cp_wait_all();
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        for (int k = s >= 2 ? s - 2 : 0; k < s; ++k) tc::arrive(full + 8 * (k % NST));
-    } else if (lane == 0) {   // ---- MMA issuer
-        bool ok = true;
-        for (int s = 0; s < S && ok; ++s) {
-            const int e = s / F;
-            ok = tc::role_wait(full + 8 * (s % NST), (s / NST) & 1, gave_up);
-            if (ok && s % F == 0) ok = tc::role_wait(acce + 8 * (e & 1), ((e >> 1) & 1) ^ 1, gave_up);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const uint32_t xs = base_a + (uint32_t)((s % NST) * L::STAGE), gs = xs + (uint32_t)L::X_BYTES;
-            const uint32_t d = tmem + (uint32_t)((e & 1) * 3 * N);
-#pragma unroll
-            for (int dw = 0; dw < 3; ++dw) {
-#pragma unroll
-                for (int kc = 0; kc < kTileP / 16; ++kc) {
-                    const uint32_t xa = xs + (uint32_t)((16 * kc + dw) * 16);   // slot pixel 0 is w0 - 1
-                    const uint32_t ga = gs + (uint32_t)(16 * kc * 16);
-                    const uint64_t xd = tc::sdesc(xa, 128, tc::kPixS * 16), gd = tc::sdesc(ga, 128, tc::kPixS * 16);
-                    tc::mma(d + (uint32_t)(dw * N), L::A_IS_G ? gd : xd, L::A_IS_G ? xd : gd, tc::idesc_mn<N>(),
-                            (s % F > 0 || kc > 0) ? 1u : 0u);
-                }
+        __syncwarp();
+        if (lane == 0) {
+            for (int k = n >= 2 ? n - 2 : 0; k < n; ++k) tc::arrive(fullx + 8 * (k % NX));
+            // after a wait that ran out, the tensor-map copies in flight still write this CTA's memory
+            if (!ok) {
+                for (int k = n > NX ? n - NX : 0; k < n; ++k) tc::bar_wait(fullx + 8 * (k % NX), (k / NX) & 1);
+                for (int k = ng > NG ? ng - NG : 0; k < ng; ++k) tc::bar_wait(fullg + 8 * (k % NG), (k / NG) & 1);
             }
-            tc::commit(empty + 8 * (s % NST));
-            if (s % F == F - 1 || s == S - 1) tc::commit(accf + 8 * (e & 1));
         }
-        tc::commit(drained);   // every MMA issued, also after a wait that ran out
-        tc::bar_wait(drained, 0);
+    } else {   // ---- MMA issuer (one lane; the warp waits with it)
+        int n = 0, g0 = 0, e = 0;   // X rows, G rows of the earlier runs, chunks
+        for (int c = blockIdx.x; c < chunks && ok; c += gridDim.x, ++e) {
+            const int t1 = min(ntiles, (c + 1) * rows_per_chunk);
+            ok = __all_sync(0xffffffffu, tc::role_wait(acce, (e & 1) ^ 1, gave_up));
+            uint32_t more1 = 0u, more2 = 0u;   // the accumulators hold earlier sums of this chunk
+            for (int t = c * rows_per_chunk; t < t1 && ok;) {
+                const int cnt = min(t1 - t, H - t % H);
+                for (int i = 0; i < cnt + 2; ++i, ++n) {
+                    ok = tc::role_wait(fullx + 8 * (n % NX), (n / NX) & 1, gave_up);
+                    if (i < cnt) ok = ok && tc::role_wait(fullg + 8 * ((g0 + i) % NG), ((g0 + i) / NG) & 1, gave_up);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    const bool pair = i >= 1;   // G row i - 1 or i - 2 exists
+                    if (tc::elect_one()) {
+                        constexpr bool XS = tc::Row<CX>::SWZ;
+                        const uint32_t xs = base_a + (uint32_t)(L::X_OFF + (n % NX) * L::XB);
+                        const tc::Desc x0 = XS ? tc::sdesc128_mn(xs + tc::Row<CX>::MAIN - 128, 128)
+                                               : tc::sdesc(xs, 128, tc::kPixS * 16);
+                        const uint32_t gs = base_a + (uint32_t)L::G_OFF, z1 = base_a + (uint32_t)L::Z1_OFF,
+                                       z2 = base_a + (uint32_t)L::Z2_OFF;
+                        // the 16-pixel products of one A operand with the X row (slot pixel 0 is w0 - 1)
+                        auto products = [&](uint32_t d, tc::Desc a, int m, uint32_t accumulate) {
+#pragma unroll
+                            for (int kc = 0; kc < kTileP / 16; ++kc) {
+                                if constexpr (XS) {
+                                    tc::mma(d, a.at(kc * 2048), x0.at(kc * 2048), tc::idesc_mn(m, N),
+                                            kc > 0 ? 1u : accumulate);
+                                } else {
+#pragma unroll
+                                    for (int dw = 0; dw < 3; ++dw)
+                                        tc::mma(d + (uint32_t)(dw * CX), a.at(kc * 2048), x0.at((16 * kc + dw) * 16),
+                                                tc::idesc_mn(m, CX), kc > 0 ? 1u : accumulate);
+                                }
+                            }
+                        };
+                        if (i < cnt) products(tmem + (uint32_t)N, tc::sdesc128_mn(gs + (uint32_t)(((g0 + i) % NG) * L::GB), 128), 64, more2);
+                        if (pair) {
+                            const uint32_t ga = gs + (uint32_t)(((g0 + i + 2 * NG - 2) % NG) * L::GB);   // row i - 2
+                            const uint32_t gb = gs + (uint32_t)(((g0 + i + NG - 1) % NG) * L::GB);       // row i - 1
+                            const bool ha = i >= 2, hb = i - 1 < cnt;
+                            if (ha && hb && gb > ga) {
+                                products(tmem, tc::sdesc128_mn(ga, gb - ga), 128, more1);
+                            } else {
+                                if (ha) products(tmem, tc::sdesc128_mn(ga, z2 - ga), 128, more1);
+                                if (hb) products(tmem, tc::sdesc128_mn(z1, gb - z1), 128, ha ? 1u : more1);
+                            }
+                        }
+                        tc::commit(emptyx + 8 * (n % NX));
+                        if (i >= 2) tc::commit(emptyg + 8 * ((g0 + i - 2) % NG));
+                    }
+                    __syncwarp();
+                    more2 = 1u;
+                    if (pair) more1 = 1u;
+                }
+                g0 += cnt;
+                t += cnt;
+            }
+            if (ok && tc::elect_one()) tc::commit(accf);
+            __syncwarp();
+        }
+        if (tc::elect_one()) {
+            tc::commit(drained);   // every MMA issued, also after a wait that ran out
+            tc::bar_wait(drained, 0);
+        }
     }
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -1409,14 +1625,38 @@ int conv_grid(const qgn_cnn* n, int batch) {
     return std::max(1, std::min(tiles, 148));
 }
 
+// The tensor map of `rows` image rows of W pixels x 64 channels (BF16, NHWC), copied 128 pixels at a
+// time into the 128-byte swizzle.  The encoder is a driver entry point, looked up once.
+cudaError_t row_map(const __nv_bfloat16* p, int W, int rows, CUtensorMap* map) {
+    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &r) != cudaSuccess) f = nullptr;
+        return reinterpret_cast<Encode>(f);
+    }();
+    if (!encode) return cudaErrorNotSupported;
+    const cuuint64_t dims[3] = {64, (cuuint64_t)W, (cuuint64_t)rows}, strides[2] = {128, (cuuint64_t)W * 128};
+    const cuuint32_t box[3] = {64, kTileP, 1}, es[3] = {1, 1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16*>(p), dims, strides, box, es,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 template <int CIN, int COUT, int EPI>
 cudaError_t launch_conv_t(qgn_cnn* n, const __nv_bfloat16* x, const __nv_bfloat16* wt, const float* bias, int batch,
                           float* outf, __nv_bfloat16* outb, const float* dact) {
     if (n->engine != 1) {
         constexpr int SM = tc::Lay<CIN, COUT>::SMEM;
         if (cudaError_t e = smem_opt_in(k_conv_tc<CIN, COUT, EPI>, SM); e != cudaSuccess) return e;
-        ::qgn::launch(k_conv_tc<CIN, COUT, EPI>, conv_grid(n, batch), kRoleThreads, SM, n->stream, x, wt, bias, batch, n->H,
-                      n->W, outf, outb, dact, n->d_err);
+        CUtensorMap map = {};
+        if (CIN == 64)
+            if (cudaError_t e = row_map(x, n->W, batch * n->H, &map); e != cudaSuccess) return e;
+        ::qgn::launch(k_conv_tc<CIN, COUT, EPI>, conv_grid(n, batch), kConvThreads, SM, n->stream, map, x, wt, bias, batch,
+                      n->H, n->W, outf, outb, dact, n->d_err);
         return cudaGetLastError();
     }
     constexpr int SM = conv_smem<CIN, COUT>();
@@ -1439,19 +1679,37 @@ cudaError_t launch_conv(qgn_cnn* n, int cin, int cout, const __nv_bfloat16* x, c
     return cudaErrorInvalidValue;
 }
 
-// weight- and bias-gradient partials of one layer: *nchunks of the first in part, *nbias of the
-// second in bpart (the tcgen05 kernel) or, with the mma.sync engine, in part after the first are
-// reduced (see backward)
+// partials of the tcgen05 weight gradient: row segments per partial and their number
+int wg_rows(const qgn_cnn* n, int batch) {
+    const int tiles = batch * n->H * (n->W / kTileP);
+    return std::min(kWgRows, (tiles + 147) / 148);
+}
+int wg_chunks(const qgn_cnn* n, int batch) {
+    const int tiles = batch * n->H * (n->W / kTileP), r = wg_rows(n, batch);
+    return (tiles + r - 1) / r;
+}
+
+// weight-gradient partials of one layer into part (*nchunks of them); the tcgen05 kernel also leaves
+// as many bias-gradient partials in bpart
+template <int CX, bool SWAP>
+cudaError_t launch_wgrad_tc(qgn_cnn* n, const __nv_bfloat16* x, const __nv_bfloat16* g, int batch, int* nchunks) {
+    constexpr int SM = tc::WgLay<CX>::SMEM;
+    if (cudaError_t e = smem_opt_in(k_wgrad_tc<CX, SWAP>, SM); e != cudaSuccess) return e;
+    CUtensorMap xm = {}, gm = {};
+    if (CX == 64)
+        if (cudaError_t e = row_map(x, n->W, batch * n->H, &xm); e != cudaSuccess) return e;
+    if (cudaError_t e = row_map(g, n->W, batch * n->H, &gm); e != cudaSuccess) return e;
+    const int chunks = *nchunks = wg_chunks(n, batch);
+    ::qgn::launch(k_wgrad_tc<CX, SWAP>, std::min(chunks, 148), kWgThreads, SM, n->stream, xm, gm, x, batch, n->H, n->W,
+                  wg_rows(n, batch), chunks, n->part, n->bpart, n->d_err);
+    return cudaGetLastError();
+}
+
 template <int CIN, int COUT>
 cudaError_t launch_wgrad_t(qgn_cnn* n, const __nv_bfloat16* x, const __nv_bfloat16* g, int batch, int* nchunks) {
-    if (n->engine != 1) {   // one CTA per (row range, tap row), the three taps in TMEM
-        const int chunks = std::min(batch * n->H, kWgChunks);
-        *nchunks = chunks;
-        constexpr int SM = tc::WgLay<CIN, COUT>::SMEM;
-        if (cudaError_t e = smem_opt_in(k_wgrad_tc<CIN, COUT>, SM); e != cudaSuccess) return e;
-        ::qgn::launch(k_wgrad_tc<CIN, COUT>, 3 * chunks, kRoleThreads, SM, n->stream, x, g, batch, n->H, n->W, n->part,
-                      n->bpart, n->d_err);
-        return cudaGetLastError();
+    if (n->engine != 1) {
+        if constexpr (COUT == 64) return launch_wgrad_tc<CIN, false>(n, x, g, batch, nchunks);
+        else return launch_wgrad_tc<COUT, true>(n, g, x, batch, nchunks);
     }
     const int chunks = (batch * n->H + kWChunkRows - 1) / kWChunkRows;
     *nchunks = chunks;
@@ -1501,18 +1759,17 @@ int backward(qgn_cnn* net, int batch) {
         int chunks = 0;
         NCK(launch_wgrad(net, net->ci[l], net->co[l], net->act[l], gcur, batch, &chunks));
         const int nw = 9 * net->co[l] * net->ci[l];
-        ::qgn::launch(k_reduce_wgrad, (nw + 255) / 256, 256, 0, net->stream, net->part, chunks, nw, net->gw[l]);
-        NCK(cudaGetLastError());
         const float* bpart = net->bpart;
         int nbias = chunks;
         if (net->engine == 1) {
             const int ppb = 1024;
             nbias = (int)((np + ppb - 1) / ppb);
-            ::qgn::launch(k_bias_part, nbias, 64, 0, net->stream, gcur, np, net->co[l], ppb, net->part);
+            ::qgn::launch(k_bias_part, nbias, 64, 0, net->stream, gcur, np, net->co[l], ppb, net->part + (size_t)chunks * nw);
             NCK(cudaGetLastError());
-            bpart = net->part;
+            bpart = net->part + (size_t)chunks * nw;
         }
-        ::qgn::launch(k_reduce_wgrad, 1, 64, 0, net->stream, bpart, nbias, net->co[l], net->gb[l]);
+        ::qgn::launch(k_reduce_wgrad, (nw + kRedOut - 1) / kRedOut + 1, 4 * kRedOut, 0, net->stream, net->part, chunks, nw,
+                      net->gw[l], bpart, nbias, net->co[l], net->gb[l]);
         NCK(cudaGetLastError());
         if (l > 0) {
             NCK(launch_conv<EPI_GELU_GRAD>(net, net->co[l], net->ci[l], gcur, net->wb[l], nullptr, batch, nullptr,
@@ -1681,6 +1938,8 @@ int qgn_cnn_create(int cin, int width, int cout, int layers, int H, int W, int m
         net->gb[l] = net->grads + np;
         np += net->co[l];
     }
+    // most partials of any batch up to max_batch: 148, or one per kWgRows rows
+    const size_t max_chunks = std::max<size_t>(148, ((size_t)max_batch * H * (W / kTileP) + kWgRows - 1) / kWgRows);
     std::mt19937_64 rng(seed);
     for (int l = 0; l < layers; ++l) {
         const int nw = 9 * net->co[l] * net->ci[l];
@@ -1703,10 +1962,10 @@ int qgn_cnn_create(int cin, int width, int cout, int layers, int H, int W, int m
         ::qgn::launch(k_weights_bf16, (nw + 255) / 256, 256, 0, net->stream, net->w[l], nw, net->co[l], net->ci[l], net->wf[l],
                                                                   net->wb[l]);
         const size_t chunks = (size_t)((max_batch * H + kWChunkRows - 1) / kWChunkRows);
-        part = std::max(part, std::max(chunks, (size_t)kWgChunks) * nw);
-        part = std::max(part, ((NP + 1023) / 1024) * (size_t)net->co[l]);
+        // (the mma.sync engine's bias partials follow its weight partials)
+        part = std::max(part, std::max(chunks * nw + ((NP + 1023) / 1024) * (size_t)net->co[l], max_chunks * nw));
     }
-    if (nalloc(net, &net->bpart, (size_t)kWgChunks * net->width) || nalloc(net, &net->act[layers], 16) || nalloc(net, &net->gA, NP * net->width) ||
+    if (nalloc(net, &net->bpart, max_chunks * net->width) || nalloc(net, &net->act[layers], 16) || nalloc(net, &net->gA, NP * net->width) ||
         nalloc(net, &net->gB, NP * net->width) || nalloc(net, &net->part, part) ||
         nalloc(net, &net->loss_part, 148) || nalloc(net, &net->ytgt, NP * pad16(cout)) ||
         nalloc(net, &net->d_err, 1) || nalloc(net, &net->flags, 1024))
