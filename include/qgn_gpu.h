@@ -221,7 +221,7 @@ int qgn_rhs_static(const qgn_params* p, const double* H, const double* uBar, con
  * contexts made by qgn_create with scheme QGN_SCHEME_BSRK3 and precision QGN_PREC_FP64 --
  * advanced together with BSRK3.f90's scheme.  Grid sizes nx, ny in {128, 256, 512} and
  * layer counts 2..8 or 16 may differ between members; C_d must be 0.  Each pass of an
- * attempt is one launch for all members, the attempts run as a device-conditioned CUDA
+ * attempt is one launch for all members (the x pass: one per grid size), the attempts run as a device-conditioned CUDA
  * graph loop, and the first advance autotunes the tile widths and grid sizes.
  *
  * The ensemble borrows the contexts (they must outlive it) and works on their buffers:
@@ -241,7 +241,8 @@ int qgn_ens_tuning(qgn_ens* ens, int pass, int* threads, int* ctas_per_sm, float
  * a transform of n points runs on n / that many threads, in radix passes of that size) */
 int qgn_ens_fft_radix(qgn_ens* ens, int pass, int* elements_per_thread);
 /* pin a pass to one tile variant instead of tuning it: CTA threads (as qgn_ens_tuning reports
- * them), elements per thread and CTAs per SM (0 = one CTA per tile).  Variants: y-inverse
+ * them), elements per thread and CTAs per SM (0 = one CTA per tile; the x pass always takes one
+ * CTA per tile and limits the CTAs resident on an SM to this many).  Variants: y-inverse
  * 64/128/256 threads at 16 or 8 elements, x pass 96/192/384 at 16 and 192/384 at 8, y-forward
  * 64/128/256 at 16 and 128/256 at 8; QGN_PREC_MIXED adds 32 elements (y-inverse 64/128/256,
  * x pass 96/192/384, y-forward 64/128).  QGN_ERR_CONFIG for any other combination. */

@@ -3,8 +3,8 @@
 //
 // Every pass of an attempt -- stage combination + GetPsi, the three right-hand-side passes,
 // the error combination, the error transform and the controller -- is ONE launch for the
-// whole ensemble: a table of tile counts maps each CTA of a persistent grid-stride loop to
-// a member and a tile, and the tile bodies of the single-field kernels (rhs_tiles.cuh) run
+// whole ensemble (the x pass: one per grid size): a table maps each CTA, or each turn of a
+// persistent grid-stride loop, to a member and a tile, and the tile bodies of the single-field kernels (rhs_tiles.cuh) run
 // on it with the member's geometry.  All members take their attempts in lockstep; members
 // that have taken their steps (or halted) drop out of the tile loops.  The attempts of an
 // advance run as the body of a CUDA graph WHILE node whose condition the controller kernel
@@ -114,15 +114,14 @@ __host__ __device__ constexpr int ens_regcap() {
 }
 constexpr int kPointTile = 256;
 
-__device__ __forceinline__ int ens_find(const int* __restrict__ start, int nm, int t) {
-    int lo = 0, hi = nm - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (start[mid] <= t) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
+// The tiles of a pass: tile t is tile t - start[i] of entry i = map[t] (a member, or a member of a
+// group).  Looked up, not searched for: five dependent loads before a CTA knew its member were a good
+// part of the short kernels.
+struct TileTab {
+    const int* start;
+    const int* map;
+    int total;
+};
 
 // stage 0 is the FSAL evaluation RHS0 = GetRHS(q_hat) (BSRK3.f90:12-17), stages 1..3 the
 // attempt's stages; a member takes part in a pass when it needs that evaluation
@@ -150,83 +149,100 @@ __device__ __forceinline__ const CT* stage_input(const EnsMember& M, int s) {
 }
 
 // ---- stage combination + GetPsi (BSRK3.f90:21-28, QGN_Module.f90:315-341) ------------------
+// One mode, all layers per thread.  The state and right-hand sides are requested before the mode
+// matrices are staged, so that the tile's two dependent rounds of loads overlap; a noinline body
+// per layer count, called after the staging, read them one round later: 32 members of 128^2 to 512^2
+// took 106 us (FP32), now 72 us.  Latency-bound still: 16 warps per SM at 128 registers.
+struct EnsModes {
+    double proj[kMaxNZ * kMaxNZ], back[kMaxNZ * kMaxNZ], ev[kMaxNZ];
+};
+
 template <int NZ, class CT>
-__device__ __noinline__ void ens_stage_point(const EnsMember& M, const Geom& g, size_t p, int s,
-                                                const double* proj, const double* back, const double* ev) {
-    constexpr int NZC = NZ > 0 ? NZ : kMaxNZ;
-    const int nz = NZ > 0 ? NZ : g.nz;
-    const size_t P = (size_t)g.nkx * g.nky;
-    const int kx = (int)(p / g.nky), m = (int)(p % g.nky);
-    const double kxv = g.dkx * kx, kyv = g.kyval(g.jfull(m));
-    const double k2 = kxv * kxv + kyv * kyv;
-    const double dt = M.sc->dt;
-    const CT* N0 = static_cast<const CT*>(M.N[0]);
-    const CT* N1 = static_cast<const CT*>(M.N[1]);
-    const CT* N2 = static_cast<const CT*>(M.N[2]);
-    double2 qv[NZC], pv[NZC];
+__device__ __forceinline__ void ens_stage_tile(const EnsMember& M, const Geom& g, int tile, int s, EnsModes& sm) {
+    const unsigned P = (unsigned)(g.nkx * g.nky);
+    const unsigned p = (unsigned)tile * kPointTile + threadIdx.x;
+    const bool ok = p < P;
+    double2 qv[NZ], pv[NZ];
+    if (ok) {
+        const double dt = M.sc->dt;
+        const double2* q = M.q;
 #pragma unroll
-    for (int l = 0; l < NZC; ++l) {
-        if (l < nz) {
-            const size_t idx = (size_t)l * P + p;
-            double2 v = M.q[idx];
-            if (s == 1) {
-                axpy(v, 0.5 * dt, N0[idx]);
-            } else if (s == 2) {
-                axpy(v, 0.75 * dt, N1[idx]);
-            } else if (s == 3) {
-                axpy(v, (2.0 / 9.0) * dt, N0[idx]);
-                axpy(v, (1.0 / 3.0) * dt, N1[idx]);
-                axpy(v, (4.0 / 9.0) * dt, N2[idx]);
+        for (int l = 0; l < NZ; ++l) qv[l] = q[(size_t)l * P + p];
+        auto coef = [&](int j) {
+            return (s == 1 ? 0.5 : s == 2 ? 0.75 : j == 0 ? 2.0 / 9.0 : j == 1 ? 1.0 / 3.0 : 4.0 / 9.0) * dt;
+        };
+        const int first = s == 2 ? 1 : 0, last = s == 3 ? 2 : s - 1;
+        if (sizeof(CT) == 8 && s == 3) {   // FP32: all three right-hand sides requested at once
+            CT r[3][NZ];
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int l = 0; l < NZ; ++l) r[j][l] = (static_cast<const CT*>(M.N[j]) + p)[(size_t)l * P];
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int l = 0; l < NZ; ++l) axpy(qv[l], coef(j), r[j][l]);
+        } else {
+#pragma unroll 1
+            for (int j = first; j <= last; ++j) {   // FP64: one right-hand side's layers at a time
+                const double c = coef(j);
+                const CT* R = static_cast<const CT*>(M.N[j]) + p;
+                CT r[NZ];
+#pragma unroll
+                for (int l = 0; l < NZ; ++l) r[l] = R[(size_t)l * P];
+#pragma unroll
+                for (int l = 0; l < NZ; ++l) axpy(qv[l], c, r[l]);
             }
-            qv[l] = v;
         }
     }
-    modal_invert<NZ>(proj, back, ev, M.mc->Htot, nz, k2, p == 0, qv, pv);
+    for (int i = threadIdx.x; i < NZ * NZ; i += kPointTile) {
+        sm.proj[i] = M.mc->proj[i];
+        sm.back[i] = M.mc->back[i];
+    }
+    if (threadIdx.x < NZ) sm.ev[threadIdx.x] = M.mc->evals[threadIdx.x];
+    __syncthreads();
+    if (!ok) return;
+    const int kx = (int)(p / (unsigned)g.nky), m = (int)(p % (unsigned)g.nky);
+    const double kxv = g.dkx * kx, kyv = g.kyval(g.jfull(m));
+    const double k2 = kxv * kxv + kyv * kyv;
+    modal_invert<NZ>(sm.proj, sm.back, sm.ev, M.mc->Htot, NZ, k2, p == 0, qv, pv);
     CT* Qs = const_cast<CT*>(stage_input<CT>(M, s));
     CT* psi = static_cast<CT*>(M.psi);
+    const bool keep = sizeof(CT) == 8 && s == 3;   // the FP64 candidate of the mixed mode
 #pragma unroll
-    for (int l = 0; l < NZC; ++l) {
-        if (l < nz) {
-            const size_t idx = (size_t)l * P + p;
-            Qs[idx] = to_ct<CT>(qv[l]);
-            psi[idx] = to_ct<CT>(pv[l]);
-            if (sizeof(CT) == 8 && s == 3) M.qc[idx] = qv[l];
-        }
+    for (int l = 0; l < NZ; ++l) {
+        const size_t idx = (size_t)l * P + p;
+        Qs[idx] = to_ct<CT>(qv[l]);
+        psi[idx] = to_ct<CT>(pv[l]);
+        if (keep) M.qc[idx] = qv[l];
     }
 }
 
-template <class CT>
-__global__ void __launch_bounds__(256, 2) k_ens_stage(const EnsMember* __restrict__ mem, const int* __restrict__ start,
-                                                   int nm, int s) {
+// one CTA per tile (in a loop over tiles every form of this spilled kilobytes per thread); NZ16: some
+// member has 16 layers
+template <class CT, bool NZ16>
+__global__ void __launch_bounds__(kPointTile, 2)
+    k_ens_stage(const EnsMember* __restrict__ mem, TileTab tab, int s) {
     QGN_PDL_ENTRY();
-    __shared__ double s_proj[kMaxNZ * kMaxNZ], s_back[kMaxNZ * kMaxNZ], s_ev[kMaxNZ];
-    const int total = start[nm];
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        const int mi = ens_find(start, nm, t);
-        const EnsMember& M = mem[mi];
-        if (!ens_runs(M, s)) continue;
-        const Geom g = M.g;
-        const int nz = g.nz;
-        __syncthreads();   // the previous tile's readers of the mode tables are done
-        for (int i = threadIdx.x; i < nz * nz; i += blockDim.x) {
-            s_proj[i] = M.mc->proj[i];
-            s_back[i] = M.mc->back[i];
-        }
-        for (int i = threadIdx.x; i < nz; i += blockDim.x) s_ev[i] = M.mc->evals[i];
-        __syncthreads();
-        const size_t p = (size_t)(t - start[mi]) * kPointTile + threadIdx.x;
-        if (p >= (size_t)g.nkx * g.nky) continue;
-        switch (nz) {
-            case 2: ens_stage_point<2, CT>(M, g, p, s, s_proj, s_back, s_ev); break;
-            case 3: ens_stage_point<3, CT>(M, g, p, s, s_proj, s_back, s_ev); break;
-            case 4: ens_stage_point<4, CT>(M, g, p, s, s_proj, s_back, s_ev); break;
-            case 5: ens_stage_point<5, CT>(M, g, p, s, s_proj, s_back, s_ev); break;
-            case 6: ens_stage_point<6, CT>(M, g, p, s, s_proj, s_back, s_ev); break;
-            case 7: ens_stage_point<7, CT>(M, g, p, s, s_proj, s_back, s_ev); break;
-            case 8: ens_stage_point<8, CT>(M, g, p, s, s_proj, s_back, s_ev); break;
-            case 16: ens_stage_point<16, CT>(M, g, p, s, s_proj, s_back, s_ev); break;
-            default: break;   // qgn_ens_create admits these layer counts only
-        }
+    __shared__ EnsModes sm;
+    const int t = blockIdx.x;
+    const int mi = tab.map[t];
+    const EnsMember& M = mem[mi];
+    if (!ens_runs(M, s)) return;
+    const Geom g = M.g;
+    const int tile = t - tab.start[mi];
+    switch (g.nz) {
+        case 2: ens_stage_tile<2, CT>(M, g, tile, s, sm); break;
+        case 3: ens_stage_tile<3, CT>(M, g, tile, s, sm); break;
+        case 4: ens_stage_tile<4, CT>(M, g, tile, s, sm); break;
+        case 5: ens_stage_tile<5, CT>(M, g, tile, s, sm); break;
+        case 6: ens_stage_tile<6, CT>(M, g, tile, s, sm); break;
+        case 7: ens_stage_tile<7, CT>(M, g, tile, s, sm); break;
+        case 8: ens_stage_tile<8, CT>(M, g, tile, s, sm); break;
+        case 16:
+            if constexpr (NZ16) ens_stage_tile<16, CT>(M, g, tile, s, sm);
+            break;
+        default: break;   // qgn_ens_create admits these layer counts only
     }
 }
 
@@ -236,22 +252,21 @@ __device__ __noinline__ void ens_yinv_one(const EnsMember& M, const Geom& g, int
     using C = YInvCfg<N, CT, TV>;
     static_assert(C::THREADS == tv_width(TV), "y-inverse tile width must give TV threads");
     const int nbx = (g.nkx + C::TKX - 1) / C::TKX;
-    yinv_tile<N, 3, CT, TV>(g, local % nbx, local / nbx, stage_input<CT>(M, s), static_cast<const CT*>(M.psi),
+    yinv_tile<N, 3, CT, TV>(g, threadIdx.x, local % nbx, local / nbx, stage_input<CT>(M, s), static_cast<const CT*>(M.psi),
                             static_cast<CT*>(M.hq), static_cast<CT*>(M.hp), static_cast<CT*>(M.hu),
                             static_cast<const CT*>(M.twy));
 }
 
 template <class CT, int TV>
 __global__ void __launch_bounds__(tv_width(TV), minb(tv_width(TV), ens_regcap<CT, TV>()))
-    k_ens_yinv(const EnsMember* __restrict__ mem, const int* __restrict__ start, int nm, int s) {
+    k_ens_yinv(const EnsMember* __restrict__ mem, TileTab tab, int s) {
     QGN_PDL_ENTRY();
-    const int total = start[nm];
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        const int mi = ens_find(start, nm, t);
+    for (int t = blockIdx.x; t < tab.total; t += gridDim.x) {
+        const int mi = tab.map[t];
         const EnsMember& M = mem[mi];
         if (!ens_runs(M, s)) continue;
         const Geom g = M.g;
-        const int local = t - start[mi];
+        const int local = t - tab.start[mi];
         switch (g.ny) {
             case 128: ens_yinv_one<128, CT, TV>(M, g, local, s); break;
             case 256: ens_yinv_one<256, CT, TV>(M, g, local, s); break;
@@ -262,35 +277,31 @@ __global__ void __launch_bounds__(tv_width(TV), minb(tv_width(TV), ens_regcap<CT
     }
 }
 
+// The x pass of the members of one grid size (idx: their numbers).  The
+// geometry is a kernel parameter, the row length a constant, and a CTA takes one tile: in a loop over
+// tiles, the same body spills 0.4 to 0.8 KB per thread (in FP32 as well, at 96 registers), whether it
+// is inlined or called, and in a call it also saves its registers on entry.  32 members of 128^2 to
+// 512^2, FP32: one looping launch for all sizes 181 us, the three launches 112 us.
 template <int N, class CT, int TV>
-__device__ __noinline__ void ens_xpass_one(const EnsMember& M, const Geom& g, int local) {
+__global__ void __launch_bounds__(3 * tv_width(TV), minb(3 * tv_width(TV), ens_regcap<CT, TV>()))
+    k_ens_xpass(Geom g, const EnsMember* __restrict__ mem, const int* __restrict__ idx, TileTab tab, int s) {
+    QGN_PDL_ENTRY();
     using C = XCfg<N, false, CT, TV>;
     static_assert(C::THREADS == 3 * tv_width(TV), "x-pass tile width must give 3 TV threads");
     const int nbx = (g.ny / 2 + C::RP - 1) / C::RP;
-    xpass_tile<N, false, CT, TV>(g, local % nbx, local / nbx, static_cast<const CT*>(M.hq),
+    const int t = blockIdx.x;
+    const int gi = tab.map[t];
+    const EnsMember& M = mem[idx[gi]];
+    if (!ens_runs(M, s)) return;
+    const int local = t - tab.start[gi];
+#ifdef QGN_CHECK
+    Geom gm = M.g;     // this member's layer count bounds the checked indices
+#else
+    const Geom& gm = g;
+#endif
+    xpass_tile<N, false, CT, TV>(gm, threadIdx.x, local % nbx, local / nbx, static_cast<const CT*>(M.hq),
                                  static_cast<const CT*>(M.hp), static_cast<const CT*>(M.hu), static_cast<CT*>(M.hpp),
                                  static_cast<CT*>(M.hpd), static_cast<const CT*>(M.twx));
-}
-
-template <class CT, int TV>
-__global__ void __launch_bounds__(3 * tv_width(TV), minb(3 * tv_width(TV), ens_regcap<CT, TV>()))
-    k_ens_xpass(const EnsMember* __restrict__ mem, const int* __restrict__ start, int nm, int s) {
-    QGN_PDL_ENTRY();
-    const int total = start[nm];
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        const int mi = ens_find(start, nm, t);
-        const EnsMember& M = mem[mi];
-        if (!ens_runs(M, s)) continue;
-        const Geom g = M.g;
-        const int local = t - start[mi];
-        switch (g.nx) {
-            case 128: ens_xpass_one<128, CT, TV>(M, g, local); break;
-            case 256: ens_xpass_one<256, CT, TV>(M, g, local); break;
-            case 512: ens_xpass_one<512, CT, TV>(M, g, local); break;
-            default: break;
-        }
-        __syncthreads();
-    }
 }
 
 template <int N, class CT, int TV>
@@ -298,7 +309,7 @@ __device__ __noinline__ void ens_yfwd_one(const EnsMember& M, const Geom& g, int
     using C = YFwdCfg<N, false, CT, TV>;
     static_assert(C::THREADS == tv_width(TV), "y-forward tile width must give TV threads");
     const int nbx = (g.nkx + C::TKX - 1) / C::TKX;
-    yfwd_tile<N, false, CT, TV>(g, local % nbx, local / nbx, M.lc, stage_input<CT>(M, s),
+    yfwd_tile<N, false, CT, TV>(g, threadIdx.x, local % nbx, local / nbx, M.lc, stage_input<CT>(M, s),
                                 static_cast<const CT*>(M.psi), static_cast<const CT*>(M.hpp),
                                 static_cast<const CT*>(M.hpd), static_cast<CT*>(M.N[s]),
                                 static_cast<const CT*>(M.twy));
@@ -306,15 +317,14 @@ __device__ __noinline__ void ens_yfwd_one(const EnsMember& M, const Geom& g, int
 
 template <class CT, int TV>
 __global__ void __launch_bounds__(tv_width(TV), minb(tv_width(TV), ens_regcap<CT, TV>()))
-    k_ens_yfwd(const EnsMember* __restrict__ mem, const int* __restrict__ start, int nm, int s) {
+    k_ens_yfwd(const EnsMember* __restrict__ mem, TileTab tab, int s) {
     QGN_PDL_ENTRY();
-    const int total = start[nm];
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        const int mi = ens_find(start, nm, t);
+    for (int t = blockIdx.x; t < tab.total; t += gridDim.x) {
+        const int mi = tab.map[t];
         const EnsMember& M = mem[mi];
         if (!ens_runs(M, s)) continue;
         const Geom g = M.g;
-        const int local = t - start[mi];
+        const int local = t - tab.start[mi];
         switch (g.ny) {
             case 128: ens_yfwd_one<128, CT, TV>(M, g, local, s); break;
             case 256: ens_yfwd_one<256, CT, TV>(M, g, local, s); break;
@@ -327,14 +337,13 @@ __global__ void __launch_bounds__(tv_width(TV), minb(tv_width(TV), ens_regcap<CT
 
 // ---- embedded error (BSRK3.f90:30-34), FP64 -------------------------------------------------
 template <class CT>
-__global__ void __launch_bounds__(256) k_ens_err(EnsMember* __restrict__ mem, const int* __restrict__ start, int nm) {
+__global__ void __launch_bounds__(256) k_ens_err(EnsMember* __restrict__ mem, TileTab tab) {
     QGN_PDL_ENTRY();
-    const int total = start[nm];
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        const int mi = ens_find(start, nm, t);
+    for (int t = blockIdx.x; t < tab.total; t += gridDim.x) {
+        const int mi = tab.map[t];
         const EnsMember& M = mem[mi];
         if (!M.active) continue;
-        const int local = t - start[mi];
+        const int local = t - tab.start[mi];
         if (local == 0 && threadIdx.x == 0) {
             M.sc->maxbits = 0ULL;
             M.sc->accept = 0;
@@ -356,20 +365,19 @@ __device__ __noinline__ void ens_yinv1_one(const EnsMember& M, const Geom& g, in
     using C = YInvCfg<N, double2, 128>;
     static_assert(C::THREADS == 128, "");
     const int nbx = (g.nkx + C::TKX - 1) / C::TKX;
-    yinv_tile<N, 1, double2, 128>(g, local % nbx, local / nbx, M.err, nullptr, static_cast<double2*>(M.hq), nullptr,
+    yinv_tile<N, 1, double2, 128>(g, threadIdx.x, local % nbx, local / nbx, M.err, nullptr, static_cast<double2*>(M.hq), nullptr,
                                   nullptr, M.twy64);
 }
 
 __global__ void __launch_bounds__(128, minb(128)) k_ens_yinv1(const EnsMember* __restrict__ mem,
-                                                              const int* __restrict__ start, int nm) {
+                                                              TileTab tab) {
     QGN_PDL_ENTRY();
-    const int total = start[nm];
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        const int mi = ens_find(start, nm, t);
+    for (int t = blockIdx.x; t < tab.total; t += gridDim.x) {
+        const int mi = tab.map[t];
         const EnsMember& M = mem[mi];
         if (!M.active) continue;
         const Geom g = M.g;
-        const int local = t - start[mi];
+        const int local = t - tab.start[mi];
         switch (g.ny) {
             case 128: ens_yinv1_one<128>(M, g, local); break;
             case 256: ens_yinv1_one<256>(M, g, local); break;
@@ -389,15 +397,14 @@ __device__ __noinline__ void ens_xinv1_one(const EnsMember& M, const Geom& g, in
 }
 
 __global__ void __launch_bounds__(128, minb(128)) k_ens_xinv1(const EnsMember* __restrict__ mem,
-                                                              const int* __restrict__ start, int nm) {
+                                                              TileTab tab) {
     QGN_PDL_ENTRY();
-    const int total = start[nm];
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        const int mi = ens_find(start, nm, t);
+    for (int t = blockIdx.x; t < tab.total; t += gridDim.x) {
+        const int mi = tab.map[t];
         const EnsMember& M = mem[mi];
         if (!M.active) continue;
         const Geom g = M.g;
-        const int local = t - start[mi];
+        const int local = t - tab.start[mi];
         switch (g.nx) {
             case 128: ens_xinv1_one<128>(M, g, local); break;
             case 256: ens_xinv1_one<256>(M, g, local); break;
@@ -473,10 +480,6 @@ constexpr int yinv_smem() {
     return cmax(YInvCfg<128, CT, TV>::SMEM, cmax(YInvCfg<256, CT, TV>::SMEM, YInvCfg<512, CT, TV>::SMEM));
 }
 template <class CT, int TV>
-constexpr int xpass_smem() {
-    return cmax(XCfg<128, false, CT, TV>::SMEM, cmax(XCfg<256, false, CT, TV>::SMEM, XCfg<512, false, CT, TV>::SMEM));
-}
-template <class CT, int TV>
 constexpr int yfwd_smem() {
     return cmax(YFwdCfg<128, false, CT, TV>::SMEM,
                 cmax(YFwdCfg<256, false, CT, TV>::SMEM, YFwdCfg<512, false, CT, TV>::SMEM));
@@ -526,6 +529,20 @@ struct qgn_ens {
     std::vector<EnsMember> h_mem;
     int* d_start = nullptr;          // EP_COUNT tables of nm+1 prefix sums
     std::vector<int> h_start;
+    std::vector<int> h_map;          // tile -> member of every pass, the pass's part at map_at[pass]
+    int map_at[EP_COUNT] = {};
+    int* d_map = nullptr;
+    size_t map_cap = 0;              // entries of d_map
+    // members of one grid size, for the x pass: their numbers and tile prefix sums at `table` of d_xgroups
+    struct XGroup {
+        int nx, ny;
+        std::vector<int> members;
+        int table = 0, tiles = 0, map_at = 0;
+    };
+    std::vector<XGroup> xgroups;
+    std::vector<int> h_xgroups;      // per group: members, then their count + 1 prefix sums (tile -> member of
+                                     // the group: h_map at map_at)
+    int* d_xgroups = nullptr;
     int* d_any = nullptr;
     int* h_any = nullptr;            // pinned
     int variant[TP_COUNT] = {kDefaultVariant, kDefaultVariant, kDefaultVariant};
@@ -574,9 +591,11 @@ int variant_count(const qgn_ens* e, int tp) {
     return fp32(e) ? ens_variant_count<float2>(tp) : ens_variant_count<double2>(tp);
 }
 
-const int* start_of(const qgn_ens* e, int pass) { return e->d_start + (size_t)pass * (e->mem.size() + 1); }
-
 int total_of(const qgn_ens* e, int pass) { return e->h_start[(size_t)pass * (e->mem.size() + 1) + e->mem.size()]; }
+
+TileTab tab_of(const qgn_ens* e, int pass) {
+    return TileTab{e->d_start + (size_t)pass * (e->mem.size() + 1), e->d_map + e->map_at[pass], total_of(e, pass)};
+}
 
 int grid_for(const qgn_ens* e, int pass, int tp) {
     const int total = total_of(e, pass);
@@ -587,18 +606,73 @@ int grid_for(const qgn_ens* e, int pass, int tp) {
 void build_tables(qgn_ens* e) {
     const size_t nm = e->mem.size();
     e->h_start.assign((size_t)EP_COUNT * (nm + 1), 0);
+    e->h_map.clear();
     for (int pass = 0; pass < EP_COUNT; ++pass) {
         int tv = 0;
         if (pass == EP_YINV) tv = tv_of(e, TP_YINV);
         if (pass == EP_XPASS) tv = tv_of(e, TP_XPASS);
         if (pass == EP_YFWD) tv = tv_of(e, TP_YFWD);
         int* st = &e->h_start[(size_t)pass * (nm + 1)];
-        for (size_t m = 0; m < nm; ++m) st[m + 1] = st[m] + member_tiles(e->mem[m]->g, pass, tv);
+        e->map_at[pass] = (int)e->h_map.size();
+        for (size_t m = 0; m < nm; ++m) {
+            st[m + 1] = st[m] + member_tiles(e->mem[m]->g, pass, tv);
+            e->h_map.resize(e->map_at[pass] + st[m + 1], (int)m);
+        }
+    }
+    const int xtv = tv_of(e, TP_XPASS);
+    e->h_xgroups.clear();
+    for (qgn_ens::XGroup& x : e->xgroups) {
+        x.table = (int)e->h_xgroups.size();
+        e->h_xgroups.insert(e->h_xgroups.end(), x.members.begin(), x.members.end());
+        x.map_at = (int)e->h_map.size();
+        int sum = 0;
+        for (size_t i = 0; i < x.members.size(); ++i) {
+            e->h_xgroups.push_back(sum);
+            sum += member_tiles(e->mem[x.members[i]]->g, EP_XPASS, xtv);
+            e->h_map.resize(x.map_at + sum, (int)i);
+        }
+        e->h_xgroups.push_back(sum);
+        x.tiles = sum;
     }
 }
 
+// the grid sizes of the members, largest first (the tail of a large launch costs the most)
+void group_members(qgn_ens* e) {
+    for (size_t m = 0; m < e->mem.size(); ++m) {
+        const Geom& g = e->mem[m]->g;
+        auto it = std::find_if(e->xgroups.begin(), e->xgroups.end(),
+                               [&](const qgn_ens::XGroup& x) { return x.nx == g.nx && x.ny == g.ny; });
+        if (it == e->xgroups.end()) {
+            qgn_ens::XGroup x;
+            x.nx = g.nx;
+            x.ny = g.ny;
+            e->xgroups.push_back(x);
+            it = e->xgroups.end() - 1;
+        }
+        it->members.push_back((int)m);
+    }
+    std::sort(e->xgroups.begin(), e->xgroups.end(), [](const qgn_ens::XGroup& a, const qgn_ens::XGroup& b) {
+        return (long long)a.nx * a.ny * (1 << 12) + a.nx > (long long)b.nx * b.ny * (1 << 12) + b.nx;
+    });
+}
+
 int upload_tables(qgn_ens* e) {
+    if (e->h_map.size() > e->map_cap) {   // (a captured graph holds the old address)
+        if (e->gexec) {
+            ECK(cudaStreamSynchronize(e->stream));
+            cudaGraphExecDestroy(e->gexec);
+            e->gexec = nullptr;
+        }
+        if (e->d_map) ECK(cudaFree(e->d_map));
+        e->d_map = nullptr;
+        e->map_cap = 0;
+        ECK(cudaMalloc((void**)&e->d_map, sizeof(int) * e->h_map.size()));
+        e->map_cap = e->h_map.size();
+    }
+    ECK(cudaMemcpyAsync(e->d_map, e->h_map.data(), sizeof(int) * e->h_map.size(), cudaMemcpyHostToDevice, e->stream));
     ECK(cudaMemcpyAsync(e->d_start, e->h_start.data(), sizeof(int) * e->h_start.size(), cudaMemcpyHostToDevice,
+                        e->stream));
+    ECK(cudaMemcpyAsync(e->d_xgroups, e->h_xgroups.data(), sizeof(int) * e->h_xgroups.size(), cudaMemcpyHostToDevice,
                         e->stream));
     return QGN_OK;
 }
@@ -642,9 +716,11 @@ template <class CT>
 int launch_stage(qgn_ens* e, int s) {
     double bytes = 0.0;
     for (qgn_ctx* c : e->mem) bytes += (double)c->g.csize() * (16.0 + 2.0 * sizeof(CT) + (s == 3 ? 3 : (s ? 1 : 0)) * sizeof(CT));
+    bool nz16 = false;
+    for (qgn_ctx* c : e->mem) nz16 = nz16 || c->g.nz == 16;
     QGN_LAUNCH(KID_STAGE, bytes, e->stream,
-               ::qgn::launch(k_ens_stage<CT>, grid_for(e, EP_POINT, -1), kPointTile, 0, e->stream, e->d_mem, start_of(e, EP_POINT),
-                                                                                        (int)e->mem.size(), s));
+               ::qgn::launch(nz16 ? k_ens_stage<CT, true> : k_ens_stage<CT, false>, grid_for(e, EP_POINT, -1), kPointTile, 0,
+                             e->stream, e->d_mem, tab_of(e, EP_POINT), s));
     ECK(cudaGetLastError());
     return QGN_OK;
 }
@@ -656,22 +732,45 @@ int launch_yinv_tv(qgn_ens* e, int s, int grid) {
     double bytes = 0.0;
     for (qgn_ctx* c : e->mem) bytes += sizeof(CT) * (2.0 * c->g.csize() + 3.0 * c->g.nz * c->g.ny * c->g.nkx);
     QGN_LAUNCH(KID_YINV, bytes, e->stream,
-               ::qgn::launch(k_ens_yinv<CT, TV>, grid, tv_width(TV), SM, e->stream, e->d_mem, start_of(e, EP_YINV),
-                             (int)e->mem.size(), s));
+               ::qgn::launch(k_ens_yinv<CT, TV>, grid, tv_width(TV), SM, e->stream, e->d_mem, tab_of(e, EP_YINV), s));
+    ECK(cudaGetLastError());
+    return QGN_OK;
+}
+
+template <int N, class CT, int TV>
+int launch_xgroup(qgn_ens* e, const qgn_ens::XGroup& x, int s) {
+    // one CTA per tile; k > 0 CTAs per SM are a limit on the resident ones, by their shared memory
+    constexpr int kSmShared = 227 * 1024;
+    const int gm = e->grid_mode[TP_XPASS], ng = (int)x.members.size();
+    const int SM = gm == 0 ? XCfg<N, false, CT, TV>::SMEM
+                           : std::max(XCfg<N, false, CT, TV>::SMEM, kSmShared / (gm + 1) / 1024 * 1024);
+    ECK(smem_attr(k_ens_xpass<N, CT, TV>, SM));
+    double bytes = 0.0;
+    for (int m : x.members) {
+        const Geom& g = e->mem[m]->g;
+        bytes += 5.0 * sizeof(CT) * g.nz * g.ny * g.nkx;
+    }
+    const int grid = std::max(1, x.tiles);
+    const int* idx = e->d_xgroups + x.table;
+    QGN_LAUNCH(KID_XPASS, bytes, e->stream,
+               ::qgn::launch(k_ens_xpass<N, CT, TV>, grid, 3 * tv_width(TV), SM, e->stream, e->mem[x.members[0]]->g, e->d_mem,
+                             idx, TileTab{idx + ng, e->d_map + x.map_at, x.tiles}, s));
     ECK(cudaGetLastError());
     return QGN_OK;
 }
 
 template <class CT, int TV>
-int launch_xpass_tv(qgn_ens* e, int s, int grid) {
-    constexpr int SM = xpass_smem<CT, TV>();
-    ECK(smem_attr(k_ens_xpass<CT, TV>, SM));
-    double bytes = 0.0;
-    for (qgn_ctx* c : e->mem) bytes += 5.0 * sizeof(CT) * c->g.nz * c->g.ny * c->g.nkx;
-    QGN_LAUNCH(KID_XPASS, bytes, e->stream,
-               ::qgn::launch(k_ens_xpass<CT, TV>, grid, 3 * tv_width(TV), SM, e->stream, e->d_mem, start_of(e, EP_XPASS),
-                                                                   (int)e->mem.size(), s));
-    ECK(cudaGetLastError());
+int launch_xpass_tv(qgn_ens* e, int s) {
+    for (const qgn_ens::XGroup& x : e->xgroups) {
+        int r = QGN_ERR_CONFIG;
+        switch (x.nx) {
+            case 128: r = launch_xgroup<128, CT, TV>(e, x, s); break;
+            case 256: r = launch_xgroup<256, CT, TV>(e, x, s); break;
+            case 512: r = launch_xgroup<512, CT, TV>(e, x, s); break;
+            default: break;
+        }
+        if (r != QGN_OK) return r;
+    }
     return QGN_OK;
 }
 
@@ -682,8 +781,7 @@ int launch_yfwd_tv(qgn_ens* e, int s, int grid) {
     double bytes = 0.0;
     for (qgn_ctx* c : e->mem) bytes += sizeof(CT) * c->g.nz * c->g.nkx * (2.0 * c->g.ny + 3.0 * c->g.nky);
     QGN_LAUNCH(KID_YFWD, bytes, e->stream,
-               ::qgn::launch(k_ens_yfwd<CT, TV>, grid, tv_width(TV), SM, e->stream, e->d_mem, start_of(e, EP_YFWD),
-                             (int)e->mem.size(), s));
+               ::qgn::launch(k_ens_yfwd<CT, TV>, grid, tv_width(TV), SM, e->stream, e->d_mem, tab_of(e, EP_YFWD), s));
     ECK(cudaGetLastError());
     return QGN_OK;
 }
@@ -699,8 +797,7 @@ int launch_yinv_v(qgn_ens* e, int v, int s, std::index_sequence<I...>) {
 template <class CT, size_t... I>
 int launch_xpass_v(qgn_ens* e, int v, int s, std::index_sequence<I...>) {
     int r = QGN_ERR_CONFIG;
-    const int grid = grid_for(e, EP_XPASS, TP_XPASS);
-    (void)((v == (int)I ? (r = launch_xpass_tv<CT, ens_variant<CT>(TP_XPASS, (int)I)>(e, s, grid), true) : false) || ...);
+    (void)((v == (int)I ? (r = launch_xpass_tv<CT, ens_variant<CT>(TP_XPASS, (int)I)>(e, s), true) : false) || ...);
     return r;
 }
 template <class CT, size_t... I>
@@ -753,17 +850,15 @@ int launch_attempt(qgn_ens* e, const cudaGraphConditionalHandle* loop) {
     }
     const int nm = (int)e->mem.size();
     QGN_LAUNCH(KID_LINCOMB, eb, e->stream,
-               ::qgn::launch(k_ens_err<CT>, grid_for(e, EP_ELEM, -1), kPointTile, 0, e->stream, e->d_mem, start_of(e, EP_ELEM), nm));
+               ::qgn::launch(k_ens_err<CT>, grid_for(e, EP_ELEM, -1), kPointTile, 0, e->stream, e->d_mem, tab_of(e, EP_ELEM)));
     ECK(cudaGetLastError());
     ECK(smem_attr(k_ens_yinv1, yinv1_smem()));
     QGN_LAUNCH(KID_YINV, yb, e->stream,
-               ::qgn::launch(k_ens_yinv1, grid_for(e, EP_YINV1, -1), 128, yinv1_smem(), e->stream, e->d_mem, start_of(e, EP_YINV1),
-                                                                                      nm));
+               ::qgn::launch(k_ens_yinv1, grid_for(e, EP_YINV1, -1), 128, yinv1_smem(), e->stream, e->d_mem, tab_of(e, EP_YINV1)));
     ECK(cudaGetLastError());
     ECK(smem_attr(k_ens_xinv1, xinv1_smem()));
     QGN_LAUNCH(KID_XINV1, xb, e->stream,
-               ::qgn::launch(k_ens_xinv1, grid_for(e, EP_XINV1, -1), 128, xinv1_smem(), e->stream, e->d_mem, start_of(e, EP_XINV1),
-                                                                                      nm));
+               ::qgn::launch(k_ens_xinv1, grid_for(e, EP_XINV1, -1), 128, xinv1_smem(), e->stream, e->d_mem, tab_of(e, EP_XINV1)));
     ECK(cudaGetLastError());
     QGN_LAUNCH(KID_SCALAR, 0.0, e->stream,
                ::qgn::launch(k_ens_ctrl, 1, 256, 0, e->stream, e->d_mem, nm, loop ? *loop : 0, loop ? 1 : 0, e->d_any));
@@ -935,6 +1030,10 @@ int qgn_ens_create(qgn_ctx* const* members, int nmembers, int precision, qgn_ens
     if (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(QGN_ERR_CUDA);
     if (cudaMalloc((void**)&e->d_mem, sizeof(EnsMember) * nmembers) != cudaSuccess) return fail(QGN_ERR_CUDA);
     if (cudaMalloc((void**)&e->d_start, sizeof(int) * (size_t)EP_COUNT * (nmembers + 1)) != cudaSuccess)
+        return fail(QGN_ERR_CUDA);
+    group_members(e);
+    // a group of n members has 2 n + 1 entries
+    if (cudaMalloc((void**)&e->d_xgroups, sizeof(int) * (2 * (size_t)nmembers + e->xgroups.size())) != cudaSuccess)
         return fail(QGN_ERR_CUDA);
     if (cudaMalloc((void**)&e->d_any, sizeof(int)) != cudaSuccess) return fail(QGN_ERR_CUDA);
     if (cudaMallocHost((void**)&e->h_any, sizeof(int)) != cudaSuccess) return fail(QGN_ERR_CUDA);
@@ -1114,6 +1213,8 @@ int qgn_ens_destroy(qgn_ens* e) {
     e->prof.release();
     if (e->d_mem) cudaFree(e->d_mem);
     if (e->d_start) cudaFree(e->d_start);
+    if (e->d_xgroups) cudaFree(e->d_xgroups);
+    if (e->d_map) cudaFree(e->d_map);
     if (e->d_any) cudaFree(e->d_any);
     if (e->h_any) cudaFreeHost(e->h_any);
     if (e->stream) cudaStreamDestroy(e->stream);

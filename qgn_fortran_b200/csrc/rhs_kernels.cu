@@ -44,9 +44,9 @@ __global__ void __launch_bounds__(YInvCfg<NY, CT, TV>::THREADS, minb(YInvCfg<NY,
            CT* __restrict__ pv, CT* __restrict__ pu, const CT* __restrict__ twy) {
     QGN_PDL_ENTRY();
     if constexpr (yinv_spread<NY, CT, TV>() && NF > 1)
-        yinv_tile<NY, NF, CT, TV>(g, blockIdx.x, blockIdx.y, q, psi, pq, pv, pu, twy, blockIdx.z, blockIdx.z + 1);
+        yinv_tile<NY, NF, CT, TV>(g, threadIdx.x, blockIdx.x, blockIdx.y, q, psi, pq, pv, pu, twy, blockIdx.z, blockIdx.z + 1);
     else
-        yinv_tile<NY, NF, CT, TV>(g, blockIdx.x, blockIdx.y, q, psi, pq, pv, pu, twy);
+        yinv_tile<NY, NF, CT, TV>(g, threadIdx.x, blockIdx.x, blockIdx.y, q, psi, pq, pv, pu, twy);
 }
 
 template <int NX, bool DRAG, class CT, int TV = 0>
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(XCfg<NX, DRAG, CT, TV>::THREADS,
             const CT* __restrict__ pu, CT* __restrict__ pp, CT* __restrict__ pd,
             const CT* __restrict__ twx) {
     QGN_PDL_ENTRY();
-    xpass_tile<NX, DRAG, CT, TV>(g, blockIdx.x, blockIdx.y, pq, pv, pu, pp, pd, twx);
+    xpass_tile<NX, DRAG, CT, TV>(g, threadIdx.x, blockIdx.x, blockIdx.y, pq, pv, pu, pp, pd, twx);
 }
 
 template <int NY, bool DRAG, class CT, int TV = 0>
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(YFwdCfg<NY, DRAG, CT, TV>::THREADS,
            CT* __restrict__ out, const CT* __restrict__ twy, const CT* __restrict__ extra) {
     QGN_PDL_ENTRY();
     // with drag, the bottom layer's tiles transform twice: they go first
-    yfwd_tile<NY, DRAG, CT, TV>(g, blockIdx.x, DRAG ? g.nz - 1 - blockIdx.y : blockIdx.y, lc, q, psi, pp, pd, out, twy, extra);
+    yfwd_tile<NY, DRAG, CT, TV>(g, threadIdx.x, blockIdx.x, DRAG ? g.nz - 1 - blockIdx.y : blockIdx.y, lc, q, psi, pp, pd, out, twy, extra);
 }
 
 template <int NX, int EPI, int TV = 0, class CT = double2>

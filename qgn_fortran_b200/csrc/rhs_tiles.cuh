@@ -3,7 +3,7 @@
 // Each body transforms one tile (a group of kx columns or of row pairs of one layer) whose
 // coordinates the caller passes, so the same code serves the single-field launches
 // (tile = blockIdx) and the ensemble launches, where a table maps a CTA to a member and tile.
-// Bodies synchronise the whole CTA: every thread of the CTA must call them.
+// Bodies synchronise the whole CTA: every thread of the CTA must call them with its thread index.
 #pragma once
 #include "qgn_internal.cuh"
 #include "fft.cuh"
@@ -249,7 +249,7 @@ __device__ __forceinline__ bool bar_wait_bounded(uint64_t* bar, uint32_t parity)
 template <int NY, int NF, class CT, int TV = 0>
 // f_begin/f_end: the fields this CTA transforms (all NF by default; one each when a launch
 // spreads the fields over CTAs)
-__device__ __forceinline__ void yinv_tile(const Geom g, int bx, int l, const CT* __restrict__ q,
+__device__ __forceinline__ void yinv_tile(const Geom g, int tid, int bx, int l, const CT* __restrict__ q,
                                           const CT* __restrict__ psi, CT* __restrict__ pq, CT* __restrict__ pv,
                                           CT* __restrict__ pu, const CT* __restrict__ twy, int f_begin = 0,
                                           int f_end = NF) {
@@ -257,7 +257,6 @@ __device__ __forceinline__ void yinv_tile(const Geom g, int bx, int l, const CT*
     using RT = typename CTraits<CT>::R;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     CT* sm = reinterpret_cast<CT*>(sm_raw);
-    const int tid = threadIdx.x;
     const int kx0 = bx * C::TKX;
     const int slot = tid % C::TKX, lane = tid / C::TKX;
     const int kx = kx0 + slot;
@@ -363,14 +362,13 @@ __device__ __forceinline__ void yinv_tile(const Geom g, int bx, int l, const CT*
 // which it replaces, was 15 us of latency per right-hand side (64 CTAs at 512^2).
 // ------------------------------------------------------------------------------------
 template <int NX, bool DRAG, class CT, int TV = 0>
-__device__ __forceinline__ void xpass_tile(const Geom g, int bx, int layer, const CT* __restrict__ pq,
+__device__ __forceinline__ void xpass_tile(const Geom g, int tid, int bx, int layer, const CT* __restrict__ pq,
                                            const CT* __restrict__ pv, const CT* __restrict__ pu,
                                            CT* __restrict__ pp, CT* __restrict__ pd, const CT* __restrict__ twx) {
     using C = XCfg<NX, DRAG, CT, TV>;
     using RT = typename CTraits<CT>::R;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     CT* sm = reinterpret_cast<CT*>(sm_raw);
-    const int tid = threadIdx.x;
     const int npairs = g.ny / 2;
     const int nkx = g.nkx;
     const int slot = tid / C::G, lane = tid % C::G;
@@ -467,7 +465,7 @@ __device__ __forceinline__ CT unpack_pair(const CT* __restrict__ P, size_t i, in
 }
 
 template <int NY, bool DRAG, class CT, int TV = 0>
-__device__ __forceinline__ void yfwd_tile(const Geom g, int bx, int l, const LayerConst* __restrict__ lc,
+__device__ __forceinline__ void yfwd_tile(const Geom g, int tid, int bx, int l, const LayerConst* __restrict__ lc,
                                           const CT* __restrict__ q, const CT* __restrict__ psi,
                                           const CT* __restrict__ pp, const CT* __restrict__ pd,
                                           CT* __restrict__ out, const CT* __restrict__ twy,
@@ -476,7 +474,6 @@ __device__ __forceinline__ void yfwd_tile(const Geom g, int bx, int l, const Lay
     using RT = typename CTraits<CT>::R;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     CT* sm = reinterpret_cast<CT*>(sm_raw);
-    const int tid = threadIdx.x;
     const int kx0 = bx * C::TKX;
     const int slot = tid % C::SLOTS, lane = tid / C::SLOTS;
     const int fld = slot / C::TKX, c = slot % C::TKX;
