@@ -24,8 +24,8 @@
 //   k_cnn_fused           every layer of a small-batch inference, rows exchanged through L2
 #include "qgn_internal.cuh"
 #include "cnn.cuh"
+#include "tmap.cuh"
 
-#include <cuda.h>        // CUtensorMap (types only: the encoder is looked up at run time)
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -1626,24 +1626,11 @@ int conv_grid(const qgn_cnn* n, int batch) {
 }
 
 // The tensor map of `rows` image rows of W pixels x 64 channels (BF16, NHWC), copied 128 pixels at a
-// time into the 128-byte swizzle.  The encoder is a driver entry point, looked up once.
+// time into the 128-byte swizzle
 cudaError_t row_map(const __nv_bfloat16* p, int W, int rows, CUtensorMap* map) {
-    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static const Encode encode = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult r;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &r) != cudaSuccess) f = nullptr;
-        return reinterpret_cast<Encode>(f);
-    }();
-    if (!encode) return cudaErrorNotSupported;
     const cuuint64_t dims[3] = {64, (cuuint64_t)W, (cuuint64_t)rows}, strides[2] = {128, (cuuint64_t)W * 128};
-    const cuuint32_t box[3] = {64, kTileP, 1}, es[3] = {1, 1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16*>(p), dims, strides, box, es,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+    const cuuint32_t box[3] = {64, kTileP, 1};
+    return tensor_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, p, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 template <int CIN, int COUT, int EPI>

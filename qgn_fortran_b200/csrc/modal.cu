@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256, 3) k_modal_mma(Geom g, const ModalConst* 
     constexpr int KC = NP / 4, NT = NP / 8;
     using RI = decltype(TI::x);
     using RO = decltype(TO::x);
-    extern __shared__ __align__(16) unsigned char sm_raw[];
+    extern __shared__ __align__(128) unsigned char sm_raw[];
     double* fp = reinterpret_cast<double*>(sm_raw);   // [KC][NT][32] proj fragments
     double* fb = fp + KC * NT * 32;                   // [NT][2][NT][32] back fragments
     const int nz = g.nz;

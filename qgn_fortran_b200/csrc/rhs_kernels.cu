@@ -18,6 +18,7 @@
 #include "fft.cuh"
 #include "prof.cuh"
 #include "rhs_tiles.cuh"
+#include "tmap.cuh"
 
 #include <cuda_bf16.h>
 
@@ -60,15 +61,23 @@ __global__ void __launch_bounds__(XCfg<NX, DRAG, CT, TV>::THREADS,
     xpass_tile<NX, DRAG, CT, TV>(g, threadIdx.x, blockIdx.x, blockIdx.y, pq, pv, pu, pp, pd, twx);
 }
 
+// y-forward launches whose rows come by tensor-map copies: the default tiles of 256 points and more
+// (shorter columns are a fraction of a launch's latency, and their tiles' rows are whole lines)
+template <int NY, int TV>
+__host__ __device__ constexpr bool yfwd_mapped() { return TV == 0 && NY >= 256; }
+
 template <int NY, bool DRAG, class CT, int TV = 0>
 __global__ void __launch_bounds__(YFwdCfg<NY, DRAG, CT, TV>::THREADS,
                                   minb(YFwdCfg<NY, DRAG, CT, TV>::THREADS, YFwdCfg<NY, DRAG, CT, TV>::TP == 8 ? 64 : regcap<CT>()))
     k_yfwd(Geom g, const LayerConst* __restrict__ lc, const CT* __restrict__ q,
            const CT* __restrict__ psi, const CT* __restrict__ pp, const CT* __restrict__ pd,
-           CT* __restrict__ out, const CT* __restrict__ twy, const CT* __restrict__ extra) {
+           CT* __restrict__ out, const CT* __restrict__ twy, const CT* __restrict__ extra,
+           const __grid_constant__ YfwdMaps maps) {
     QGN_PDL_ENTRY();
     // with drag, the bottom layer's tiles transform twice: they go first
-    yfwd_tile<NY, DRAG, CT, TV>(g, threadIdx.x, blockIdx.x, DRAG ? g.nz - 1 - blockIdx.y : blockIdx.y, lc, q, psi, pp, pd, out, twy, extra);
+    yfwd_tile<NY, DRAG, CT, TV, yfwd_mapped<NY, TV>()>(g, threadIdx.x, blockIdx.x,
+                                                       DRAG ? g.nz - 1 - blockIdx.y : blockIdx.y, lc, q, psi, pp, pd, out,
+                                                       twy, extra, &maps);
 }
 
 template <int NX, int EPI, int TV = 0, class CT = double2>
@@ -103,7 +112,7 @@ __global__ void __launch_bounds__(X1Cfg<NX, TV>::THREADS, minb(X1Cfg<NX, TV>::TH
             const float* __restrict__ y = nullptr, int cout_p = 0, const float* __restrict__ osc = nullptr) {
     QGN_PDL_ENTRY();
     using C = X1Cfg<NX, TV>;
-    extern __shared__ __align__(16) unsigned char sm_raw[];
+    extern __shared__ __align__(128) unsigned char sm_raw[];
     double2* sm = reinterpret_cast<double2*>(sm_raw);
     const int tid = threadIdx.x;
     const int l = blockIdx.y;
@@ -138,7 +147,7 @@ __global__ void __launch_bounds__(YInvCfg<NY>::THREADS, minb(YInvCfg<NY>::THREAD
     k_yfwd1(Geom g, const double2* __restrict__ hq, double2* __restrict__ out, const double2* __restrict__ twy) {
     QGN_PDL_ENTRY();
     using C = YInvCfg<NY>;
-    extern __shared__ __align__(16) unsigned char sm_raw[];
+    extern __shared__ __align__(128) unsigned char sm_raw[];
     double2* sm = reinterpret_cast<double2*>(sm_raw);
     const int tid = threadIdx.x;
     const int l = blockIdx.y;
@@ -254,17 +263,37 @@ static cudaError_t launch_xpass(const Geom& g, const CT* hq, const CT* hp, const
     });
 }
 
+// the half-transformed rows [layers][ny][2][nkxp] as a tensor map: boxes of 2 TKX reals (TKX columns), both
+// parts and up to 256 rows
+template <class CT, int NY, int TKX>
+static cudaError_t yfwd_map(const Geom& g, const CT* P, int layers, CUtensorMap* map) {
+    const cuuint64_t row = (cuuint64_t)g.nkxp * sizeof(CT);
+    const cuuint64_t dims[4] = {2 * (cuuint64_t)g.nkxp, 2, NY, (cuuint64_t)layers};
+    const cuuint64_t strides[3] = {row, 2 * row, 2 * row * NY};
+    const cuuint32_t box[4] = {2 * TKX, 2, NY < 256 ? NY : 256, 1};
+    return tensor_map(map, sizeof(CT) == 16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, P, dims,
+                      strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
 template <int NY, bool DRAG, class CT, int TV>
 static cudaError_t yfwd_go(const Geom& g, const LayerConst* lc, const CT* q, const CT* psi, const CT* hpp, const CT* hpd,
                            CT* out, const CT* twy, const CT* extra, cudaStream_t s) {
     using C = YFwdCfg<NY, DRAG, CT, TV>;
+    constexpr bool MAP = yfwd_mapped<NY, TV>();
+    constexpr int SMEM = C::SMEM + (MAP ? 16 : 0);   // the copies' barrier
     cudaError_t e;
-    if ((e = set_smem(k_yfwd<NY, DRAG, CT, TV>, C::SMEM)) != cudaSuccess) return e;
+    if ((e = set_smem(k_yfwd<NY, DRAG, CT, TV>, SMEM)) != cudaSuccess) return e;
+    YfwdMaps maps{};
+    if (MAP && g.wait_err) {
+        if ((e = yfwd_map<CT, NY, C::TKX>(g, hpp, g.nz, &maps.p)) != cudaSuccess) return e;
+        if (DRAG && (e = yfwd_map<CT, NY, C::TKX>(g, hpd, 1, &maps.d)) != cudaSuccess) return e;
+        maps.use = 1;
+    }
     dim3 grid((g.nkx + C::TKX - 1) / C::TKX, g.nz);
     const double lb = (double)sizeof(CT) * g.nkx;
     QGN_LAUNCH(KID_YFWD, lb * (g.nz * (2.0 * NY + 3.0 * g.nky) + (DRAG ? 2.0 * NY : 0.0)), s,
-               ::qgn::launch(k_yfwd<NY, DRAG, CT, TV>, grid, C::THREADS, C::SMEM, s, g, lc, q, psi, hpp, hpd, out, twy,
-                                                                          extra));
+               ::qgn::launch(k_yfwd<NY, DRAG, CT, TV>, grid, C::THREADS, SMEM, s, g, lc, q, psi, hpp, hpd, out, twy, extra,
+                             maps));
     return cudaGetLastError();
 }
 

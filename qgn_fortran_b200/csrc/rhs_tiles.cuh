@@ -8,6 +8,7 @@
 #include "qgn_internal.cuh"
 #include "fft.cuh"
 
+#include <cuda.h>        // CUtensorMap (type only)
 #include <cuda_bf16.h>
 
 namespace qgn {
@@ -221,6 +222,14 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
         "l"(src), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
 }
+// one box of a tensor map, its corner at (x, 0, y, l)
+__device__ __forceinline__ void tensor_g2s(void* dst, const CUtensorMap* map, int x, int y, int l, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];\n" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(x), "r"(0), "r"(y), "r"(l), "r"(smem_u32(bar))
+        : "memory");
+}
 // bounded wait for phase `parity` of the barrier; false when it ran out
 __device__ __forceinline__ bool bar_wait_bounded(uint64_t* bar, uint32_t parity) {
     const uint32_t a = smem_u32(bar);
@@ -255,7 +264,7 @@ __device__ __forceinline__ void yinv_tile(const Geom g, int tid, int bx, int l, 
                                           int f_end = NF) {
     using C = YInvCfg<NY, CT, TV>;
     using RT = typename CTraits<CT>::R;
-    extern __shared__ __align__(16) unsigned char sm_raw[];
+    extern __shared__ __align__(128) unsigned char sm_raw[];
     CT* sm = reinterpret_cast<CT*>(sm_raw);
     const int kx0 = bx * C::TKX;
     const int slot = tid % C::TKX, lane = tid / C::TKX;
@@ -367,7 +376,7 @@ __device__ __forceinline__ void xpass_tile(const Geom g, int tid, int bx, int la
                                            CT* __restrict__ pp, CT* __restrict__ pd, const CT* __restrict__ twx) {
     using C = XCfg<NX, DRAG, CT, TV>;
     using RT = typename CTraits<CT>::R;
-    extern __shared__ __align__(16) unsigned char sm_raw[];
+    extern __shared__ __align__(128) unsigned char sm_raw[];
     CT* sm = reinterpret_cast<CT*>(sm_raw);
     const int npairs = g.ny / 2;
     const int nkx = g.nkx;
@@ -437,9 +446,71 @@ __device__ __forceinline__ void xpass_tile(const Geom g, int tid, int bx, int la
 
 // ------------------------------------------------------------------------------------
 // yfwd: forward y transforms of uq, vq columns and assembly of the right-hand side.
-// Slots are lane-interleaved: slot = tid % (2 TKX), slot = field*TKX + column.  The first
-// radix pass reads the half-transformed rows straight from HBM.
+// Slots are lane-interleaved: slot = tid % (2 TKX), slot = field*TKX + column.
+//
+// With a tensor map of the half-transformed rows (MAP) the tile -- TKX columns of both parts of every
+// row, 2 TKX values per row -- is first copied into the slots' shared memory as [row][part][column] by
+// the copy engine, and the first radix pass reads it there.  Plain loads of the rows take 16 or 32 bytes
+// from each of 16 lines per warp (two columns), so the pass was bound by the L1's line rate: 38 % of
+// its L1 wavefronts were these loads.  The staged form needs a fourth of them, and reads both parts
+// instead of exchanging them by shuffles.  When the copies have landed, the columns of q and psi that
+// the assembly will read are requested into L2, behind the transforms.  1024^2 x 8 FP64 66.1 -> 62.8 us
+// staged -> 58.9 us with the request (63.9 us when it goes out before the copies), FP32 43.5 -> 39.7 ->
+// 36.6 us, 2048^2 x 16 FP32 281 -> 255 -> 225 us, 512^2 x 32 FP64 55.8 -> 49.8 -> 45.9 us (B200).
+// Without one (ensembles, small tiles) the first radix pass reads the rows straight from HBM.
 // ------------------------------------------------------------------------------------
+struct YfwdMaps {       // of hpp and, with drag, of hpd; use = 0: none (plain staging loads)
+    CUtensorMap p, d;
+    int use;
+};
+
+// The tile's columns of one compact field, requested into L2 (n elements from `first`, widened to
+// 16-byte boundaries; a compact field's buffer holds 16 bytes per element in either precision)
+template <class CT>
+__device__ __forceinline__ void prefetch_columns(const CT* first, int n) {
+    const unsigned long long a = reinterpret_cast<unsigned long long>(first);
+    const unsigned long long lo = a & ~15ull, hi = (a + (unsigned long long)n * sizeof(CT) + 15ull) & ~15ull;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(lo), "r"((uint32_t)(hi - lo)) : "memory");
+}
+
+template <class CT>
+__device__ __forceinline__ CT split_p(CT X, CT P1, int kx, int fld) {
+    using RT = typename CTraits<CT>::R;
+    const CT Y = kx == 0 ? cconj(X) : cconj(P1);
+    return fld == 0 ? cmk<CT>((RT)0.5 * (X.x + Y.x), (RT)0.5 * (X.y + Y.y))
+                    : cmk<CT>((RT)0.5 * (X.y - Y.y), -(RT)0.5 * (X.x - Y.x));
+}
+
+// the tile's columns of every row of layer l into sm as [NY][2][TKX]; bar: a barrier past the slots,
+// fresh for each call (initialised and invalidated here)
+template <int NY, int TKX, class CT>
+__device__ __forceinline__ void stage_rows(const Geom& g, int tid, int threads, int kx0, int l, const CUtensorMap* map,
+                                           bool use, const CT* __restrict__ P, size_t len, CT* sm, uint64_t* bar) {
+    if (use) {
+        constexpr int ROWS = NY < 256 ? NY : 256;   // rows per box
+        // the slots' earlier accesses are ordered before the copies' writes
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        if (tid == 0) bar_init(bar);
+        __syncthreads();
+        if (tid == 0) {
+            bar_expect_tx(bar, (uint32_t)(NY * 2 * TKX * (int)sizeof(CT)));
+            for (int y = 0; y < NY; y += ROWS) tensor_g2s(sm + (size_t)y * 2 * TKX, map, 2 * kx0, y, l, bar);
+        }
+        if (!bar_wait_bounded(bar, 0)) {
+            atomicExch(g.wait_err, 1);            // the controller halts the run on it
+            bar_wait_bounded(bar, 0);             // once more for the copies still in flight
+        }
+    } else {
+        for (int e = tid; e < NY * 2 * TKX; e += threads) {
+            const int c = e % TKX, part = (e / TKX) % 2, y = e / (2 * TKX);
+            const size_t i = p_index(g, l, y, part, kx0 + c);
+            const bool ok = kx0 + c < g.nkx && in_bounds(g, i, len);
+            sm[e] = ok ? P[i] : cmk<CT>(0.0, 0.0);
+        }
+        __syncthreads();
+    }
+}
+
 // split of the packed forward x transform of row y at kx: fld 0 -> (uq)^, fld 1 -> (vq)^
 __device__ __forceinline__ double2 unpack_p(const double2* __restrict__ P, const Geom& g, int l, int y, int kx,
                                             int fld) {
@@ -464,15 +535,15 @@ __device__ __forceinline__ CT unpack_pair(const CT* __restrict__ P, size_t i, in
                     : cmk<CT>((typename CTraits<CT>::R)0.5 * (X.y - Y.y), -(typename CTraits<CT>::R)0.5 * (X.x - Y.x));
 }
 
-template <int NY, bool DRAG, class CT, int TV = 0>
+template <int NY, bool DRAG, class CT, int TV = 0, bool MAP = false>
 __device__ __forceinline__ void yfwd_tile(const Geom g, int tid, int bx, int l, const LayerConst* __restrict__ lc,
                                           const CT* __restrict__ q, const CT* __restrict__ psi,
                                           const CT* __restrict__ pp, const CT* __restrict__ pd,
                                           CT* __restrict__ out, const CT* __restrict__ twy,
-                                          const CT* __restrict__ extra = nullptr) {
+                                          const CT* __restrict__ extra = nullptr, const YfwdMaps* maps = nullptr) {
     using C = YFwdCfg<NY, DRAG, CT, TV>;
     using RT = typename CTraits<CT>::R;
-    extern __shared__ __align__(16) unsigned char sm_raw[];
+    extern __shared__ __align__(128) unsigned char sm_raw[];
     CT* sm = reinterpret_cast<CT*>(sm_raw);
     const int kx0 = bx * C::TKX;
     const int slot = tid % C::SLOTS, lane = tid / C::SLOTS;
@@ -486,6 +557,12 @@ __device__ __forceinline__ void yfwd_tile(const Geom g, int tid, int bx, int l, 
     // loops below read 8-16 consecutive rows per wavefront, which a pad element every TP rows
     // would split across one bank group twice
     auto omap = [](int y) { return y; };
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm_raw + C::SMEM);   // (MAP)
+    auto ld_staged = [&](int y) -> CT {
+        const CT X = sm[(2 * y) * C::TKX + c], P1 = sm[(2 * y + 1) * C::TKX + c];
+        const CT v = split_p(X, P1, kx0 + c, fld);
+        return colok ? v : cmk<CT>(0.0, 0.0);
+    };
 
     if (DRAG && bottom) {
         // drag_hat = i ky (|u|u)^ - i kx (|u|v)^ on the bottom layer (QGN_Module.f90:284-292)
@@ -494,7 +571,13 @@ __device__ __forceinline__ void yfwd_tile(const Geom g, int tid, int bx, int l, 
             const bool ok = colok && in_bounds(g, i, (size_t)g.ny * 2 * g.nkxp);
             return unpack_pair(pd, i, kx0 + c, fld, ok, C::TKX);
         };
-        fft_fused<NY, -1, SRC_FN, DST_SMEM_MAP, C::TP, false, C::SLOTS>(xs, lane, true, twy, ldd, omap);
+        if constexpr (MAP) {
+            stage_rows<NY, C::TKX>(g, tid, C::THREADS, kx0, 0, &maps->d, maps->use, pd, (size_t)g.ny * 2 * g.nkxp, sm, bar);
+            fft_fused<NY, -1, SRC_FN_SMEM, DST_SMEM_MAP, C::TP, false, C::SLOTS>(xs, lane, true, twy, ld_staged, omap);
+            if (maps->use && tid == 0) bar_inval(bar);   // every waiter has passed the barrier
+        } else {
+            fft_fused<NY, -1, SRC_FN, DST_SMEM_MAP, C::TP, false, C::SLOTS>(xs, lane, true, twy, ldd, omap);
+        }
         const RT dc = (RT)lc->dragc;
         for (int e = tid; e < C::TKX * nky; e += C::THREADS) {
             const int cc = e / nky, m = e % nky;
@@ -517,7 +600,15 @@ __device__ __forceinline__ void yfwd_tile(const Geom g, int tid, int bx, int l, 
         const bool ok = colok && in_bounds(g, i, 2 * g.hsize());
         return unpack_pair(pp, i, kx0 + c, fld, ok, C::TKX);
     };
-    fft_fused<NY, -1, SRC_FN, DST_SMEM_MAP, C::TP, false, C::SLOTS>(xs, lane, true, twy, ld, omap);
+    if constexpr (MAP) {
+        stage_rows<NY, C::TKX>(g, tid, C::THREADS, kx0, l, &maps->p, maps->use, pp, 2 * g.hsize(), sm, bar);
+        const int ncol = cmin(C::TKX, g.nkx - kx0);
+        if (tid >= 32 && tid < 34) prefetch_columns((tid == 32 ? q : psi) + (colbase + kx0) * nky, ncol * nky);
+        fft_fused<NY, -1, SRC_FN_SMEM, DST_SMEM_MAP, C::TP, false, C::SLOTS>(xs, lane, true, twy, ld_staged, omap);
+        if (maps->use && tid == 0) bar_inval(bar);
+    } else {
+        fft_fused<NY, -1, SRC_FN, DST_SMEM_MAP, C::TP, false, C::SLOTS>(xs, lane, true, twy, ld, omap);
+    }
 
     const RT ub = (RT)lc->uBar[l], bq = (RT)lc->betaq[l];
     const RT ek = (RT)lc->ekman;
@@ -589,7 +680,7 @@ __device__ __forceinline__ void xinv1_tile(const Geom g, int bx, int l, const CT
                                            int chan = 0) {
     static_assert(EPI == 0 || sizeof(CT) == 16, "FP32 rows: max only");
     using C = X1Cfg<NX, TV, CT>;
-    extern __shared__ __align__(16) unsigned char sm_raw[];
+    extern __shared__ __align__(128) unsigned char sm_raw[];
     CT* sm = reinterpret_cast<CT*>(sm_raw);
     __shared__ double smax[32];
     const int tid = threadIdx.x;

@@ -798,7 +798,7 @@ __global__ void __launch_bounds__(StageYinvCfg<NY, NZ>::THREADS)
                  const DevScalars* __restrict__ sc, double2* __restrict__ pq, double2* __restrict__ pv,
                  double2* __restrict__ pu, const double2* __restrict__ twy) {
     QGN_PDL_ENTRY();
-    extern __shared__ __align__(16) unsigned char sm_raw[];
+    extern __shared__ __align__(128) unsigned char sm_raw[];
     stage_yinv_col<S, NZ, NY>(g, blockIdx.x, cp, q, qout, psi, lc, ma, sc, pq, pv, pu, twy, sm_raw);
 }
 
@@ -816,7 +816,7 @@ __global__ void __launch_bounds__(StageYinvCfg<NY, NZ>::THREADS)
                       double2* __restrict__ pu, const double2* __restrict__ twy) {
     QGN_PDL_ENTRY();
     using C = StageYinvCfg<NY, NZ>;
-    extern __shared__ __align__(16) unsigned char sm_raw[];
+    extern __shared__ __align__(128) unsigned char sm_raw[];
     double2* slots = reinterpret_cast<double2*>(sm_raw);
     const int tid = threadIdx.x;
     const int kx = blockIdx.x;
