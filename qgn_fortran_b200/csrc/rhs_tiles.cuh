@@ -222,6 +222,15 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
         "l"(src), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
 }
+// n elements from `first` requested into L2, widened to 16-byte boundaries (the fields' buffers hold 16
+// bytes per element in either precision)
+template <class CT>
+__device__ __forceinline__ void prefetch_l2(const CT* first, int n) {
+    const unsigned long long a = reinterpret_cast<unsigned long long>(first);
+    const unsigned long long lo = a & ~15ull, hi = (a + (unsigned long long)n * sizeof(CT) + 15ull) & ~15ull;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(lo), "r"((uint32_t)(hi - lo)) : "memory");
+}
+
 // one box of a tensor map, its corner at (x, 0, y, l)
 __device__ __forceinline__ void tensor_g2s(void* dst, const CUtensorMap* map, int x, int y, int l, uint64_t* bar) {
     asm volatile(
@@ -464,15 +473,6 @@ struct YfwdMaps {       // of hpp and, with drag, of hpd; use = 0: none (plain s
     int use;
 };
 
-// The tile's columns of one compact field, requested into L2 (n elements from `first`, widened to
-// 16-byte boundaries; a compact field's buffer holds 16 bytes per element in either precision)
-template <class CT>
-__device__ __forceinline__ void prefetch_columns(const CT* first, int n) {
-    const unsigned long long a = reinterpret_cast<unsigned long long>(first);
-    const unsigned long long lo = a & ~15ull, hi = (a + (unsigned long long)n * sizeof(CT) + 15ull) & ~15ull;
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(lo), "r"((uint32_t)(hi - lo)) : "memory");
-}
-
 template <class CT>
 __device__ __forceinline__ CT split_p(CT X, CT P1, int kx, int fld) {
     using RT = typename CTraits<CT>::R;
@@ -603,7 +603,7 @@ __device__ __forceinline__ void yfwd_tile(const Geom g, int tid, int bx, int l, 
     if constexpr (MAP) {
         stage_rows<NY, C::TKX>(g, tid, C::THREADS, kx0, l, &maps->p, maps->use, pp, 2 * g.hsize(), sm, bar);
         const int ncol = cmin(C::TKX, g.nkx - kx0);
-        if (tid >= 32 && tid < 34) prefetch_columns((tid == 32 ? q : psi) + (colbase + kx0) * nky, ncol * nky);
+        if (tid >= 32 && tid < 34) prefetch_l2((tid == 32 ? q : psi) + (colbase + kx0) * nky, ncol * nky);
         fft_fused<NY, -1, SRC_FN_SMEM, DST_SMEM_MAP, C::TP, false, C::SLOTS>(xs, lane, true, twy, ld_staged, omap);
         if (maps->use && tid == 0) bar_inval(bar);
     } else {
