@@ -45,12 +45,14 @@ __host__ __device__ constexpr int regcap(int fp64 = 128, int fp32 = 64) { return
 // the single-field launches; a non-zero value is the CTA size in threads (per slot group for
 // the x pass), the same for every transform length, which lets one launch cover fields of
 // different sizes (ensembles).
-// elements per thread of an x transform (fft.cuh): 32 for the 512- and 1024-point transforms of
-// the single-field x pass (two radix passes instead of three, each transform in one warp: the
-// FP32 x pass ran 9 % faster, the FP64 one cut the 1024^2 x 8 step by 2 % despite 168
-// registers), 16 otherwise.  The y passes keep 16 in FP32: their CTAs interleave columns
-// across warps, and at 32 elements they had half the threads per column and ran 1.3-1.7x
-// slower on B200.
+// elements per thread of an x transform (fft.cuh): 32 for the 512-point and longer transforms of
+// the single-field x pass (two radix passes instead of three, each transform of up to 1024 points in
+// one warp: the FP32 x pass ran 9 % faster, the FP64 one cut the 1024^2 x 8 step by 2 % despite 168
+// registers), 16 otherwise.  2048 points take two warps and a third, radix-2 pass, which is fused with
+// the second by shuffles (fft_pass_tail2, interleave 1): the 2048^2 x 16 x pass took 1061 us in FP64 and 511 us in
+// FP32 with 16 elements and block barriers between all passes, 839 and 470 us this way.  The y passes
+// keep 16 in FP32: their CTAs interleave columns across warps, and at 32 elements they had half the
+// threads per column and ran 1.3-1.7x slower on B200.
 // A non-zero tile-variant code carries the CTA width in its low 16 bits and, above them, the
 // elements per thread of its transforms (8, 16 or 32; 0 there means 16): the ensemble's
 // autotuner searches both.
@@ -59,19 +61,25 @@ __host__ __device__ constexpr int tv_radix(int tv) { return tv >> 16; }
 __host__ __device__ constexpr int tv_make(int width, int radix) { return width | (radix << 16); }
 template <class CT, int N, int TV>
 __host__ __device__ constexpr int fft_tp() {
-    return TV == 0 ? ((N == 512 || N == 1024) ? 32 : 16) : (tv_radix(TV) ? tv_radix(TV) : 16);
+    return TV == 0 ? ((N >= 512) ? 32 : 16) : (tv_radix(TV) ? tv_radix(TV) : 16);
 }
 // elements per thread of a y transform: 8 for the FP64 512- and 1024-point columns of the
 // single-field launches, 16 otherwise.  Half the registers per thread (64, two 512-thread CTAs
 // per SM) doubles the resident warps of these latency-bound kernels at the price of a fourth
 // radix pass at 1024 points: on B200 the 512^2 step ran 11 % and the 1024^2 step 1 % faster.
+// Columns per CTA (TKX) in FP64: at 2048 points a tile of the usual width is a 1024-thread CTA, alone on
+// its SM; two columns of 16 elements per thread (y-inverse) and one (y-forward, whose rows come by
+// tensor-map copies, so narrow pieces cost no L1 wavefronts) are 603 -> 477 us and 516 -> 411 us for
+// 2048^2 x 16.  One column also suits the 1024-point y-forward (59.2 -> 55.5 us for 1024^2 x 8) but not
+// the 512-point one (45.7 -> 48.8 us for 512^2 x 32); two in the y-inverse of 1024 points are slower
+// (62.7 -> 68.4 us: its row stores fall to 32-byte pieces), as in the FP32 one of 2048 (274 -> 319 us).
 // QGN_Y_TP64 (build-time tuning knob, default 8) overrides the FP64 value.
 #ifndef QGN_Y_TP64
 #define QGN_Y_TP64 8
 #endif
 template <class CT, int N, int TV>
 __host__ __device__ constexpr int fft_tp_y() {
-    return TV == 0 ? ((sizeof(CT) == 16 && N >= 512) ? QGN_Y_TP64 : 16) : (tv_radix(TV) ? tv_radix(TV) : 16);
+    return TV == 0 ? ((sizeof(CT) == 16 && N >= 512 && N < 2048) ? QGN_Y_TP64 : 16) : (tv_radix(TV) ? tv_radix(TV) : 16);
 }
 // Row pairs per CTA of the single-field x pass with one warp per transform (a build-time tuning
 // knob).  One row pair (three warps, 96 threads, four CTAs per SM at 168 registers) couples only
@@ -85,7 +93,7 @@ template <int NY, class CT = double2, int TV = 0>
 struct YInvCfg {
     static constexpr int TP = fft_tp_y<CT, NY, TV>();
     static constexpr int G = FFTShape<NY, TP>::G;
-    static constexpr int TKX = TV == 0 ? cmin(cmax(4, 128 / G), 16) : cmax(1, tv_width(TV) / G);
+    static constexpr int TKX = TV == 0 ? (NY >= 2048 && sizeof(CT) == 16 ? 2 : cmin(cmax(4, 128 / G), 16)) : cmax(1, tv_width(TV) / G);
     static constexpr int THREADS = TKX * G;
     static constexpr int TS = slot_stride(NY, interleave_target(TKX, (int)sizeof(CT)), (int)sizeof(CT), TP);
     static constexpr int SMEM = TKX * TS * (int)sizeof(CT);
@@ -113,7 +121,7 @@ struct YFwdCfg {
     static constexpr int TP = fft_tp_y<CT, NY, TV>();
     static constexpr int G = FFTShape<NY, TP>::G;
     // tid ^ TKX stays in the warp
-    static constexpr int TKX = TV == 0 ? cmin(cmax(2, 64 / G), 16) : cmin(cmax(1, tv_width(TV) / (2 * G)), 16);
+    static constexpr int TKX = TV == 0 ? (NY >= 1024 && sizeof(CT) == 16 ? 1 : cmin(cmax(2, 64 / G), 16)) : cmin(cmax(1, tv_width(TV) / (2 * G)), 16);
     static constexpr int SLOTS = 2 * TKX;
     static constexpr int THREADS = SLOTS * G;
     static constexpr int TS = slot_stride(NY, interleave_target(SLOTS, (int)sizeof(CT)), (int)sizeof(CT), TP);
@@ -414,7 +422,7 @@ __device__ __forceinline__ void xpass_tile(const Geom g, int tid, int bx, int la
         plane[x] = v.x;
         plane[C::TS + x] = v.y;
     };
-    fft_fused<NX, +1, SRC_FN, DST_SMEM_STORE, C::TP, (C::G <= 32)>(xs, lane, pair_ok && !(drag && s_of == 0), twx,
+    fft_fused<NX, +1, SRC_FN, DST_SMEM_STORE, C::TP, (C::G <= 32), (C::G > 32 && TV == 0 ? 1 : 0)>(xs, lane, pair_ok && !(drag && s_of == 0), twx,
                                                                      ld_inv, st_inv);
 
     // ---- forward: slot 0 = u1 q1 + i v1 q1, 1 = u2 q2 + i v2 q2 (grid/(nx*ny) scaling as in
@@ -450,7 +458,7 @@ __device__ __forceinline__ void xpass_tile(const Geom g, int tid, int bx, int la
             if (in_bounds(g, i, olen)) out[i] = v;
         }
     };
-    fft_fused<NX, -1, SRC_FN_SMEM, DST_FN, C::TP, (C::G <= 32)>(xs, lane, pair_ok && s_of < 2, twx, ld_fwd, st_fwd);
+    fft_fused<NX, -1, SRC_FN_SMEM, DST_FN, C::TP, (C::G <= 32), (C::G > 32 && TV == 0 ? 1 : 0)>(xs, lane, pair_ok && s_of < 2, twx, ld_fwd, st_fwd);
 }
 
 // ------------------------------------------------------------------------------------
