@@ -214,9 +214,9 @@ int ark_attempt(qgn_ctx* ctx, bool leith, const cudaGraphConditionalHandle* loop
         const double2* extra = closure_tendency(ctx);
         CK(launch_ark_stage_yinv(g, b, 1, st));
         for (int s = 1; s < 6; ++s) {
-            CK(launch_rhs_x(g, b, false, st));
+            CK(launch_rhs_x_columns(g, b, st));
             if (s < 5) CK(launch_yfwd_stage_yinv(g, b, s + 1, extra, st));
-            else CK(launch_rhs_yfwd(g, b, b.Qs[5], b.psi, b.N[5], false, st, extra));
+            else CK(launch_rhs_yfwd_columns(g, b, b.Qs[5], b.psi, b.N[5], st, extra));
         }
     } else for (int s = 1; s < 6; ++s) {
         QGN_NVTX(kStageRange[s]);
@@ -262,9 +262,9 @@ int ark_prologue(qgn_ctx* ctx, bool leith) {
         if (ctx->closure && !drag_on(ctx)) {
             RET(closure_fork(ctx));
             CK(launch_ark_stage_yinv(g, b, 0, st));
-            CK(launch_rhs_x(g, b, false, st));
+            CK(launch_rhs_x_columns(g, b, st));
             RET(closure_join(ctx));
-            CK(launch_rhs_yfwd(g, b, b.q, b.psi, b.N[0], false, st, closure_tendency(ctx)));
+            CK(launch_rhs_yfwd_columns(g, b, b.q, b.psi, b.N[0], st, closure_tendency(ctx)));
             return QGN_OK;
         }
         if (ctx->closure) {
@@ -272,7 +272,12 @@ int ark_prologue(qgn_ctx* ctx, bool leith) {
             RET(closure_eval(ctx, b.psi, st));
         }
         CK(launch_ark_stage_yinv(g, b, 0, st));
-        CK(launch_rhs_tail(g, b, b.q, b.psi, b.N[0], drag_on(ctx), st, closure_tendency(ctx)));
+        if (drag_on(ctx)) {
+            CK(launch_rhs_tail(g, b, b.q, b.psi, b.N[0], true, st, closure_tendency(ctx)));
+        } else {
+            CK(launch_rhs_x_columns(g, b, st));
+            CK(launch_rhs_yfwd_columns(g, b, b.q, b.psi, b.N[0], st, closure_tendency(ctx)));
+        }
     } else {
         CK(launch_modal(g, b, b.q, b.psi, st));
         // the learned closure (if attached): S of this step's state and the budget check that

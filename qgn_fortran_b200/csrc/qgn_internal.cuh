@@ -215,6 +215,10 @@ cudaError_t launch_rhs_tail(const Geom& g, const Buffers& b, const double2* q, c
 cudaError_t launch_rhs_x(const Geom& g, const Buffers& b, bool do_drag, cudaStream_t s);
 cudaError_t launch_rhs_yfwd(const Geom& g, const Buffers& b, const double2* q, const double2* psi, double2* out,
                             bool do_drag, cudaStream_t s, const double2* extra = nullptr);
+// the same passes of the small grids' column path (ny 128, 256 or 512)
+cudaError_t launch_rhs_x_columns(const Geom& g, const Buffers& b, cudaStream_t s);
+cudaError_t launch_rhs_yfwd_columns(const Geom& g, const Buffers& b, const double2* q, const double2* psi, double2* out,
+                                    cudaStream_t s, const double2* extra);
 cudaError_t launch_rhs32(const Geom& g, const Buffers& b, const float2* q, const float2* psi, float2* out, bool do_drag,
                          cudaStream_t s);
 // y-inverse + x-pass of one compact field with a max|.| reduction into sc->maxbits

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(YInvCfg<NY, CT, TV>::THREADS, minb(YInvCfg<NY,
         yinv_tile<NY, NF, CT, TV>(g, threadIdx.x, blockIdx.x, blockIdx.y, q, psi, pq, pv, pu, twy);
 }
 
-template <int NX, bool DRAG, class CT, int TV = 0>
+template <int NX, bool DRAG, class CT, int TV = 0, bool PT = false>
 __global__ void __launch_bounds__(XCfg<NX, DRAG, CT, TV>::THREADS,
                                   minb(XCfg<NX, DRAG, CT, TV>::THREADS,
                                        XCfg<NX, DRAG, CT, TV>::TP == 32 ? (sizeof(CT) == 16 ? 168 : 112) : regcap<CT>(NX >= 1024 ? 112 : 128, 80)))
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(XCfg<NX, DRAG, CT, TV>::THREADS,
             const CT* __restrict__ pu, CT* __restrict__ pp, CT* __restrict__ pd,
             const CT* __restrict__ twx) {
     QGN_PDL_ENTRY();
-    if constexpr (TV == 0 && NX >= 512 && sizeof(CT) == 16) {
+    if constexpr (TV == 0 && NX >= 512 && sizeof(CT) == 16 && !PT) {
         constexpr int RP = XCfg<NX, DRAG, CT, TV>::RP;
         const int t = blockIdx.y * gridDim.x + blockIdx.x + kAhead;
         const int bx = t % gridDim.x, l = t / gridDim.x;
@@ -81,15 +81,15 @@ __global__ void __launch_bounds__(XCfg<NX, DRAG, CT, TV>::THREADS,
                             ((size_t)l * (g.ny / 2) + bx * RP) * 2 * g.nkxp,
                         cmin(RP, g.ny / 2 - bx * RP) * 2 * g.nkxp);
     }
-    xpass_tile<NX, DRAG, CT, TV>(g, threadIdx.x, blockIdx.x, blockIdx.y, pq, pv, pu, pp, pd, twx);
+    xpass_tile<NX, DRAG, CT, TV, PT>(g, threadIdx.x, blockIdx.x, blockIdx.y, pq, pv, pu, pp, pd, twx);
 }
 
 // y-forward launches whose rows come by tensor-map copies: the default tiles of 256 points and more
 // (shorter columns are a fraction of a launch's latency, and their tiles' rows are whole lines)
-template <int NY, int TV>
-__host__ __device__ constexpr bool yfwd_mapped() { return TV == 0 && NY >= 256; }
+template <int NY, int TV, bool PT = false>
+__host__ __device__ constexpr bool yfwd_mapped() { return TV == 0 && NY >= 256 && !PT; }
 
-template <int NY, bool DRAG, class CT, int TV = 0>
+template <int NY, bool DRAG, class CT, int TV = 0, bool PT = false>
 __global__ void __launch_bounds__(YFwdCfg<NY, DRAG, CT, TV>::THREADS,
                                   minb(YFwdCfg<NY, DRAG, CT, TV>::THREADS, YFwdCfg<NY, DRAG, CT, TV>::TP == 8 ? 64 : regcap<CT>()))
     k_yfwd(Geom g, const LayerConst* __restrict__ lc, const CT* __restrict__ q,
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(YFwdCfg<NY, DRAG, CT, TV>::THREADS,
            const __grid_constant__ YfwdMaps maps) {
     QGN_PDL_ENTRY();
     // with drag, the bottom layer's tiles transform twice: they go first
-    yfwd_tile<NY, DRAG, CT, TV, yfwd_mapped<NY, TV>()>(g, threadIdx.x, blockIdx.x,
+    yfwd_tile<NY, DRAG, CT, TV, yfwd_mapped<NY, TV, PT>(), PT>(g, threadIdx.x, blockIdx.x,
                                                        DRAG ? g.nz - 1 - blockIdx.y : blockIdx.y, lc, q, psi, pp, pd, out,
                                                        twy, extra, &maps);
 }
@@ -254,16 +254,16 @@ static cudaError_t launch_yinv(const Geom& g, int nf, const CT* q, const CT* psi
     });
 }
 
-template <int NX, bool DRAG, class CT, int TV>
+template <int NX, bool DRAG, class CT, int TV, bool PT = false>
 static cudaError_t xpass_go(const Geom& g, const CT* hq, const CT* hp, const CT* hu, CT* hpp, CT* hpd, const CT* twx,
                             cudaStream_t s) {
     using C = XCfg<NX, DRAG, CT, TV>;
     cudaError_t e;
-    if ((e = set_smem(k_xpass<NX, DRAG, CT, TV>, C::SMEM)) != cudaSuccess) return e;
+    if ((e = set_smem(k_xpass<NX, DRAG, CT, TV, PT>, C::SMEM)) != cudaSuccess) return e;
     dim3 grid((g.ny / 2 + C::RP - 1) / C::RP, g.nz + (DRAG ? 1 : 0));
     const double es = (double)sizeof(CT);
     QGN_LAUNCH(KID_XPASS, (5.0 * g.nz + (DRAG ? 4.0 : 0.0)) * es * (double)g.ny * g.nkx, s,
-               ::qgn::launch(k_xpass<NX, DRAG, CT, TV>, grid, C::THREADS, C::SMEM, s, g, hq, hp, hu, hpp, hpd, twx));
+               ::qgn::launch(k_xpass<NX, DRAG, CT, TV, PT>, grid, C::THREADS, C::SMEM, s, g, hq, hp, hu, hpp, hpd, twx));
     return cudaGetLastError();
 }
 
@@ -298,14 +298,14 @@ static cudaError_t yfwd_map(const Geom& g, const CT* P, int layers, CUtensorMap*
                       strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
-template <int NY, bool DRAG, class CT, int TV>
+template <int NY, bool DRAG, class CT, int TV, bool PT = false>
 static cudaError_t yfwd_go(const Geom& g, const LayerConst* lc, const CT* q, const CT* psi, const CT* hpp, const CT* hpd,
                            CT* out, const CT* twy, const CT* extra, cudaStream_t s) {
     using C = YFwdCfg<NY, DRAG, CT, TV>;
-    constexpr bool MAP = yfwd_mapped<NY, TV>();
+    constexpr bool MAP = yfwd_mapped<NY, TV, PT>();
     constexpr int SMEM = C::SMEM + (MAP ? 16 : 0);   // the copies' barrier
     cudaError_t e;
-    if ((e = set_smem(k_yfwd<NY, DRAG, CT, TV>, SMEM)) != cudaSuccess) return e;
+    if ((e = set_smem(k_yfwd<NY, DRAG, CT, TV, PT>, SMEM)) != cudaSuccess) return e;
     YfwdMaps maps{};
     if (MAP && g.wait_err) {
         if ((e = yfwd_map<CT, NY, C::TKX>(g, hpp, g.nz, &maps.p)) != cudaSuccess) return e;
@@ -315,7 +315,7 @@ static cudaError_t yfwd_go(const Geom& g, const LayerConst* lc, const CT* q, con
     dim3 grid((g.nkx + C::TKX - 1) / C::TKX, g.nz);
     const double lb = (double)sizeof(CT) * g.nkx;
     QGN_LAUNCH(KID_YFWD, lb * (g.nz * (2.0 * NY + 3.0 * g.nky) + (DRAG ? 2.0 * NY : 0.0)), s,
-               ::qgn::launch(k_yfwd<NY, DRAG, CT, TV>, grid, C::THREADS, SMEM, s, g, lc, q, psi, hpp, hpd, out, twy, extra,
+               ::qgn::launch(k_yfwd<NY, DRAG, CT, TV, PT>, grid, C::THREADS, SMEM, s, g, lc, q, psi, hpp, hpd, out, twy, extra,
                              maps));
     return cudaGetLastError();
 }
@@ -336,6 +336,40 @@ static cudaError_t launch_yfwd(const Geom& g, const LayerConst* lc, const CT* q,
         }
         return drag ? yfwd_go<NY, true, CT, 0>(g, lc, q, psi, hpp, hpd, out, twy, extra, s)
                     : yfwd_go<NY, false, CT, 0>(g, lc, q, psi, hpp, hpd, out, twy, extra, s);
+    });
+}
+
+// the x pass and the y-forward pass of the small grids' column path (FP64, no drag), the forward x
+// transforms column by column (p_index<true>)
+cudaError_t launch_rhs_x_columns(const Geom& g, const Buffers& b, cudaStream_t s) {
+    return dispatch_n(g.nx, [&](auto NXc) -> cudaError_t {
+        constexpr int NX = decltype(NXc)::value;
+        if constexpr (has_narrow<NX>()) {
+            using D = XCfg<NX, false, double2>;
+            using Nn = XCfg<NX, false, double2, kNarrowX>;
+            if (narrow_better((long long)((g.ny / 2 + D::RP - 1) / D::RP) * g.nz,
+                              (long long)((g.ny / 2 + Nn::RP - 1) / Nn::RP) * g.nz))
+                return xpass_go<NX, false, double2, kNarrowX, true>(g, b.hq, b.hp, b.hu, b.hpp, nullptr, b.twx, s);
+        }
+        return xpass_go<NX, false, double2, 0, true>(g, b.hq, b.hp, b.hu, b.hpp, nullptr, b.twx, s);
+    });
+}
+
+cudaError_t launch_rhs_yfwd_columns(const Geom& g, const Buffers& b, const double2* q, const double2* psi, double2* out,
+                                    cudaStream_t s, const double2* extra) {
+    return dispatch_n(g.ny, [&](auto NYc) -> cudaError_t {
+        constexpr int NY = decltype(NYc)::value;
+        if constexpr (NY == 128 || NY == 256 || NY == 512) {
+            if constexpr (has_narrow<NY>()) {
+                using D = YFwdCfg<NY, false, double2>;
+                using Nn = YFwdCfg<NY, false, double2, kNarrowY>;
+                if (narrow_better((long long)((g.nkx + D::TKX - 1) / D::TKX) * g.nz,
+                                  (long long)((g.nkx + Nn::TKX - 1) / Nn::TKX) * g.nz))
+                    return yfwd_go<NY, false, double2, kNarrowY, true>(g, b.lc, q, psi, b.hpp, nullptr, out, b.twy, extra, s);
+            }
+            return yfwd_go<NY, false, double2, 0, true>(g, b.lc, q, psi, b.hpp, nullptr, out, b.twy, extra, s);
+        }
+        return cudaErrorInvalidValue;
     });
 }
 

@@ -193,7 +193,11 @@ __device__ __forceinline__ CT pack_hi(CT f1, CT f2) {
 
 // Layout of the forward x transforms P[k] (part 0) and P[nx-k] (part 1) of every row y: the x
 // pass's output, the forward y pass's input: rows [nz][ny][2 parts][nkxp], 2 nz ny nkxp elements.
+// PT (the column kernels of small grids): columns [nz][nkxp][2 parts][ny], so that the x pass's stores,
+// which nothing waits for, are the scattered side and a column is one contiguous load.
+template <bool PT = false>
 __host__ __device__ __forceinline__ size_t p_index(const Geom& g, int l, int y, int part, int k) {
+    if (PT) return (((size_t)l * g.nkxp + k) * 2 + part) * g.ny + y;
     return ((size_t)l * g.ny + y) * 2 * g.nkxp + (size_t)part * g.nkxp + k;
 }
 
@@ -387,7 +391,7 @@ __device__ __forceinline__ void yinv_tile(const Geom g, int tid, int bx, int l, 
 // |u|u and |u|v and runs the same forward transforms.  A second launch for the bottom layer alone,
 // which it replaces, was 15 us of latency per right-hand side (64 CTAs at 512^2).
 // ------------------------------------------------------------------------------------
-template <int NX, bool DRAG, class CT, int TV = 0>
+template <int NX, bool DRAG, class CT, int TV = 0, bool PT = false>
 __device__ __forceinline__ void xpass_tile(const Geom g, int tid, int bx, int layer, const CT* __restrict__ pq,
                                            const CT* __restrict__ pv, const CT* __restrict__ pu,
                                            CT* __restrict__ pp, CT* __restrict__ pd, const CT* __restrict__ twx) {
@@ -451,10 +455,10 @@ __device__ __forceinline__ void xpass_tile(const Geom g, int tid, int bx, int la
     CT* out = drag ? pd : pp;
     auto st_fwd = [&](int k, CT v) {
         if (k < nkx) {
-            const size_t i = p_index(g, ol, y, 0, k);
+            const size_t i = p_index<PT>(g, ol, y, 0, k);
             if (in_bounds(g, i, olen)) out[i] = v;
         } else if (k > NX - nkx) {
-            const size_t i = p_index(g, ol, y, 1, NX - k);
+            const size_t i = p_index<PT>(g, ol, y, 1, NX - k);
             if (in_bounds(g, i, olen)) out[i] = v;
         }
     };
@@ -519,15 +523,6 @@ __device__ __forceinline__ void stage_rows(const Geom& g, int tid, int threads, 
     }
 }
 
-// split of the packed forward x transform of row y at kx: fld 0 -> (uq)^, fld 1 -> (vq)^
-__device__ __forceinline__ double2 unpack_p(const double2* __restrict__ P, const Geom& g, int l, int y, int kx,
-                                            int fld) {
-    const double2 X = P[p_index(g, l, y, 0, kx)];
-    const double2 Y = kx == 0 ? cconj(X) : cconj(P[p_index(g, l, y, 1, kx)]);
-    return fld == 0 ? make_double2(0.5 * (X.x + Y.x), 0.5 * (X.y + Y.y))
-                    : make_double2(0.5 * (X.y - Y.y), -0.5 * (X.x - Y.x));
-}
-
 // the thread of field fld loads part fld (P[k] for fld 0, P[nx-k] for fld 1) at index i and
 // swaps it with its partner's, so each value is read once
 template <class CT>
@@ -543,12 +538,13 @@ __device__ __forceinline__ CT unpack_pair(const CT* __restrict__ P, size_t i, in
                     : cmk<CT>((typename CTraits<CT>::R)0.5 * (X.y - Y.y), -(typename CTraits<CT>::R)0.5 * (X.x - Y.x));
 }
 
-template <int NY, bool DRAG, class CT, int TV = 0, bool MAP = false>
+template <int NY, bool DRAG, class CT, int TV = 0, bool MAP = false, bool PT = false>
 __device__ __forceinline__ void yfwd_tile(const Geom g, int tid, int bx, int l, const LayerConst* __restrict__ lc,
                                           const CT* __restrict__ q, const CT* __restrict__ psi,
                                           const CT* __restrict__ pp, const CT* __restrict__ pd,
                                           CT* __restrict__ out, const CT* __restrict__ twy,
                                           const CT* __restrict__ extra = nullptr, const YfwdMaps* maps = nullptr) {
+    static_assert(!(PT && (MAP || DRAG)), "columns come by plain loads, without drag");
     using C = YFwdCfg<NY, DRAG, CT, TV>;
     using RT = typename CTraits<CT>::R;
     extern __shared__ __align__(128) unsigned char sm_raw[];
@@ -604,7 +600,7 @@ __device__ __forceinline__ void yfwd_tile(const Geom g, int tid, int bx, int l, 
     // the (uq)^ and (vq)^ slots of one column load P[k] and P[nx-k] respectively and swap
     // them with a shuffle (partner tid ^ TKX, same warp), so each value is read once
     auto ld = [&](int y) -> CT {
-        const size_t i = p_index(g, l, y, fld, kx0 + c);
+        const size_t i = p_index<PT>(g, l, y, fld, kx0 + c);
         const bool ok = colok && in_bounds(g, i, 2 * g.hsize());
         return unpack_pair(pp, i, kx0 + c, fld, ok, C::TKX);
     };

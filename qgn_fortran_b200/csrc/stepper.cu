@@ -706,6 +706,8 @@ struct StageYinvCfg {
     static_assert(2 * HY <= TS, "de-interleaved rows fit the slot");
     static_assert(G >= 8 && G <= 32, "one slot per 8..32 lanes");
     static constexpr int SLOT_BYTES = SLOTS * TS * 16;
+    // the staged forward x transforms fit the last NZ slots and the column arrays (nky >= NY/2)
+    static_assert(2 * NY <= TS + NY, "staging");
 };
 
 // Stage S (S = 0: the state itself) of column kx: q_S at every kept mode of the column for all
@@ -821,14 +823,40 @@ __global__ void __launch_bounds__(StageYinvCfg<NY, NZ>::THREADS)
     const int tid = threadIdx.x;
     const int kx = blockIdx.x;
     const int nky = g.nky;
-    {   // forward y transforms of (uq)^ (slots 0..NZ-1) and (vq)^ (slots NZ..2NZ-1), unpadded
+    // The column's forward x transforms of every layer, [part][y] each, staged where the third of the
+    // slots that the forward transforms leave idle and the stage's column arrays lie, by one bulk copy per
+    // layer.  Read row by row from the rows' layout -- one 16-byte piece per line, twice per field -- they
+    // were 3 us of this kernel at 128^2 x 4 and 8 us at 256^2 x 2.
+    double2* stage = slots + 2 * NZ * C::TS;
+    {
+        uint64_t* bar = reinterpret_cast<uint64_t*>(sm_raw + C::SLOT_BYTES + 2 * NZ * nky * 16);
+        if (g.wait_err) {
+            if (tid == 0) bar_init(bar);
+            __syncthreads();
+            if (tid == 0) {
+                bar_expect_tx(bar, (uint32_t)(NZ * 2 * NY * 16));
+                for (int l = 0; l < NZ; ++l)
+                    bulk_g2s(stage + l * 2 * NY, pp + p_index<true>(g, l, 0, 0, kx), 2 * NY * 16, bar);
+            }
+            if (!bar_wait_bounded(bar, 0)) {
+                atomicExch(g.wait_err, 1);            // the controller halts the run on it
+                bar_wait_bounded(bar, 0);            // once more for the copies still in flight
+            }
+        } else {
+            for (int e = tid; e < NZ * 2 * NY; e += C::THREADS)
+                stage[e] = pp[p_index<true>(g, e / (2 * NY), e % NY, (e / NY) % 2, kx)];
+            __syncthreads();
+        }
+        // forward y transforms of (uq)^ (slots 0..NZ-1) and (vq)^ (slots NZ..2NZ-1), unpadded
         const int slot = tid / C::G, lane = tid % C::G;
         const int f = slot / NZ, l = slot % NZ;
         const bool act = slot < 2 * NZ;
         double2* xs = slots + slot * C::TS;
-        auto ld = [&](int y) -> double2 { return unpack_p(pp, g, act ? l : 0, y, kx, f); };
+        const double2* col = stage + (act ? l : 0) * 2 * NY;
+        auto ld = [&](int y) -> double2 { return split_p(col[y], col[NY + y], kx, f); };
         auto omap = [](int y) { return y; };
         fft_fused<NY, -1, SRC_FN, DST_SMEM_MAP, 16, true>(xs, lane, act, twy, ld, omap);
+        if (g.wait_err && tid == 0) bar_inval(bar);
     }
     const double kxv = g.dkx * kx;
     const bool expl = lc->explicit_diss != 0;
@@ -885,7 +913,7 @@ static cudaError_t column_smem(const void* kern, int bytes) {
 template <int NZ, int NY, class Kern, class... Args>
 static cudaError_t stage_yinv_launch(const Geom& g, Kern kern, int kid, double nb, cudaStream_t st, Args... args) {
     using C = StageYinvCfg<NY, NZ>;
-    const int smem = C::SLOT_BYTES + 2 * NZ * g.nky * 16;
+    const int smem = C::SLOT_BYTES + 2 * NZ * g.nky * 16 + 16;   // (the last 16: the bulk copies' barrier)
     cudaError_t e = column_smem(reinterpret_cast<const void*>(kern), smem);
     if (e != cudaSuccess) return e;
     QGN_LAUNCH(kid, nb, st, ::qgn::launch(kern, g.nkx, C::THREADS, smem, st, args...));
