@@ -46,8 +46,11 @@ struct StagePtrs {
 };
 
 __device__ __forceinline__ void point_k(const Geom& g, size_t p, int& kx, int& m, double& k2) {
-    kx = (int)(p / g.nky);
-    m = (int)(p % g.nky);
+    // 32-bit division (a field has at most 32 x 682 x 1365 elements): the 64-bit one was as much work as
+    // the rest of a streaming kernel's thread (update 59.8 -> 57.7 us at 1024^2 x 8 FP64, 255 -> 241 us at
+    // 2048^2 x 16 mixed)
+    kx = (int)((unsigned)p / (unsigned)g.nky);
+    m = (int)((unsigned)p % (unsigned)g.nky);
     const double kxv = g.dkx * kx, kyv = g.kyval(g.jfull(m));
     k2 = kxv * kxv + kyv * kyv;
 }
@@ -67,8 +70,8 @@ __global__ void __launch_bounds__(256) k_ark_update(Geom g, StagePtrs sp, const 
         sc->accept = 0;
     }
     if (e >= total) return;
-    const int l = (int)(e / P);
-    const size_t p = e % P;
+    const int l = (int)((unsigned)e / (unsigned)P);
+    const size_t p = e - (size_t)l * P;
     int kx, m;
     double k2;
     point_k(g, p, kx, m, k2);
@@ -164,8 +167,8 @@ __global__ void __launch_bounds__(256) k_ark_comb(Geom g, CombPtrs<T> cp, const 
     const size_t total = P * g.nz;
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= total) return;
-    const int l = (int)(e / P);
-    const size_t p = e % P;
+    const int l = (int)((unsigned)e / (unsigned)P);
+    const size_t p = e - (size_t)l * P;
     int kx, m;
     double k2;
     point_k(g, p, kx, m, k2);
@@ -222,8 +225,8 @@ __global__ void __launch_bounds__(256) k_ark_update_mixed(Geom g, StagePtrs32 sp
         sc->accept = 0;
     }
     if (e >= total) return;
-    const int l = (int)(e / P);
-    const size_t p = e % P;
+    const int l = (int)((unsigned)e / (unsigned)P);
+    const size_t p = e - (size_t)l * P;
     int kx, m;
     double k2;
     point_k(g, p, kx, m, k2);
@@ -1085,12 +1088,13 @@ cudaError_t launch_lincomb(const Geom& g, const Combo& cb, double2* out, cudaStr
     return cudaGetLastError();
 }
 
-// blocks per layer of the Parseval reductions: about 8 per SM over all layers, so each thread
-// streams only a few dozen modes (with 2 per SM the Leith reduction of 1024^2 x 8 read its
-// 29.8 MB at 1.1 TB/s); the partials buffer holds 512 x kMaxNZ doubles, 3 x nz x nb at most here
+// blocks per layer of the Parseval reductions: about 4 per SM over all layers.  Fewer leave each thread
+// too many modes to stream (2 per SM: the Leith reduction of 1024^2 x 8 read its 29.8 MB at 1.1 TB/s),
+// more are counted one by one in the last-block count (8: 19.3 us, 4: 17.4 us, events included); the
+// partials buffer holds 512 x kMaxNZ doubles, 3 x nz x nb at most here
 static int parseval_blocks(const Geom& g) {
     const size_t P = (size_t)g.nkx * g.nky;
-    const size_t want = (size_t)(8 * 148 + g.nz - 1) / g.nz;
+    const size_t want = (size_t)(4 * 148 + g.nz - 1) / g.nz;
     size_t nb = (P + 255) / 256;
     if (nb > want) nb = want;
     if (nb > 512) nb = 512;
