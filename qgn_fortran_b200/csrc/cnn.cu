@@ -2035,6 +2035,11 @@ int qgn_cnn_gradients(qgn_cnn* net, const void* x, const float* y, int batch, fl
     if (!net || !x || !y || batch < 1 || batch > net->max_batch) return QGN_ERR_ARG;
     const size_t xb = npix(net, batch) * net->ci[0] * sizeof(__nv_bfloat16);
     NCK(cudaMemcpyAsync(net->act[0], x, xb, cudaMemcpyDeviceToDevice, net->stream));
+    if (reinterpret_cast<uintptr_t>(y) % 16 != 0) {   // k_mse loads 16 bytes at a time
+        const size_t yb = npix(net, batch) * net->co[net->layers - 1] * sizeof(float);
+        NCK(cudaMemcpyAsync(net->ytgt, y, yb, cudaMemcpyDeviceToDevice, net->stream));
+        y = net->ytgt;
+    }
     int rc = forward(net, batch, true);
     if (rc == QGN_OK) rc = mse(net, batch, y);
     if (rc == QGN_OK) rc = backward(net, batch);

@@ -45,3 +45,23 @@ def test_layers(cuda_ok, H, W, layers, batch, engine):
     for (gw, gb), (ww, wb) in zip(grads, wgrads):
         assert rel(gw, ww) <= 1e-3
         assert rel(gb, wb) <= 1e-3
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+def test_target_of_any_alignment(cuda_ok, offset):
+    """The loss kernel reads 16 bytes of the target at a time; a target at any float gives the same bytes."""
+    import torch
+    nz, H, W, batch = 2, 4, 128, 2
+    net = ClosureNet(nz=nz, H=H, W=W, layers=2, max_batch=batch, seed=1)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn((batch, H, W, net.cin_p), generator=g, device="cuda").to(torch.bfloat16)
+    y = torch.randn((batch, H, W, net.cout_p), generator=g, device="cuda")
+    buf = torch.zeros(y.numel() + 4, device="cuda")
+    moved = buf[offset:offset + y.numel()].view(y.shape)
+    moved.copy_(y)
+    assert moved.data_ptr() % 16 == 4 * offset
+    loss, grads = net.gradients(x, moved, batch)
+    want, wgrads = net.gradients(x, y, batch)
+    assert loss == want
+    for (gw, gb), (ww, wb) in zip(grads, wgrads):
+        assert np.array_equal(gw, ww) and np.array_equal(gb, wb)
