@@ -1250,8 +1250,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_cnn_fused(FusedArgs a) {
 // as one partial per chunk of at most kWgRows rows, which bounds the length of the FP32 sums in TMEM.
 // 64 -> 64 at batch 32 on 128^2 (B200, ncu): one CTA per tap row 195 us with one stage in flight, 146 us
 // with the roles split, 89 us with swizzled tensor-map rows and MMAs issued from uniform registers;
-// this form 51 us, its traffic alone 20.
-constexpr int kWgRows = 32;          // most row segments per partial
+// this form 51 us with partials of 28 rows, its traffic alone 20.  16 rows, the mma.sync engine's length,
+// keep the FP32 sums as short as they were: six layers' gradients 1.27 -> 1.32 ms, and the twice as long
+// sums trained a network of 4.9 % online spectrum error where these give 2.8 %.
+constexpr int kWgRows = 16;          // most row segments per partial
 namespace tc {
 template <int CX>
 struct WgLay {
@@ -1669,7 +1671,8 @@ cudaError_t launch_conv(qgn_cnn* n, int cin, int cout, const __nv_bfloat16* x, c
 // partials of the tcgen05 weight gradient: row segments per partial and their number
 int wg_rows(const qgn_cnn* n, int batch) {
     const int tiles = batch * n->H * (n->W / kTileP);
-    return std::min(kWgRows, (tiles + 147) / 148);
+    const int waves = (tiles + 148 * kWgRows - 1) / (148 * kWgRows);   // the fewest with partials that short
+    return (tiles + 148 * waves - 1) / (148 * waves);
 }
 int wg_chunks(const qgn_cnn* n, int batch) {
     const int tiles = batch * n->H * (n->W / kTileP), r = wg_rows(n, batch);
@@ -1925,8 +1928,8 @@ int qgn_cnn_create(int cin, int width, int cout, int layers, int H, int W, int m
         net->gb[l] = net->grads + np;
         np += net->co[l];
     }
-    // most partials of any batch up to max_batch: 148, or one per kWgRows rows
-    const size_t max_chunks = std::max<size_t>(148, ((size_t)max_batch * H * (W / kTileP) + kWgRows - 1) / kWgRows);
+    // most partials of any batch up to max_batch: 148 in every wave of CTAs
+    const size_t max_chunks = 148 * (((size_t)max_batch * H * (W / kTileP) + 148 * kWgRows - 1) / (148 * kWgRows));
     std::mt19937_64 rng(seed);
     for (int l = 0; l < layers; ++l) {
         const int nw = 9 * net->co[l] * net->ci[l];
