@@ -21,8 +21,8 @@ extern "C" {
  * (compact), 2..6 the half-transformed fields [nz][ny][nkxp] of the last RHS as packed row
  * pairs [nz][ny/2][2][nkxp]: 2 q, 3 v = i kx psi, 4 u = -i ky psi; 5 the forward x transforms
  * P of u*q + i v*q row by row, [nz][ny][2][nkxp] (P[k] at k and P[nx-k] at nkxp + k, for
- * k < nkx; a build with -DQGN_P_TILED=1 stores them in tiles of two kx columns instead,
- * [nz][nkxp/2][ny][2][2]).  nkxp = nx/3 rounded up to a multiple of 4.
+ * k < nkx; the column kernels of small grids store them by column instead, [nz][nkxp][2][ny]).
+ * nkxp = nx/3 rounded up to a multiple of 4.
  */
 int qgn_debug_read(qgn_ctx* ctx, int which, double* out, long long count);
 

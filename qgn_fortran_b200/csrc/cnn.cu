@@ -20,7 +20,7 @@
 //   k_mse                 loss and dL/dY = 2 (Y - T)/count, as BF16 G of the last layer
 //   k_adam                Adam on the FP32 masters, refreshing both BF16 layouts
 //   k_conv_tc<CIN,COUT,EPI>  the implicit GEMM on tcgen05 (TMEM accumulators)
-//   k_wgrad_tc<CIN,COUT>  the weight-gradient partials on tcgen05 (M = 64, MN-major operands)
+//   k_wgrad_tc<CX,SWAP>   the weight- and bias-gradient partials on tcgen05 (MN-major operands)
 //   k_cnn_fused           every layer of a small-batch inference, rows exchanged through L2
 #include "qgn_internal.cuh"
 #include "cnn.cuh"
@@ -1251,8 +1251,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_cnn_fused(FusedArgs a) {
 // 64 -> 64 at batch 32 on 128^2 (B200, ncu): one CTA per tap row 195 us with one stage in flight, 146 us
 // with the roles split, 89 us with swizzled tensor-map rows and MMAs issued from uniform registers;
 // this form 51 us with partials of 28 rows, its traffic alone 20.  16 rows, the mma.sync engine's length,
-// keep the FP32 sums as short as they were: six layers' gradients 1.27 -> 1.32 ms, and the twice as long
-// sums trained a network of 4.9 % online spectrum error where these give 2.8 %.
+// keep the FP32 sums as short as there: six layers' gradients at batch 32 1.27 -> 1.32 ms.
 constexpr int kWgRows = 16;          // most row segments per partial
 namespace tc {
 template <int CX>
