@@ -1,6 +1,7 @@
 """The layer kernels of the closure network where their row streams change shape: images of one and
 two rows (every tile's three rows wrap), runs of rows that end inside and across a CTA's range, several
-row segments per image row, batches with fewer rows than CTAs and with more.  Both tensor-core engines
+row segments per image row, batches with fewer rows than CTAs, with more, and with several chunks of rows
+per CTA of the weight gradient.  Both tensor-core engines
 against the FP64 network with the BF16 roundings of the GPU, to the bounds of
 tests/test_gpu_closure.py (forward 1e-4, gradients 1e-3 of the tensor's norm), and the tcgen05 engine's
 inference against its training forward.
@@ -20,7 +21,8 @@ def rel(a, b):
 
 @pytest.mark.parametrize("engine", ["tcgen05-layers", "mma.sync"])
 @pytest.mark.parametrize("H,W,layers,batch", [(1, 128, 2, 1), (2, 128, 3, 1), (3, 256, 3, 1), (7, 128, 3, 30),
-                                              (5, 384, 2, 11), (50, 128, 3, 3), (160, 128, 2, 1)])
+                                              (5, 384, 2, 11), (50, 128, 3, 3), (160, 128, 2, 1),
+                                              (100, 128, 2, 24)])
 def test_layers(cuda_ok, H, W, layers, batch, engine):
     import torch
     nz = 3
