@@ -34,6 +34,12 @@ int qgn_debug_read(qgn_ctx* ctx, int which, double* out, long long count);
 int qgn_cnn_debug_set_counter(qgn_cnn* net, int tile, unsigned int value);
 
 /*
+ * CTAs of an ensemble's x pass that are resident on an SM at once with its present tiles
+ * (qgn_ens_set_tiles), the most over the pass's launches.
+ */
+int qgn_ens_debug_residency(qgn_ens* ens, int* ctas_per_sm);
+
+/*
  * Bounds-checked build (libqgn_b200_check.so, every source compiled with -DQGN_CHECK): the
  * right-hand-side transforms and GetPsi test each global index against the length of the
  * array it addresses and skip, and count, an access out of range instead of making it.

@@ -546,7 +546,10 @@ struct qgn_ens {
     int* d_any = nullptr;
     int* h_any = nullptr;            // pinned
     int variant[TP_COUNT] = {kDefaultVariant, kDefaultVariant, kDefaultVariant};
-    int grid_mode[TP_COUNT] = {0, 0, 0};   // 0: one CTA per tile; k > 0: k CTAs per SM, persistent
+    // 0: one CTA per tile; k > 0: k CTAs per SM, persistent (y passes), or one CTA per tile and at most
+    // k resident on an SM (x pass)
+    int grid_mode[TP_COUNT] = {0, 0, 0};
+    int smem_sm = 0, smem_cta = 0, smem_reserved = 0;   // shared memory: of an SM, most of a CTA, reserved per CTA
     float tuned_ms[TP_COUNT] = {0.f, 0.f, 0.f};
     bool pinned[TP_COUNT] = {false, false, false};   // set by qgn_ens_set_tiles: not tuned
     bool tuned = false;
@@ -737,14 +740,28 @@ int launch_yinv_tv(qgn_ens* e, int s, int grid) {
     return QGN_OK;
 }
 
+// dynamic shared memory that keeps at most k CTAs of `need` bytes each on an SM: the least size of which
+// k + 1, with what the system reserves per CTA, do not fit (a CTA cannot have more than smem_cta, which
+// leaves room for no second one)
+int limited_smem(const qgn_ens* e, int need, int k) {
+    constexpr int kUnit = 128;   // allocation granularity
+    const int s = (e->smem_sm / (k + 1) - e->smem_reserved) / kUnit * kUnit + kUnit;
+    return std::max(need, std::min(s, e->smem_cta));
+}
+
+// occupancy: the resident CTAs per SM instead of a launch
 template <int N, class CT, int TV>
-int launch_xgroup(qgn_ens* e, const qgn_ens::XGroup& x, int s) {
+int launch_xgroup(qgn_ens* e, const qgn_ens::XGroup& x, int s, int* occupancy) {
     // one CTA per tile; k > 0 CTAs per SM are a limit on the resident ones, by their shared memory
-    constexpr int kSmShared = 227 * 1024;
     const int gm = e->grid_mode[TP_XPASS], ng = (int)x.members.size();
-    const int SM = gm == 0 ? XCfg<N, false, CT, TV>::SMEM
-                           : std::max(XCfg<N, false, CT, TV>::SMEM, kSmShared / (gm + 1) / 1024 * 1024);
+    const int SM = gm == 0 ? XCfg<N, false, CT, TV>::SMEM : limited_smem(e, XCfg<N, false, CT, TV>::SMEM, gm);
     ECK(smem_attr(k_ens_xpass<N, CT, TV>, SM));
+    if (occupancy) {
+        int n = 0;
+        ECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_ens_xpass<N, CT, TV>, 3 * tv_width(TV), SM));
+        *occupancy = std::max(*occupancy, n);
+        return QGN_OK;
+    }
     double bytes = 0.0;
     for (int m : x.members) {
         const Geom& g = e->mem[m]->g;
@@ -760,13 +777,13 @@ int launch_xgroup(qgn_ens* e, const qgn_ens::XGroup& x, int s) {
 }
 
 template <class CT, int TV>
-int launch_xpass_tv(qgn_ens* e, int s) {
+int launch_xpass_tv(qgn_ens* e, int s, int* occupancy) {
     for (const qgn_ens::XGroup& x : e->xgroups) {
         int r = QGN_ERR_CONFIG;
         switch (x.nx) {
-            case 128: r = launch_xgroup<128, CT, TV>(e, x, s); break;
-            case 256: r = launch_xgroup<256, CT, TV>(e, x, s); break;
-            case 512: r = launch_xgroup<512, CT, TV>(e, x, s); break;
+            case 128: r = launch_xgroup<128, CT, TV>(e, x, s, occupancy); break;
+            case 256: r = launch_xgroup<256, CT, TV>(e, x, s, occupancy); break;
+            case 512: r = launch_xgroup<512, CT, TV>(e, x, s, occupancy); break;
             default: break;
         }
         if (r != QGN_OK) return r;
@@ -795,9 +812,10 @@ int launch_yinv_v(qgn_ens* e, int v, int s, std::index_sequence<I...>) {
     return r;
 }
 template <class CT, size_t... I>
-int launch_xpass_v(qgn_ens* e, int v, int s, std::index_sequence<I...>) {
+int launch_xpass_v(qgn_ens* e, int v, int s, std::index_sequence<I...>, int* occupancy = nullptr) {
     int r = QGN_ERR_CONFIG;
-    (void)((v == (int)I ? (r = launch_xpass_tv<CT, ens_variant<CT>(TP_XPASS, (int)I)>(e, s), true) : false) || ...);
+    (void)((v == (int)I ? (r = launch_xpass_tv<CT, ens_variant<CT>(TP_XPASS, (int)I)>(e, s, occupancy), true) : false) ||
+           ...);
     return r;
 }
 template <class CT, size_t... I>
@@ -814,6 +832,14 @@ int launch_pass(qgn_ens* e, int tp, int s) {
     if (tp == TP_YINV) return launch_yinv_v<CT>(e, v, s, std::make_index_sequence<ens_variant_count<CT>(TP_YINV)>{});
     if (tp == TP_XPASS) return launch_xpass_v<CT>(e, v, s, std::make_index_sequence<ens_variant_count<CT>(TP_XPASS)>{});
     return launch_yfwd_v<CT>(e, v, s, std::make_index_sequence<ens_variant_count<CT>(TP_YFWD)>{});
+}
+
+// CTAs of the x pass resident on an SM as it is launched now (the most of its launches)
+template <class CT>
+int xpass_occupancy(qgn_ens* e, int* occupancy) {
+    *occupancy = 0;
+    return launch_xpass_v<CT>(e, e->variant[TP_XPASS], 0, std::make_index_sequence<ens_variant_count<CT>(TP_XPASS)>{},
+                              occupancy);
 }
 
 template <class CT>
@@ -1026,7 +1052,12 @@ int qgn_ens_create(qgn_ctx* const* members, int nmembers, int precision, qgn_ens
         return code;
     };
     if (cudaSetDevice(e->device) != cudaSuccess) return fail(QGN_ERR_CUDA);
-    cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, e->device);
+    const std::pair<int*, cudaDeviceAttr> attrs[] = {{&e->sms, cudaDevAttrMultiProcessorCount},
+                                                     {&e->smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor},
+                                                     {&e->smem_cta, cudaDevAttrMaxSharedMemoryPerBlockOptin},
+                                                     {&e->smem_reserved, cudaDevAttrReservedSharedMemoryPerBlock}};
+    for (const auto& a : attrs)
+        if (cudaDeviceGetAttribute(a.first, a.second, e->device) != cudaSuccess) return fail(QGN_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(QGN_ERR_CUDA);
     if (cudaMalloc((void**)&e->d_mem, sizeof(EnsMember) * nmembers) != cudaSuccess) return fail(QGN_ERR_CUDA);
     if (cudaMalloc((void**)&e->d_start, sizeof(int) * (size_t)EP_COUNT * (nmembers + 1)) != cudaSuccess)
@@ -1178,6 +1209,12 @@ int qgn_ens_set_tiles(qgn_ens* e, int pass, int threads, int elements_per_thread
         }
     }
     return ens_err(e, QGN_ERR_CONFIG, "no tile variant with these threads and elements per thread");
+}
+
+int qgn_ens_debug_residency(qgn_ens* e, int* ctas_per_sm) {
+    if (!e || !ctas_per_sm) return QGN_ERR_ARG;
+    ECK(cudaSetDevice(e->device));
+    return fp32(e) ? xpass_occupancy<float2>(e, ctas_per_sm) : xpass_occupancy<double2>(e, ctas_per_sm);
 }
 
 int qgn_ens_profile_enable(qgn_ens* e, int on) {
