@@ -34,6 +34,14 @@ int qgn_debug_read(qgn_ctx* ctx, int which, double* out, long long count);
 int qgn_cnn_debug_set_counter(qgn_cnn* net, int tile, unsigned int value);
 
 /*
+ * Failure injection: set a flag that a bounded device wait of this context sets when it runs out.
+ * which: 0 the adaptive steps' flag (the next attempt halts the run), 1 the flag of everything else
+ * (right-hand sides, physical fields, training samples, fixed-step schemes: the next such call
+ * returns QGN_ERR_CUDA and clears it).
+ */
+int qgn_debug_set_wait(qgn_ctx* ctx, int which, int value);
+
+/*
  * CTAs of an ensemble's x pass that are resident on an SM at once with its present tiles
  * (qgn_ens_set_tiles), the most over the pass's launches.
  */

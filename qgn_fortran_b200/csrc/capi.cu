@@ -17,6 +17,8 @@
 using namespace qgn;
 
 namespace qgn {
+static const char* const kWaitText = "a bounded device wait ran out";
+
 Prof*& current_prof() {
     thread_local Prof* p = nullptr;
     return p;
@@ -30,6 +32,19 @@ void drop_graphs(qgn_ctx* ctx) {
             ctx->gexec[w] = nullptr;
         }
     ctx->graphs_ready = false;
+}
+
+Geom call_geom(const qgn_ctx* ctx) {
+    Geom g = ctx->g;
+    g.wait_err = const_cast<int*>(ctx->call_wait);
+    return g;
+}
+
+int take_call_wait(qgn_ctx* ctx) {
+    if (!*ctx->call_wait) return QGN_OK;
+    *ctx->call_wait = 0;
+    ctx->last_error = kWaitText;
+    return QGN_ERR_CUDA;
 }
 }  // namespace qgn
 
@@ -170,9 +185,23 @@ const char* status_text(int st) {
     switch (st) {
         case QGN_ERR_NONFINITE: return "non-finite embedded error estimate";
         case QGN_ERR_REJECT_LIMIT: return "adaptive step rejected max_rejects times in a row";
-        case QGN_ERR_CUDA: return "a bounded device wait ran out";
+        case QGN_ERR_CUDA: return kWaitText;
         default: return "step failed";
     }
+}
+
+bool adaptive(int scheme) {
+    return scheme == QGN_SCHEME_ARK43_QGLEITH || scheme == QGN_SCHEME_ARK43 || scheme == QGN_SCHEME_BSRK3;
+}
+
+// after the steps of a fixed-step scheme: a wait that ran out leaves the state and AB3's history unusable
+int fixed_step_wait(qgn_ctx* ctx) {
+    const int rc = take_call_wait(ctx);
+    if (rc != QGN_OK) {
+        ctx->halted = true;
+        ctx->ab_calls = 0;
+    }
+    return rc;
 }
 
 bool drag_on(const qgn_ctx* ctx) { return ctx->p.C_d != 0.0; }
@@ -472,6 +501,7 @@ int step_bsrk3(qgn_ctx* ctx) {
         RET(read_scalars(ctx, &s));
         if (s.halt) {
             ctx->halted = true;
+            if (s.status == QGN_ERR_CUDA) ctx->first_call = true;   // RHS0 may be what lost its wait
             return set_err(ctx, s.status, status_text(s.status));
         }
         if (s.accept) {
@@ -549,7 +579,7 @@ int check_state(qgn_ctx* ctx) {
     DevScalars s;
     CK(launch_nonfinite_check(ctx->g, ctx->b.q, ctx->b.sc, ctx->stream));
     RET(read_scalars(ctx, &s));
-    if (s.wait_timeout) return set_err(ctx, QGN_ERR_CUDA, "a bounded device wait ran out");
+    RET(fixed_step_wait(ctx));
     if (s.nonfinite) return set_err(ctx, QGN_ERR_NONFINITE, "non-finite values in the state q_hat");
     return QGN_OK;
 }
@@ -692,8 +722,6 @@ int qgn_create(const qgn_params* p, const double* H, const double* S, const doub
     AL(b.red, (size_t)512 * kMaxNZ);
     AL(b.Hw, (size_t)kMaxNZ);
     AL(b.lc, 1); AL(b.mc, 1); AL(b.sc, 1);
-    if (rc == QGN_OK)   // the sticky flag a bounded device wait sets when it runs out
-        g.wait_err = reinterpret_cast<int*>(reinterpret_cast<char*>(b.sc) + offsetof(DevScalars, wait_timeout));
 #ifdef QGN_CHECK
     AL(ctx->chk, 1);
     if (rc == QGN_OK) {
@@ -710,6 +738,13 @@ int qgn_create(const qgn_params* p, const double* H, const double* S, const doub
     if (rc == QGN_OK) {
         cudaError_t e = cudaMallocHost((void**)&ctx->host_pin, sizeof(DevScalars) + 64);
         if (e != cudaSuccess) fail("cudaMallocHost", e);
+    }
+    if (rc == QGN_OK) {   // the sticky flag a bounded device wait sets when it runs out
+        ctx->call_wait = reinterpret_cast<int*>(reinterpret_cast<char*>(ctx->host_pin) + sizeof(DevScalars));
+        *ctx->call_wait = 0;
+        g.wait_err = adaptive(scheme)
+                         ? reinterpret_cast<int*>(reinterpret_cast<char*>(b.sc) + offsetof(DevScalars, wait_timeout))
+                         : const_cast<int*>(ctx->call_wait);
     }
     if (rc == QGN_OK) {
         // zero everything once: padding columns of the half fields stay zero forever
@@ -829,7 +864,7 @@ int qgn_advance_resident(qgn_ctx* ctx, int nsteps) {
     RET(advance_n(ctx, nsteps));
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->prof.harvest();
-    return QGN_OK;
+    return adaptive(ctx->scheme) ? QGN_OK : fixed_step_wait(ctx);
 }
 
 int qgn_advance(qgn_ctx* ctx, double* q_hat, double* t, double* dt, int nsteps) {
@@ -841,9 +876,7 @@ int qgn_advance(qgn_ctx* ctx, double* q_hat, double* t, double* dt, int nsteps) 
     RET(qgn_set_state(ctx, q_hat, *t, *dt));
     RET(advance_n(ctx, nsteps));
     // the adaptive schemes' controller already halts on a non-finite error estimate
-    const bool adaptive = ctx->scheme == QGN_SCHEME_ARK43_QGLEITH || ctx->scheme == QGN_SCHEME_ARK43 ||
-                          ctx->scheme == QGN_SCHEME_BSRK3;
-    if (!adaptive) RET(check_state(ctx));
+    if (!adaptive(ctx->scheme)) RET(check_state(ctx));
     RET(download_kept(ctx, ctx->b.q, q_hat));
     DevScalars s;
     RET(read_scalars(ctx, &s));
@@ -868,21 +901,21 @@ int qgn_rhs(qgn_ctx* ctx, const double* q_hat, double* rhs) {
     if (!q_hat || !rhs) return set_err(ctx, QGN_ERR_ARG, "NULL argument");
     CK(cudaSetDevice(ctx->device));
     Buffers& b = ctx->b;
+    const Geom g = call_geom(ctx);
     RET(upload_kept(ctx, q_hat, b.err));
     if (mixed(ctx)) {
         // FP32 RHS: the FP32 state copy goes to N[5], the FP32 result to qnew, widened into err
-        CK(launch_modal_mixed(ctx->g, b, b.err, f32(b.N[5]), f32(b.psi), ctx->stream));
-        CK(launch_rhs32(ctx->g, b, f32(b.N[5]), f32(b.psi), f32(b.qnew), drag_on(ctx), ctx->stream));
-        CK(launch_f2d(ctx->g.csize(), f32(b.qnew), b.err, ctx->stream));
+        CK(launch_modal_mixed(g, b, b.err, f32(b.N[5]), f32(b.psi), ctx->stream));
+        CK(launch_rhs32(g, b, f32(b.N[5]), f32(b.psi), f32(b.qnew), drag_on(ctx), ctx->stream));
+        CK(launch_f2d(g.csize(), f32(b.qnew), b.err, ctx->stream));
         RET(download_full(ctx, b.err, rhs));
-        CK(cudaStreamSynchronize(ctx->stream));
-        return QGN_OK;
+    } else {
+        CK(launch_modal(g, b, b.err, b.psi, ctx->stream));
+        CK(launch_rhs(g, b, b.err, b.psi, b.qnew, drag_on(ctx), ctx->stream));
+        RET(download_full(ctx, b.qnew, rhs));
     }
-    CK(launch_modal(ctx->g, b, b.err, b.psi, ctx->stream));
-    CK(launch_rhs(ctx->g, b, b.err, b.psi, b.qnew, drag_on(ctx), ctx->stream));
-    RET(download_full(ctx, b.qnew, rhs));
     CK(cudaStreamSynchronize(ctx->stream));
-    return QGN_OK;
+    return take_call_wait(ctx);
 }
 
 int qgn_psi(qgn_ctx* ctx, const double* q_hat, double* psi_hat) {
@@ -956,7 +989,7 @@ int qgn_physical(qgn_ctx* ctx, const double* q_hat, double* q_phys, double* psi_
     if (!ctx) return QGN_ERR_ARG;
     ProfScope ps_(ctx, __func__);
     CK(cudaSetDevice(ctx->device));
-    const Geom& g = ctx->g;
+    const Geom g = call_geom(ctx);
     Buffers& b = ctx->b;
     const size_t np = (size_t)g.nz * g.ny * g.nx;
     if (!b.phys) CK(dalloc(&b.phys, np));
@@ -975,7 +1008,7 @@ int qgn_physical(qgn_ctx* ctx, const double* q_hat, double* q_phys, double* psi_
         CK(cudaMemcpyAsync(psi_phys, b.phys, sizeof(double) * np, cudaMemcpyDeviceToHost, ctx->stream));
     }
     CK(cudaStreamSynchronize(ctx->stream));
-    return QGN_OK;
+    return take_call_wait(ctx);
 }
 
 int qgn_physical_modal(qgn_ctx* ctx, const double* q_hat, double* q_mode, double* p_mode, double* J_mode) {
@@ -983,7 +1016,7 @@ int qgn_physical_modal(qgn_ctx* ctx, const double* q_hat, double* q_mode, double
     ProfScope ps_(ctx, __func__);
     if (!q_mode || !p_mode || !J_mode) return set_err(ctx, QGN_ERR_ARG, "NULL output");
     CK(cudaSetDevice(ctx->device));
-    const Geom& g = ctx->g;
+    const Geom g = call_geom(ctx);
     Buffers& b = ctx->b;
     const Geom gf = full_geom(g);
     const size_t np = (size_t)g.nz * g.ny * g.nx;
@@ -1006,7 +1039,7 @@ int qgn_physical_modal(qgn_ctx* ctx, const double* q_hat, double* q_mode, double
     CK(cudaMemcpyAsync(p_mode, outs + np, sizeof(double) * np, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(J_mode, outs + 2 * np, sizeof(double) * np, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    return QGN_OK;
+    return take_call_wait(ctx);
 }
 
 int qgn_set_state_physical(qgn_ctx* ctx, const double* q_phys, double t, double dt) {
@@ -1075,6 +1108,15 @@ int qgn_debug_read(qgn_ctx* ctx, int which, double* out, long long count) {
     if ((size_t)count < 2 * n) return set_err(ctx, QGN_ERR_ARG, "output too small");
     CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaMemcpy(out, src, sizeof(double2) * n, cudaMemcpyDeviceToHost));
+    return QGN_OK;
+}
+
+int qgn_debug_set_wait(qgn_ctx* ctx, int which, int value) {
+    if (!ctx || which < 0 || which > 1) return QGN_ERR_ARG;
+    CK(cudaSetDevice(ctx->device));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (which == 1) *ctx->call_wait = value;
+    else CK(cudaMemcpy(&ctx->b.sc->wait_timeout, &value, sizeof(value), cudaMemcpyHostToDevice));
     return QGN_OK;
 }
 

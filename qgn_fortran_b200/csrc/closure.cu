@@ -374,8 +374,8 @@ int qgn_closure_snapshot(qgn_ctx* fine, qgn_ctx* coarse, const float* in_scale, 
     if (rc != QGN_OK) return rc;
     double* P0 = nullptr;
     if ((rc = snap_scratch(coarse, &P0)) != QGN_OK) return rc;
-    const Geom& gf = fine->g;
-    const Geom& gc = coarse->g;
+    const Geom gf = call_geom(fine);
+    const Geom gc = call_geom(coarse);
     const Buffers& bf = fine->b;
     const Buffers& bc = coarse->b;
     cudaStream_t s = fine->stream;
@@ -401,7 +401,8 @@ int qgn_closure_snapshot(qgn_ctx* fine, qgn_ctx* coarse, const float* in_scale, 
     ::qgn::launch(k_pack_in, grid_of(npix), 256, 0, s, nz, npix, P0, P1, sc, cin_p, static_cast<__nv_bfloat16*>(x_dev));
     ::qgn::launch(k_pack_out, grid_of(npix), 256, 0, s, nz, npix, P2, sc + 2 * nz, cout_p, y_dev);
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return QGN_ERR_CUDA;
-    return QGN_OK;
+    const int rf = take_call_wait(fine), rcs = take_call_wait(coarse);
+    return rf != QGN_OK ? rf : rcs;
 }
 
 int qgn_closure_attach(qgn_ctx* ctx, qgn_cnn* net, const float* in_scale, const float* out_scale, double A8_background,

@@ -1155,7 +1155,8 @@ int qgn_ens_advance(qgn_ens* e, int nsteps) {
         c->b.N[3] = static_cast<double2*>(M.N[3]);
         c->b.Qs[0] = c->b.q;
         // an FP64 ensemble leaves a valid FP64 RHS0 for the member's own BSRK3 steps
-        c->first_call = fp32(e) || M.need_fsal != 0;
+        // (and none after a wait that ran out: RHS0 may be what lost it)
+        c->first_call = fp32(e) || M.need_fsal != 0 || (s1[m].halt && s1[m].status == QGN_ERR_CUDA);
         e->seen_version[m] = c->state_version;
         if (s1[m].halt) {
             c->halted = true;
@@ -1166,6 +1167,7 @@ int qgn_ens_advance(qgn_ens* e, int nsteps) {
         char buf[160];
         std::snprintf(buf, sizeof(buf), "member %d halted: %s", first_bad,
                       s1[first_bad].status == QGN_ERR_NONFINITE ? "non-finite embedded error estimate"
+                      : s1[first_bad].status == QGN_ERR_CUDA    ? "a bounded device wait ran out"
                                                                 : "adaptive step rejected max_rejects times in a row");
         return ens_err(e, s1[first_bad].status ? s1[first_bad].status : QGN_ERR_CUDA, buf);
     }

@@ -29,7 +29,7 @@ struct Geom {
     int nkx, nky, kylo, kyshift, nkxp;
     double dkx, dky, inv_nxny;
     unsigned long long* chk = nullptr;   // failed-check counter of the bounds-checked build (device)
-    int* wait_err = nullptr;             // set to 1 when a bounded device wait runs out (device);
+    int* wait_err = nullptr;             // set to 1 when a bounded device wait runs out (device or pinned);
                                          // null: the kernels take no path that waits
     __host__ __device__ size_t csize() const { return (size_t)nz * nkx * nky; }
     __host__ __device__ size_t hsize() const { return (size_t)nz * ny * nkxp; }
@@ -167,6 +167,7 @@ struct qgn_ctx {
     qgn::Closure* closure = nullptr;   // learned closure of a coarse ARK43_QGLeith model (closure.cu)
     qgn::ModalConst mc_host{};     // host copy of b.mc (b.mc_h points here)
     double* host_pin = nullptr;    // pinned scalar readback
+    volatile int* call_wait = nullptr;   // pinned, written by the device: a bounded wait ran out (call_geom)
     std::vector<void*> owned;      // every device allocation made at creation
     std::string last_error;
     qgn::Prof prof;                // launch counts and per-kernel event timing
@@ -198,6 +199,14 @@ int closure_join(qgn_ctx* ctx);
 void closure_free(qgn_ctx* ctx);
 const double2* closure_tendency(const qgn_ctx* ctx);
 void drop_graphs(qgn_ctx* ctx);
+
+// ---- bounded waits outside the adaptive steps (capi.cu) -----------------------------------
+// The adaptive schemes' controller halts a run whose attempt lost a wait (wait_timeout).  What no
+// controller watches -- an evaluation beside the run, a step of a fixed-step scheme -- reports to the
+// context's pinned flag instead, which costs the call no copy: the geometry to launch it with, and,
+// once its work is done, whether a wait ran out (clears the flag; QGN_ERR_CUDA).
+Geom call_geom(const qgn_ctx* ctx);
+int take_call_wait(qgn_ctx* ctx);
 
 // ---- GetPsi (modal.cu) ------------------------------------------------------------------
 cudaError_t launch_modal(const Geom& g, const Buffers& b, const double2* q, double2* psi, cudaStream_t s);
