@@ -47,6 +47,9 @@ int qgn_debug_set_wait(qgn_ctx* ctx, int which, int value);
  */
 int qgn_ens_debug_residency(qgn_ens* ens, int* ctas_per_sm);
 
+/* How often an ensemble's tile tables have gone to the device: once per change of the tiles. */
+int qgn_ens_debug_uploads(qgn_ens* ens, int* count);
+
 /*
  * Bounds-checked build (libqgn_b200_check.so, every source compiled with -DQGN_CHECK): the
  * right-hand-side transforms and GetPsi test each global index against the length of the

@@ -65,7 +65,7 @@ struct EnsMember {
     int need_fsal;        // RHS0 of the current state is still to be computed
 };
 
-// passes with their own tile tables
+// passes with their own tile tables (EP_XPASS: one per grid size)
 enum { EP_POINT = 0, EP_ELEM, EP_YINV, EP_XPASS, EP_YFWD, EP_YINV1, EP_XINV1, EP_COUNT };
 // passes the autotuner chooses for
 enum { TP_YINV = 0, TP_XPASS, TP_YFWD, TP_COUNT };
@@ -533,6 +533,8 @@ struct qgn_ens {
     int map_at[EP_COUNT] = {};
     int* d_map = nullptr;
     size_t map_cap = 0;              // entries of d_map
+    bool tables_new = true;          // built since the last upload
+    int uploads = 0;
     // members of one grid size, for the x pass: their numbers and tile prefix sums at `table` of d_xgroups
     struct XGroup {
         int nx, ny;
@@ -610,10 +612,11 @@ void build_tables(qgn_ens* e) {
     const size_t nm = e->mem.size();
     e->h_start.assign((size_t)EP_COUNT * (nm + 1), 0);
     e->h_map.clear();
+    e->tables_new = true;
     for (int pass = 0; pass < EP_COUNT; ++pass) {
+        if (pass == EP_XPASS) continue;
         int tv = 0;
         if (pass == EP_YINV) tv = tv_of(e, TP_YINV);
-        if (pass == EP_XPASS) tv = tv_of(e, TP_XPASS);
         if (pass == EP_YFWD) tv = tv_of(e, TP_YFWD);
         int* st = &e->h_start[(size_t)pass * (nm + 1)];
         e->map_at[pass] = (int)e->h_map.size();
@@ -659,7 +662,9 @@ void group_members(qgn_ens* e) {
     });
 }
 
+// the tables to the device, if they are not those of the last upload
 int upload_tables(qgn_ens* e) {
+    if (!e->tables_new) return QGN_OK;
     if (e->h_map.size() > e->map_cap) {   // (a captured graph holds the old address)
         if (e->gexec) {
             ECK(cudaStreamSynchronize(e->stream));
@@ -677,6 +682,8 @@ int upload_tables(qgn_ens* e) {
                         e->stream));
     ECK(cudaMemcpyAsync(e->d_xgroups, e->h_xgroups.data(), sizeof(int) * e->h_xgroups.size(), cudaMemcpyHostToDevice,
                         e->stream));
+    e->tables_new = false;
+    ++e->uploads;
     return QGN_OK;
 }
 
@@ -1217,6 +1224,12 @@ int qgn_ens_debug_residency(qgn_ens* e, int* ctas_per_sm) {
     if (!e || !ctas_per_sm) return QGN_ERR_ARG;
     ECK(cudaSetDevice(e->device));
     return fp32(e) ? xpass_occupancy<float2>(e, ctas_per_sm) : xpass_occupancy<double2>(e, ctas_per_sm);
+}
+
+int qgn_ens_debug_uploads(qgn_ens* e, int* count) {
+    if (!e || !count) return QGN_ERR_ARG;
+    *count = e->uploads;
+    return QGN_OK;
 }
 
 int qgn_ens_profile_enable(qgn_ens* e, int on) {
