@@ -220,7 +220,8 @@ static cudaError_t launch_modal_any(const Geom& g, const Buffers& b, const TI* q
             case 8: return modal_small<8, TI, TO, COPY>(g, b, q, psi, qcopy, s);
             default: break;
         }
-        if (g.nz == 16 && sizeof(TI) == 8) return modal_small<16, TI, TO, COPY>(g, b, q, psi, qcopy, s);
+        if constexpr (sizeof(TI) == 8)
+            if (g.nz == 16) return modal_small<16, TI, TO, COPY>(g, b, q, psi, qcopy, s);
         if (g.nz <= 16) return modal_wide<16, TI, TO, COPY>(g, b, q, psi, qcopy, s);
         if (g.nz <= 24) return modal_wide<24, TI, TO, COPY>(g, b, q, psi, qcopy, s);
         return modal_wide<32, TI, TO, COPY>(g, b, q, psi, qcopy, s);

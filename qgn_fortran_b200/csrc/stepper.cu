@@ -832,23 +832,18 @@ __global__ void __launch_bounds__(StageYinvCfg<NY, NZ>::THREADS)
     // were 3 us of this kernel at 128^2 x 4 and 8 us at 256^2 x 2.
     double2* stage = slots + 2 * NZ * C::TS;
     {
+        // (only contexts come here, and a context has a wait flag)
         uint64_t* bar = reinterpret_cast<uint64_t*>(sm_raw + C::SLOT_BYTES + 2 * NZ * nky * 16);
-        if (g.wait_err) {
-            if (tid == 0) bar_init(bar);
-            __syncthreads();
-            if (tid == 0) {
-                bar_expect_tx(bar, (uint32_t)(NZ * 2 * NY * 16));
-                for (int l = 0; l < NZ; ++l)
-                    bulk_g2s(stage + l * 2 * NY, pp + p_index<true>(g, l, 0, 0, kx), 2 * NY * 16, bar);
-            }
-            if (!bar_wait_bounded(bar, 0)) {
-                atomicExch(g.wait_err, 1);            // the controller halts the run on it
-                bar_wait_bounded(bar, 0);            // once more for the copies still in flight
-            }
-        } else {
-            for (int e = tid; e < NZ * 2 * NY; e += C::THREADS)
-                stage[e] = pp[p_index<true>(g, e / (2 * NY), e % NY, (e / NY) % 2, kx)];
-            __syncthreads();
+        if (tid == 0) bar_init(bar);
+        __syncthreads();
+        if (tid == 0) {
+            bar_expect_tx(bar, (uint32_t)(NZ * 2 * NY * 16));
+            for (int l = 0; l < NZ; ++l)
+                bulk_g2s(stage + l * 2 * NY, pp + p_index<true>(g, l, 0, 0, kx), 2 * NY * 16, bar);
+        }
+        if (!bar_wait_bounded(bar, 0)) {
+            atomicExch(g.wait_err, 1);            // the controller halts the run on it
+            bar_wait_bounded(bar, 0);            // once more for the copies still in flight
         }
         // forward y transforms of (uq)^ (slots 0..NZ-1) and (vq)^ (slots NZ..2NZ-1), unpadded
         const int slot = tid / C::G, lane = tid % C::G;
@@ -859,7 +854,7 @@ __global__ void __launch_bounds__(StageYinvCfg<NY, NZ>::THREADS)
         auto ld = [&](int y) -> double2 { return split_p(col[y], col[NY + y], kx, f); };
         auto omap = [](int y) { return y; };
         fft_fused<NY, -1, SRC_FN, DST_SMEM_MAP, 16, true>(xs, lane, act, twy, ld, omap);
-        if (g.wait_err && tid == 0) bar_inval(bar);
+        if (tid == 0) bar_inval(bar);
     }
     const double kxv = g.dkx * kx;
     const bool expl = lc->explicit_diss != 0;
@@ -993,7 +988,7 @@ static cudaError_t stage_yinv_dispatch(const Geom& g, const Buffers& b, int s, b
 // small grids (at most kSmallStage kept mode-layers, a built (ny, nz) pair, the shared memory
 // fits) take the column kernels; QGN_NO_FUSED_STAGE=1 keeps the separate kernels
 bool stage_yinv_ok(const Geom& g, const Buffers& b) {
-    if (!b.mc_h || g.csize() > kSmallStage || std::getenv("QGN_NO_FUSED_STAGE")) return false;
+    if (!b.mc_h || !g.wait_err || g.csize() > kSmallStage || std::getenv("QGN_NO_FUSED_STAGE")) return false;
     if (g.nz != 2 && g.nz != 4 && g.nz != 8 && g.nz != 16) return false;
     if (!stage_yinv_built(g.ny, g.nz)) return false;
     const int TS = g.ny + g.ny / 16 + 8;
