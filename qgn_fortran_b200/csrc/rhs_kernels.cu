@@ -64,10 +64,15 @@ __global__ void __launch_bounds__(YInvCfg<NY, CT, TV>::THREADS, minb(YInvCfg<NY,
         yinv_tile<NY, NF, CT, TV>(g, threadIdx.x, blockIdx.x, blockIdx.y, q, psi, pq, pv, pu, twy);
 }
 
+// CTAs of the x pass resident on an SM (its registers, at the budget of the form, are what limits them)
+template <int NX, class CT, int TV>
+constexpr int x_resident() {
+    using C = XCfg<NX, false, CT, TV>;
+    return minb(C::THREADS, C::TP == 32 ? (sizeof(CT) == 16 ? 168 : 112) : regcap<CT>(NX >= 1024 ? 112 : 128, 80));
+}
+
 template <int NX, bool DRAG, class CT, int TV = 0, bool PT = false>
-__global__ void __launch_bounds__(XCfg<NX, DRAG, CT, TV>::THREADS,
-                                  minb(XCfg<NX, DRAG, CT, TV>::THREADS,
-                                       XCfg<NX, DRAG, CT, TV>::TP == 32 ? (sizeof(CT) == 16 ? 168 : 112) : regcap<CT>(NX >= 1024 ? 112 : 128, 80)))
+__global__ void __launch_bounds__(XCfg<NX, DRAG, CT, TV>::THREADS, x_resident<NX, CT, TV>())
     k_xpass(Geom g, const CT* __restrict__ pq, const CT* __restrict__ pv,
             const CT* __restrict__ pu, CT* __restrict__ pp, CT* __restrict__ pd,
             const CT* __restrict__ twx) {
@@ -120,6 +125,18 @@ template <int N>
 constexpr bool has_narrow() { return N >= 64 && N <= 256; }
 static bool narrow_better(long long ctas_default, long long ctas_narrow) {
     return ctas_default < 2 * 148 && ctas_narrow > ctas_default;
+}
+
+// Rows of 2048 points have two forms with one row pair per CTA: 32 elements per thread (192 threads) and
+// this one, 16 elements per thread (384 threads), whose transforms are shorter and of which fewer are
+// resident.  A CTA of it is done sooner, so it is taken where it needs no more waves of CTAs -- at most
+// one per SM in FP64, two or, between 444 and 592 CTAs, four in FP32; B200, us per launch, 32 / 16
+// elements: FP64 128 CTAs 20.8 / 15.5, 160 22.9 / 24.8, 256 22.9 / 24.9, 1024 67.8 / 74.3; FP32 128
+// 14.6 / 12.7, 256 16.7 / 16.4, 384 20.3 / 21.5, 512 27.1 / 25.1, 640 30.8 / 31.1, 768 33.0 / 35.2.
+constexpr int kWideX = tv_make(128, 16);
+static bool wide_better(long long ctas, int wide_per_sm, int per_sm) {
+    auto waves = [&](long long resident) { return (ctas + 148 * resident - 1) / (148 * resident); };
+    return waves(wide_per_sm) <= waves(per_sm);
 }
 
 // ------------------------------------------------------------------------------------
@@ -267,22 +284,33 @@ static cudaError_t xpass_go(const Geom& g, const CT* hq, const CT* hp, const CT*
     return cudaGetLastError();
 }
 
+// calls go with the tile form (as a constant) of the x pass for this grid
+template <int NX, class CT, class F>
+static cudaError_t with_x_form(const Geom& g, bool drag, F&& go) {
+    auto blocks = [&](int pairs) { return (long long)((g.ny / 2 + pairs - 1) / pairs); };   // per layer
+    using D = XCfg<NX, false, CT>;
+    if constexpr (has_narrow<NX>()) {
+        using N = XCfg<NX, false, CT, kNarrowX>;
+        if (narrow_better(blocks(D::RP) * g.nz, blocks(N::RP) * g.nz)) return go(std::integral_constant<int, kNarrowX>{});
+    }
+    if constexpr (NX == 2048) {
+        static_assert(D::RP == 1 && XCfg<NX, false, CT, kWideX>::RP == 1, "one row pair per CTA in both forms");
+        if (wide_better(blocks(1) * (g.nz + (drag ? 1 : 0)), x_resident<NX, CT, kWideX>(), x_resident<NX, CT, 0>()))
+            return go(std::integral_constant<int, kWideX>{});
+    }
+    return go(std::integral_constant<int, 0>{});
+}
+
 template <class CT>
 static cudaError_t launch_xpass(const Geom& g, const CT* hq, const CT* hp, const CT* hu, CT* hpp, CT* hpd, const CT* twx,
                                 bool drag, cudaStream_t s) {
     return dispatch_n(g.nx, [&](auto NXc) -> cudaError_t {
         constexpr int NX = decltype(NXc)::value;
-        if constexpr (has_narrow<NX>()) {
-            const long long cd = (long long)((g.ny / 2 + XCfg<NX, false, CT>::RP - 1) / XCfg<NX, false, CT>::RP) * g.nz;
-            const long long cn =
-                (long long)((g.ny / 2 + XCfg<NX, false, CT, kNarrowX>::RP - 1) / XCfg<NX, false, CT, kNarrowX>::RP) *
-                g.nz;
-            if (narrow_better(cd, cn))
-                return drag ? xpass_go<NX, true, CT, kNarrowX>(g, hq, hp, hu, hpp, hpd, twx, s)
-                            : xpass_go<NX, false, CT, kNarrowX>(g, hq, hp, hu, hpp, hpd, twx, s);
-        }
-        return drag ? xpass_go<NX, true, CT, 0>(g, hq, hp, hu, hpp, hpd, twx, s)
-                    : xpass_go<NX, false, CT, 0>(g, hq, hp, hu, hpp, hpd, twx, s);
+        return with_x_form<NX, CT>(g, drag, [&](auto TVc) -> cudaError_t {
+            constexpr int TV = decltype(TVc)::value;
+            return drag ? xpass_go<NX, true, CT, TV>(g, hq, hp, hu, hpp, hpd, twx, s)
+                        : xpass_go<NX, false, CT, TV>(g, hq, hp, hu, hpp, hpd, twx, s);
+        });
     });
 }
 
@@ -344,14 +372,10 @@ static cudaError_t launch_yfwd(const Geom& g, const LayerConst* lc, const CT* q,
 cudaError_t launch_rhs_x_columns(const Geom& g, const Buffers& b, cudaStream_t s) {
     return dispatch_n(g.nx, [&](auto NXc) -> cudaError_t {
         constexpr int NX = decltype(NXc)::value;
-        if constexpr (has_narrow<NX>()) {
-            using D = XCfg<NX, false, double2>;
-            using Nn = XCfg<NX, false, double2, kNarrowX>;
-            if (narrow_better((long long)((g.ny / 2 + D::RP - 1) / D::RP) * g.nz,
-                              (long long)((g.ny / 2 + Nn::RP - 1) / Nn::RP) * g.nz))
-                return xpass_go<NX, false, double2, kNarrowX, true>(g, b.hq, b.hp, b.hu, b.hpp, nullptr, b.twx, s);
-        }
-        return xpass_go<NX, false, double2, 0, true>(g, b.hq, b.hp, b.hu, b.hpp, nullptr, b.twx, s);
+        return with_x_form<NX, double2>(g, false, [&](auto TVc) -> cudaError_t {
+            constexpr int TV = decltype(TVc)::value;
+            return xpass_go<NX, false, double2, TV, true>(g, b.hq, b.hp, b.hu, b.hpp, nullptr, b.twx, s);
+        });
     });
 }
 
