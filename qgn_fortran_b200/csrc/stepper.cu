@@ -743,6 +743,10 @@ __device__ __forceinline__ void stage_yinv_col(const Geom& g, int kx, const Comb
 #pragma unroll
         for (int l = 0; l < NZ; ++l) {
             const size_t e = (size_t)l * P + p;
+            if (!in_bounds(g, e, g.csize())) {
+                qv[l] = make_double2(0.0, 0.0);
+                continue;
+            }
             if constexpr (S == 0) {
                 qv[l] = q[e];
             } else {
@@ -764,7 +768,7 @@ __device__ __forceinline__ void stage_yinv_col(const Geom& g, int kx, const Comb
         modal_invert<NZ>(ma.proj, ma.back, ma.ev, ma.Htot, NZ, k2, p == 0, qv, pvv);
 #pragma unroll
         for (int l = 0; l < NZ; ++l) {
-            psi[(size_t)l * P + p] = pvv[l];
+            if (in_bounds(g, (size_t)l * P + p, g.csize())) psi[(size_t)l * P + p] = pvv[l];
             pcol[l * nky + m] = pvv[l];
         }
     }
@@ -787,10 +791,13 @@ __device__ __forceinline__ void stage_yinv_col(const Geom& g, int kx, const Comb
     };
     auto omap = [](int y) { return (y & 1) * C::HY + (y >> 1); };
     fft_fused<NY, +1, SRC_FN, DST_SMEM_MAP, 16, true>(xs, lane, true, twy, ld, omap);
-    double2* dst = (f == 0 ? pq : (f == 1 ? pu : pv)) + (size_t)l * (NY / 2) * 2 * g.nkxp;
+    double2* dst = f == 0 ? pq : (f == 1 ? pu : pv);
+    const size_t layer = (size_t)l * (NY / 2) * 2 * g.nkxp;
     for (int pr = lane; pr < NY / 2; pr += C::G) {
+        const size_t ro = layer + (size_t)pr * 2 * g.nkxp;
+        if (!in_bounds(g, ro + g.nkxp + kx, g.hsize())) continue;
         const double2 f1 = xs[pr], f2 = xs[C::HY + pr];
-        double2* row = dst + (size_t)pr * 2 * g.nkxp;
+        double2* row = dst + ro;
         row[kx] = pack_lo(f1, f2, kx == 0 || 2 * kx == g.nx);
         row[g.nkxp + kx] = kx > 0 ? pack_hi(f1, f2) : make_double2(0.0, 0.0);
     }
@@ -837,8 +844,10 @@ __global__ void __launch_bounds__(StageYinvCfg<NY, NZ>::THREADS)
         if (tid == 0) bar_init(bar);
         __syncthreads();
         if (tid == 0) {
-            bar_expect_tx(bar, (uint32_t)(NZ * 2 * NY * 16));
-            for (int l = 0; l < NZ; ++l)
+            int layers = 0;   // all NZ, but for a failed check
+            while (layers < NZ && in_bounds(g, p_index<true>(g, layers, NY - 1, 1, kx), 2 * g.hsize())) ++layers;
+            bar_expect_tx(bar, (uint32_t)(layers * 2 * NY * 16));
+            for (int l = 0; l < layers; ++l)
                 bulk_g2s(stage + l * 2 * NY, pp + p_index<true>(g, l, 0, 0, kx), 2 * NY * 16, bar);
         }
         if (!bar_wait_bounded(bar, 0)) {
@@ -864,6 +873,7 @@ __global__ void __launch_bounds__(StageYinvCfg<NY, NZ>::THREADS)
 #pragma unroll
         for (int l = 0; l < NZ; ++l) {
             const size_t idx = ((size_t)l * g.nkx + kx) * nky + m;
+            if (!in_bounds(g, idx, g.csize())) continue;
             const double2 fuq = slots[l * C::TS + j], fvq = slots[(NZ + l) * C::TS + j];
             const double2 qv = qprev[idx], pvv = psi[idx];
             // jaco_hat = i kx uq_hat + i ky vq_hat  (QGN_Module.f90:244-247)
