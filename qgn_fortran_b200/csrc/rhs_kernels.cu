@@ -89,10 +89,21 @@ __global__ void __launch_bounds__(XCfg<NX, DRAG, CT, TV>::THREADS, x_resident<NX
     xpass_tile<NX, DRAG, CT, TV, PT>(g, threadIdx.x, blockIdx.x, blockIdx.y, pq, pv, pu, pp, pd, twx);
 }
 
+// FP64 columns of 1024 points have two forms: one column per CTA (the default, 256 threads) and this one,
+// two columns per CTA (512 threads).  Up to a CTA per SM one column is the shorter work, and beyond two the
+// narrow CTAs fill the SMs more evenly; in between some SMs have two of them, others one, and the pairs,
+// which read their rows in 32-byte pieces instead of 16, are done sooner.  So pairs are taken where they
+// are at most one per SM and single columns are not.  With quadratic drag the bottom layer's tiles, which
+// transform twice, are the launch's length, and two of its columns on an SM are worse than one.  B200, us
+// per launch, one / two columns: 147 columns 11.1 / 12.7, 160 12.9 / 12.7, 170 13.2 / 12.6, 255 13.9 / 12.6,
+// 294 14.0 / 16.6 in 154 pairs and 14.3 / 12.6 in 147; with drag 170 16.7 / 18.7, 255 16.7 / 18.7.
+constexpr int kPairY = tv_make(512, 8);
+static bool pairs_better(long long columns, long long pairs) { return pairs <= 148 && columns > 148; }
+
 // y-forward launches whose rows come by tensor-map copies: the default tiles of 256 points and more
 // (shorter columns are a fraction of a launch's latency, and their tiles' rows are whole lines)
 template <int NY, int TV, bool PT = false>
-__host__ __device__ constexpr bool yfwd_mapped() { return TV == 0 && NY >= 256 && !PT; }
+__host__ __device__ constexpr bool yfwd_mapped() { return (TV == 0 || TV == kPairY) && NY >= 256 && !PT; }
 
 template <int NY, bool DRAG, class CT, int TV = 0, bool PT = false>
 __global__ void __launch_bounds__(YFwdCfg<NY, DRAG, CT, TV>::THREADS,
@@ -361,6 +372,11 @@ static cudaError_t launch_yfwd(const Geom& g, const LayerConst* lc, const CT* q,
                               (long long)((g.nkx + Nn::TKX - 1) / Nn::TKX) * g.nz))
                 return drag ? yfwd_go<NY, true, CT, kNarrowY>(g, lc, q, psi, hpp, hpd, out, twy, extra, s)
                             : yfwd_go<NY, false, CT, kNarrowY>(g, lc, q, psi, hpp, hpd, out, twy, extra, s);
+        }
+        if constexpr (NY == 1024 && sizeof(CT) == 16) {
+            static_assert(YFwdCfg<NY, false, CT>::TKX == 1 && YFwdCfg<NY, false, CT, kPairY>::TKX == 2, "one or two columns");
+            if (!drag && pairs_better((long long)g.nkx * g.nz, (long long)((g.nkx + 1) / 2) * g.nz))
+                return yfwd_go<NY, false, CT, kPairY>(g, lc, q, psi, hpp, hpd, out, twy, extra, s);
         }
         return drag ? yfwd_go<NY, true, CT, 0>(g, lc, q, psi, hpp, hpd, out, twy, extra, s)
                     : yfwd_go<NY, false, CT, 0>(g, lc, q, psi, hpp, hpd, out, twy, extra, s);
