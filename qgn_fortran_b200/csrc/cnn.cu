@@ -691,7 +691,7 @@ __host__ __device__ constexpr int row_arrivals() { return Row<C>::SWZ ? 2 : 1; }
 }  // namespace tc
 
 // Epilogue of one tile of the fused inference: warp w reads TMEM lanes 32 (w % 4).. (one pixel per thread) and a block
-// of columns, applies bias + GELU (or GELU' for the backward pass), and writes the tile through
+// of columns, applies bias and, but for the last layer, GELU, and writes the tile through
 // XOR-swizzled shared-memory staging so that the global stores are contiguous 16-byte pieces.
 // The tile's outputs are contiguous in global memory: pixels p0 .. p0+127, COUT channels each.
 // Columns of the accumulator each epilogue thread drains (NW warps: four TMEM sub-partitions,
@@ -772,10 +772,12 @@ __device__ __forceinline__ void conv_tc_epilogue(uint32_t tacc, size_t p0, const
 // of weights per 16 channels when each tap row was an MMA of its own with N = 64 (63 cycles measured,
 // 36 of them per tile), 4 + 6 KB for the three together.  The sum of an output is formed in the same
 // order either way (dh, dw, channels).
-// The epilogue's arithmetic is what is left: 8192 GELUs per tile, 32 instructions each.  64 -> 64 at
-// batch 32 on 128^2 (B200, ncu): loads, MMAs and epilogue one after another in the same warps 152 us
-// with an FP32 second output; the split in roles 118 us, 92 us without it (inference); this form 86 and
-// 69 us.
+// 64 -> 64 at batch 32 on 128^2 (B200, ncu): loads, MMAs and epilogue one after another in the same warps
+// 152 us with an FP32 second output; the split in roles 118 us, 92 us without it (inference); this form 86
+// and 69 us.  Of the 69, the GELUs (8192 per tile, 32 instructions each) are 29 us of issue and the MMAs
+// 15, on different warps, and neither is the bound: all sixteen epilogue warps take the same tile, wait for
+// its tcgen05.ld together and then issue together (at batch 8: tensor pipe 19 %, issue slots 34 %, long
+// scoreboard 3.5 of the stalls per issued instruction).
 // EPI_GELU stores GELU'(z) in FP32 beside the activation, where the backward pass only multiplies by
 // it: the error function is evaluated once per training step instead of twice.
 template <int CIN, int COUT, int EPI>

@@ -12,7 +12,11 @@
 // against 29.5 us here, and 42 us for 5 layers on 512 x 256 (in the explicit combinations),
 // against 8.6 us.  At exactly 16 layers both fit, and it is the input that decides (2048^2, us):
 // FP64 114.8 one-thread, 107.9 matrix units; FP32 110.0 one-thread, 115.1 matrix units, whose
-// quarter-warps read 32-byte pieces of an FP32 field.
+// quarter-warps read 32-byte pieces of an FP32 field.  (On smaller grids the one-thread form's chain of
+// products shows: FP32, 16 layers in it against 15 padded to 16 on the matrix units, events included, 64^2
+// 11.5 / 8.6, 256^2 12.4 / 9.0, 512^2 15.0 / 14.5, 1024^2 34.6 / 33.4; the rule goes by the large grids.)
+// 9 to 15 layers are padded to 16: FP32, in the generic form / here, 9 layers 64^2 30.5 / 8.7, 1024^2
+// 140.9 / 31.7; 15 layers 39.1 / 8.6 and 212.4 / 33.4.
 #include "qgn_internal.cuh"
 #include "prof.cuh"
 #include "rhs_tiles.cuh"

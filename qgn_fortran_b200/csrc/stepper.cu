@@ -907,7 +907,8 @@ __global__ void __launch_bounds__(StageYinvCfg<NY, NZ>::THREADS)
     stage_yinv_col<S, NZ, NY>(g, kx, cp, q, qout, psi, lc, ma, sc, pq, pv, pu, twy, sm_raw);
 }
 
-// the (ny, nz) pairs built: a CTA keeps its registers without spilling
+// the (ny, nz) pairs built: 3 nz transforms of the column fit a CTA's threads and shared memory.  At 16
+// layers the kernels spill 124 to 324 bytes per thread and stage 4 of 4 layers 16 to 72; the others none.
 constexpr bool stage_yinv_built(int ny, int nz) {
     return (ny == 128 && nz <= 16) || (ny == 256 && nz <= 8) || (ny == 512 && nz <= 4);
 }
@@ -1068,7 +1069,9 @@ cudaError_t launch_ark_update(const Geom& g, const Buffers& b, cudaStream_t st) 
 }
 
 // psi in the same launch for nz <= 8, where it saves reading q_tmp back (5 layers on 512 x 256:
-// 41.8 us in the generic form that kept 32 layers per thread in local memory)
+// 41.8 us in the generic form that kept 32 layers per thread in local memory).  At 16 layers that read is
+// cheaper than one thread holding them all: BSRK3's combinations with psi in one launch / in two, us, 64^2
+// 20.8 / 14.8, 256^2 21.9 / 15.6, 512^2 32.6 / 26.8, 1024^2 103.7 / 68.6.
 cudaError_t launch_combo(const Geom& g, const Buffers& b, const Combo& cb, const double2* q, double2* out,
                          double2* psi, bool want_psi, cudaStream_t st) {
     const double C = 16.0 * (double)g.csize();
